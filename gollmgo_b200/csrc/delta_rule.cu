@@ -15,17 +15,7 @@
 // of a head are spread over CTAs; eight lanes share a column and split its d rows.
 // Everything here is float32 arithmetic; only the projections that come in (x, gate) and the
 // result that goes out are in the activation type.
-#include "common.cuh"
-
-// Index of the sequence that token t belongs to: the largest b with cu[b] <= t.
-__device__ __forceinline__ int seq_of_token(const int* __restrict__ cu, int B, int t) {
-  int lo = 0, hi = B - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (cu[mid] <= t) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
+#include "short_conv.cuh"
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
@@ -86,6 +76,45 @@ __global__ void delta_prep_kernel(const TA* __restrict__ x, long long x_stride, 
     if (u < G) f *= rsqrtf((float)d);
   }
   for (int e = threadIdx.x; e < dh; e += blockDim.x) qkv_out[(size_t)t * C + c0 + e] = ys[e] * f;
+}
+
+// The same for TAPS taps, heads of 32, 64 or 128 in q and k, and channels in groups of four: grid (tokens / per, groups
+// of 128 threads + 1), four channels a thread (short_conv.cuh); the lanes of a q or k head sum its squares among
+// themselves.  Bound by the latency of a block's few dependent reads (sequence, window, rows): 2048 tokens of 16 + 2 x 4 heads of
+// 128 take 20 us (bytes at the copy rate: 6), where the kernel above, a block per token and head with 2-byte loads of every
+// row `taps` times, takes 67.
+template <typename TA, int TAPS>
+__global__ void __launch_bounds__(CONV_THREADS, 8)
+delta_prep_vec_kernel(const TA* __restrict__ x, long long x_stride, const float* __restrict__ conv_w, float* conv_state,
+                      const float* __restrict__ zb_in, long long zb_stride, const float* __restrict__ za_in, long long za_stride,
+                      int dw, const float* __restrict__ a_log, const float* __restrict__ dt_bias, const int* __restrict__ cu_q_lens,
+                      const int* __restrict__ context_lens, const int* __restrict__ state_slots, int T, int B, int G, int H, int d,
+                      int dv, int per, int single, float* __restrict__ qkv_out, float* __restrict__ beta, float* __restrict__ decay) {
+  pdl_trigger();
+  const int ta = blockIdx.x * per, tb = min(T, ta + per);
+  const int C = 2 * G * d + H * dv;
+  if (blockIdx.y == gridDim.y - 1) {
+    pdl_wait();
+    const int n = H * (1 + dw);
+    for (int i = threadIdx.x; i < (tb - ta) * n; i += CONV_THREADS) {
+      const int t = ta + i / n, e = i % n - H;
+      if (e < 0) beta[(size_t)t * H + e + H] = 1.f / (1.f + expf(-zb_in[(size_t)t * zb_stride + e + H]));
+      else decay[(size_t)t * H * dw + e] = expf(-expf(a_log[e / dw]) * softplus_f(za_in[(size_t)t * za_stride + e] + dt_bias[e]));
+    }
+    return;
+  }
+  const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) << 2;
+  const bool live = c < C, unit = c < 2 * G * d;
+  const int lanes = d >> 2;                              // of one q or k head: 8, 16 or 32
+  const float scale = c < G * d ? rsqrtf((float)d) : 1.f;
+  conv_tokens<TAPS>(x, x_stride, conv_w, (const float*)nullptr, conv_state, cu_q_lens, context_lens, state_slots, B, C,
+                    live ? c : 0, ta, tb, single && live, [&](int t, float4 y) {
+    float ss = y.x * y.x + y.y * y.y + (y.z * y.z + y.w * y.w);
+    for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float f = unit ? rsqrtf(ss + 1e-6f) * scale : 1.f;
+    y = make_float4(y.x * f, y.y * f, y.z * f, y.w * f);
+    if (live) store4(qkv_out + (size_t)t * C + c, y);
+  });
 }
 
 // grid (B, ceil(C / 128)): the window of the convolution after this step's tokens.
@@ -397,6 +426,44 @@ __global__ void delta_out_kernel(const float* __restrict__ o_raw, const TA* __re
   }
 }
 
+// A warp a head, four values a lane at a time (heads of up to 512 values, a multiple of 4): 2048 tokens of 16 heads of
+// 128 take 16 us (bytes at the copy rate: 5; the gate's exponential and division are half of it); with a block per head and a
+// value a thread 35.
+template <typename TA>
+__global__ void __launch_bounds__(256)
+delta_out_vec_kernel(const float* __restrict__ o_raw, const TA* __restrict__ gate, long long gate_stride,
+                     const float* __restrict__ w, float eps, int H, int dv, int gate_act, long long heads, TA* __restrict__ out) {
+  pdl_trigger();
+  const long long u = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (u >= heads) return;
+  const int lane = threadIdx.x & 31, h = (int)(u % H);
+  const size_t t = (size_t)(u / H);
+  pdl_wait();
+  const float* o = o_raw + (size_t)u * dv;
+  const TA* gr = gate + t * gate_stride + (size_t)h * dv;
+  float4 v[4], z[4];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = (i * 32 + lane) << 2;
+    if (c < dv) { v[i] = *reinterpret_cast<const float4*>(o + c); z[i] = load4(gr + c); }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (((i * 32 + lane) << 2) < dv) ss += v[i].x * v[i].x + v[i].y * v[i].y + (v[i].z * v[i].z + v[i].w * v[i].w);
+  const float f = rsqrtf(warp_sum(ss) / (float)dv + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = (i * 32 + lane) << 2;
+    if (c < dv) {
+      const float4 ww = w ? *reinterpret_cast<const float4*>(w + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+      auto act = [&](float g) { return gate_act == 1 ? 1.f / (1.f + expf(-g)) : silu_f(g); };
+      store4(out + (size_t)u * dv + c, make_float4(v[i].x * f * ww.x * act(z[i].x), v[i].y * f * ww.y * act(z[i].y),
+                                                   v[i].z * f * ww.z * act(z[i].z), v[i].w * f * ww.w * act(z[i].w)));
+    }
+  }
+}
+
 // ---------------------------------------------------------------- launchers
 // The window of a short convolution over the C channels x[:, 0 .. C) moved on by this step's tokens
 // (also for the state-space layer, ssm.cu).
@@ -422,6 +489,25 @@ extern "C" int gg_delta_prep(const void* x, long long x_stride, int dtype, const
   const int C = 2 * G * d + H * dv;
   GG_REQUIRE(x_stride >= C, "delta_prep: rows of %lld values hold no %d channels", x_stride, C);
   if (T == 0) return GG_OK;
+  const bool vec = taps >= 2 && taps <= 4 && (d == 32 || d == 64 || d == 128) && dv % 4 == 0 && x_stride % 4 == 0 &&
+                   ((size_t)x % 16) == 0 && ((size_t)conv_w % 16) == 0 && ((size_t)conv_state % 16) == 0 && ((size_t)qkv_out % 16) == 0 &&
+                   (C / 4 + CONV_THREADS - 1) / CONV_THREADS < 65535;
+  if (vec) {
+    const int single = T == B, per = T > 4 * B ? CONV_TOKENS : 1;
+    const dim3 vgrid((T + per - 1) / per, (C / 4 + CONV_THREADS - 1) / CONV_THREADS + 1);
+#define DP_GO(TA, TAPS)                                                                                                          \
+  gg_launch(delta_prep_vec_kernel<TA, TAPS>, vgrid, dim3(CONV_THREADS), 0, stream, (const TA*)x, x_stride, conv_w, conv_state, zb, \
+            zb_stride, za, za_stride, dw, a_log, dt_bias, cu_q_lens, context_lens, state_slots, T, B, G, H, d, dv, per, single, qkv_out, beta, decay)
+#define DP_TAPS(TA) do { if (taps == 2) DP_GO(TA, 2); else if (taps == 3) DP_GO(TA, 3); else DP_GO(TA, 4); } while (0)
+    if (dtype == GG_F32) DP_TAPS(float);
+    else if (dtype == GG_BF16) DP_TAPS(__nv_bfloat16);
+    else return gg_fail(GG_ERR_INVALID, "delta_prep: unknown dtype %d", dtype);
+#undef DP_TAPS
+#undef DP_GO
+    const int rc = gg_check_launch("delta_prep");
+    if (rc || single) return rc;
+    return conv_state_update(x, x_stride, dtype, conv_state, cu_q_lens, context_lens, state_slots, B, C, taps, stream);
+  }
   const int big = d > dv ? d : dv;
   GG_REQUIRE(big <= 8192, "delta_prep: head size %d is too large", big);
   const size_t smem = (size_t)(big + 33) * sizeof(float);
@@ -491,6 +577,16 @@ extern "C" int gg_delta_out(const float* o_raw, const void* gate, long long gate
   GG_REQUIRE(T >= 0 && H > 0 && dv > 0 && H <= 65535, "delta_out: bad sizes T=%d H=%d dv=%d", T, H, dv);
   GG_REQUIRE(gate_act == 0 || gate_act == 1, "delta_out: the gate passes silu (0) or a sigmoid (1), not %d", gate_act);
   if (T == 0) return GG_OK;
+  const long long heads = (long long)T * H;
+  if (dv % 4 == 0 && dv <= 512 && gate_stride % 4 == 0 && ((size_t)o_raw % 16) == 0 && ((size_t)gate % 16) == 0 &&
+      ((size_t)out % 16) == 0 && (!w || ((size_t)w % 16) == 0) && (dtype == GG_F32 || dtype == GG_BF16)) {
+    const dim3 vgrid((unsigned)((heads + 7) / 8));
+    if (dtype == GG_F32)
+      gg_launch(delta_out_vec_kernel<float>, vgrid, dim3(256), 0, stream, o_raw, (const float*)gate, gate_stride, w, eps, H, dv, gate_act, heads, (float*)out);
+    else
+      gg_launch(delta_out_vec_kernel<__nv_bfloat16>, vgrid, dim3(256), 0, stream, o_raw, (const __nv_bfloat16*)gate, gate_stride, w, eps, H, dv, gate_act, heads, (__nv_bfloat16*)out);
+    return gg_check_launch("delta_out");
+  }
   const int threads = dv >= 256 ? 256 : (dv >= 128 ? 128 : 64);
   const dim3 grid(T, H);
   if (dtype == GG_F32)
