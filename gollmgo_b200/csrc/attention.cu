@@ -420,7 +420,7 @@ extern "C" int gg_attn_prefill(const void* q, long long q_stride, const void* kc
     // 3 = two heads per CTA in steps of 64 keys (what 1 gave before there were steps of 128)
     static const bool wide = !(getenv("GOLLMGO_B200_ATTN_STEP") && atoi(getenv("GOLLMGO_B200_ATTN_STEP")) == 64);
     if (allow_tc == 1 && wide && attn_tc3_supported(dtype, d, page_size, nh, nkv))
-      return attn_prefill_tc3(a, num_tiles128, T, num_pages, status, stream);
+      return attn_prefill_tc3(a, num_tiles128, T, num_pages, status, false, stream);
     if (allow_tc != 2 && attn_tc2_supported(dtype, d, page_size, nh, nkv))
       return attn_prefill_tc2(a, num_tiles128, T, num_pages, status, stream);
     if (attn_tc_supported(dtype, d, page_size))
@@ -546,6 +546,7 @@ extern "C" int gg_attn_prefill_x(const void* q, long long q_stride, const void* 
                                  int dtype, const int* block_tables, int bt_stride, const int* cu_q_lens,
                                  const int* context_lens, const int* tile_seq, const int* tile_q0, int num_tiles,
                                  const int* tile64_seq, const int* tile64_q0, int num_tiles64, int allow_mma,
+                                 const int* tile128_seq, const int* tile128_q0, int num_tiles128, int T, int num_pages, int* status,
                                  void* out, int out_f32, int nh, int nkv, int d, int dv, int v_share,
                                  int page_size, int window, float scale, float softcap, int keep_first, int weights,
                                  const float* head_bias, const float* dist_bias, const int* dist_bucket, int dist_max, int chunk, const float* sink,
@@ -569,6 +570,13 @@ extern "C" int gg_attn_prefill_x(const void* q, long long q_stride, const void* 
   // what the mma.sync kernels compute: softmax without these extras, or sigmoid weights with all of them
   const bool plain = (!a.keep_first && !weights && !head_bias && !dist_bias) || attn_mma_x_sigmoid_supported(a);
   if (a.chunk || a.sink) allow_mma = allow_mma && attn_mma_x_chunk_sink_supported();
+  // softmax weights without kept keys or a bias table, even groups of heads: tcgen05 over tiles of 128 queries, where the
+  // caller gives that list (see Attention.long_tiles in parts/attention.py)
+  if (tile128_seq && status && !a.keep_first && !weights && !head_bias && !dist_bias && q_stride % 8 == 0 && ((size_t)q % 16) == 0 &&
+      attn_tc3_x_supported(dtype, d, dv > 0 ? dv : d, page_size, nh, nkv)) {
+    a.tile_seq = tile128_seq; a.tile_q0 = tile128_q0;
+    return attn_prefill_tc3(a, num_tiles128, T, num_pages, status, true, stream);
+  }
   // bfloat16 with sizes of 64 or 128: the mma.sync kernel over tiles of 64 queries
   if (plain && allow_mma && tile64_seq && attn_mma_x_supported(dtype, d, dv > 0 ? dv : d, page_size) && q_stride % 8 == 0) {
     a.tile_seq = tile64_seq; a.tile_q0 = tile64_q0;

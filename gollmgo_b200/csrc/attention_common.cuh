@@ -41,7 +41,7 @@ struct AttnArgs {
   const int* dist_bucket;   // [dist_max + 1]
   int dist_max;
   int chunk;                // > 0: the sequence is cut into chunks of this many positions, counted from 0, and a query sees
-                            // only the keys of its own chunk (all kernels but the tcgen05 ones and the plain mma.sync ones)
+                            // only the keys of its own chunk (the general kernels, their mma.sync form and attention_tc3.cu with x)
   const float* sink;        // [nh] or null: exp(sink[h]) is one more term of the softmax denominator, with no key and no value
   const float* slopes;      // [nh] or null: slopes[h] * (i - j) is taken off the scaled score (softmax weights)
   float temp_coef;          // the query at position p is multiplied by 1 + temp_coef * ln(floor((p + 1) / temp_every) + 1)
@@ -84,7 +84,10 @@ bool attn_tc2_supported(int dtype, int d, int page_size, int nh, int nkv);
 int attn_prefill_tc2(const AttnArgs& a, int num_tiles, int T, int num_pages, int* status, cudaStream_t stream);
 // the same in steps of 128 keys (attention_tc3.cu)
 bool attn_tc3_supported(int dtype, int d, int page_size, int nh, int nkv);
-int attn_prefill_tc3(const AttnArgs& a, int num_tiles, int T, int num_pages, int* status, cudaStream_t stream);
+int attn_prefill_tc3(const AttnArgs& a, int num_tiles, int T, int num_pages, int* status, bool x, cudaStream_t stream);
+// ... and with the options of the general path (softmax weights: a.dv, a.v_share, a.softcap, a.chunk, a.sink, a.slopes, the
+// query temperature, a.out_f32): x = true above
+bool attn_tc3_x_supported(int dtype, int d, int dv, int page_size, int nh, int nkv);
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);

@@ -29,7 +29,13 @@
 // the softmax groups take them (setmaxnreg.inc).  The launcher checks that what the kernel
 // was given at launch covers both numbers, since a group that asks for more than there is
 // waits for ever.
-// Tensor memory per head: columns [0, 128) scores / P, [128, 128 + d) O; head 1 at +256.
+// X: the attention of the general path (attention.cu) with softmax weights: values of another size than keys and value
+// heads that several key heads share, scores capped by a tanh, a bias by distance, a query temperature, chunks, a sink in
+// the denominator, float32 results.  A row's scores become base-2 exponents as they leave tensor memory (two packed
+// multiply-adds a pair with a bias, a tanh of the special-function unit more with a cap); everything else is the plain
+// kernel.  2048 tokens of 32 heads of 128, window 1024, with a bias, a sink and a temperature: 82 us, on mma.sync 266
+// (the plain kernel without a window: 54).
+// Tensor memory per head: columns [0, 128) scores / P, [128, 128 + dv) O; head 1 at +256.
 // All waits on barriers are bounded; a wait that runs out sets *status and the CTA winds down.
 #include "attention_common.cuh"
 #include "tc_common.cuh"
@@ -82,6 +88,13 @@ __device__ __forceinline__ void at3_fma2(float& r0, float& r1, float x0, float x
       "fma.rn.f32x2 pd, pa, pb, pc;\n\tmov.b64 {%0, %1}, pd;\n\t}"
       : "=f"(r0), "=f"(r1) : "f"(x0), "f"(x1), "f"(m), "f"(c));
 }
+// (x0, x1) = (x0, x1) * m + (c0, c1)
+__device__ __forceinline__ void at3_fma2_into(float& x0, float& x1, float m, float c0, float c1) {
+  asm("{\n\t.reg .b64 pa, pb, pc, pd;\n\t"
+      "mov.b64 pa, {%0, %1};\n\tmov.b64 pb, {%2, %2};\n\tmov.b64 pc, {%3, %4};\n\t"
+      "fma.rn.f32x2 pd, pa, pb, pc;\n\tmov.b64 {%0, %1}, pd;\n\t}"
+      : "+f"(x0), "+f"(x1) : "f"(m), "f"(c0), "f"(c1));
+}
 // (a0, a1) += (x0, x1)
 __device__ __forceinline__ void at3_add2(float& a0, float& a1, float x0, float x1) {
   asm("{\n\t.reg .b64 pa, pb, pd;\n\t"
@@ -96,7 +109,7 @@ struct At3Args {
   int* status;
 };
 
-template <int D>
+template <int D, int DV, bool X>
 __global__ void __launch_bounds__(AT3_THREADS, 1)
 attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const At3Args args) {
@@ -104,8 +117,9 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   __shared__ __align__(8) unsigned long long bars[20];
   __shared__ unsigned tmem_base_s;
   __shared__ int abort_s;
-  constexpr int HALVES = D / 64;
-  constexpr unsigned TILE_BYTES = HALVES * AT3_HALF;      // a Q, K or V tile: 128 rows x D
+  constexpr int HALVES = D / 64, V_HALVES = DV / 64;
+  constexpr unsigned TILE_BYTES = HALVES * AT3_HALF;      // a Q or K tile: 128 rows x D
+  constexpr unsigned V_BYTES = V_HALVES * AT3_HALF;       // a V tile: 128 rows x DV
   const AttnArgs& a = args.a;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned base = (tc_smem(at3_smem_raw) + 1023u) & ~1023u;
@@ -156,7 +170,9 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   const int nrows = min(AT3_BQ, qlen - q0);
   const int first = qstart + q0;                       // position of the tile's first query
   const int hi = first + nrows;
-  const int lo = a.window > 0 ? max(0, first - a.window + 1) : 0;
+  int lo = a.window > 0 ? max(0, first - a.window + 1) : 0;
+  if (X && a.chunk > 0) lo = max(lo, (first / a.chunk) * a.chunk);       // the chunk of the tile's first row starts earliest
+  const int vh = X && a.v_share > 1 ? kvh / a.v_share : kvh;
   const int kstart = (lo / AT3_BK) * AT3_BK;
   const int ntiles = (hi - kstart + AT3_BK - 1) / AT3_BK;
   const int ps = a.page_size, pages_per_tile = AT3_BK / ps;
@@ -189,17 +205,19 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const unsigned row_off = (unsigned)(lane * ps * 128);
         for (int which = 0; which < 2 && ok; ++which) {          // keys, then values
           const unsigned full = (which ? v_full0 : k_full0) + 8 * s, empty = (which ? v_empty0 : k_empty0) + 8 * s;
-          const unsigned dst = (which ? v_smem : k_smem) + s * TILE_BYTES;
+          const unsigned bytes = which ? V_BYTES : TILE_BYTES;
+          const unsigned dst = (which ? v_smem : k_smem) + s * bytes;
           const CUtensorMap* map = which ? &map_v : &map_k;
           ok = mbar_wait(empty, phase ^ 1) && !*(volatile int*)&abort_s;
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          if (lane == 0) mbar_expect_tx(full, TILE_BYTES);
+          if (lane == 0) mbar_expect_tx(full, bytes);
           __syncwarp();
           if (lane < pages_per_tile) {
 #pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf)
-              tma_load_4d(dst + hf * AT3_HALF + row_off, map, hf * 64, 0, kvh, page, full);
+            for (int hf = 0; hf < (HALVES > V_HALVES ? HALVES : V_HALVES); ++hf)
+              if (hf < (which ? V_HALVES : HALVES))
+                tma_load_4d(dst + hf * AT3_HALF + row_off, map, hf * 64, 0, which ? vh : kvh, page, full);
           }
         }
       }
@@ -210,8 +228,8 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       const int t = warp - 1;
       // instruction descriptors: f32 accumulate, bf16 inputs, M = 128; scores: N = 128 keys
       const unsigned idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-      // O += P V: N = D, B (V) is MN-major
-      const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (((unsigned)D >> 3) << 17) | ((128u >> 4) << 24);
+      // O += P V: N = DV, B (V) is MN-major
+      const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (((unsigned)DV >> 3) << 17) | ((128u >> 4) << 24);
       // the descriptors' upper words never change and a tile's k step only adds to the address
       // field of the lower word
       const unsigned hi_k = 64u | (1u << 14) | (2u << 29);                 // SBO 1024 bytes, version 1, 128-byte swizzle
@@ -222,7 +240,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         k_lo[i] = lo_word(k_smem + i * TILE_BYTES, lbo_k);
-        v_lo[i] = lo_word(v_smem + i * TILE_BYTES, lbo_v);
+        v_lo[i] = lo_word(v_smem + i * V_BYTES, lbo_v);
       }
       const unsigned tmem_s = tmem_base + t * 256, tmem_o = tmem_s + 128;
       bool ok = mbar_wait(q_full, 0);
@@ -270,7 +288,13 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const bool row_ok = r < nrows;
     const unsigned lane_addr = tmem_base + t * 256 + ((unsigned)(quarter * 32) << 16);
     const unsigned tmem_o = lane_addr + 128;
-    const float sc = a.scale * AT3_LOG2E;
+    // X: the row's own scale (a query temperature is part of it), the head's slope in base-2 exponents, the cap, and the
+    // first key of the row's chunk
+    const float sc = a.scale * AT3_LOG2E * (X ? query_temperature(a, pos) : 1.f);
+    const float slope = X && a.slopes ? a.slopes[h0 + t] * AT3_LOG2E : 0.f;
+    const float cap2 = X ? a.softcap * AT3_LOG2E : 0.f, to_cap = cap2 > 0.f ? sc / cap2 : 0.f;
+    const int row_chunk = X && a.chunk > 0 ? (pos / a.chunk) * a.chunk : 0;
+    const int tile_chunk = X && a.chunk > 0 ? ((first + nrows - 1) / a.chunk) * a.chunk : 0;
     float m_ref = -INFINITY, l = 0.f;
     const int stale_hi = (hi + ps - 1) / ps * ps;        // end of the last page that is fetched
     bool ok = true;
@@ -281,7 +305,8 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const bool interior = kb >= lo && kb + AT3_BK - 1 <= first && (a.window <= 0 || kb > first + nrows - 1 - a.window);
+      const bool interior = kb >= lo && kb + AT3_BK - 1 <= first && (a.window <= 0 || kb > first + nrows - 1 - a.window) &&
+                            (!X || kb >= tile_chunk);
       // the row's 128 scores, once, into registers (as they come: the scale to base 2 is folded
       // into the exponential's argument; masked ones -inf).  The four loads are in flight together.
       float sv[AT3_BK];
@@ -293,11 +318,37 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
         for (int i = 0; i < AT3_BK; ++i) sv[i] = __uint_as_float(raw[i]);
       }
+      if (X) {                                 // the scores as base-2 exponents
+        if (cap2 > 0.f) {
+#pragma unroll
+          for (int i = 0; i < AT3_BK; ++i) {
+            float th;
+            asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(sv[i] * to_cap));
+            sv[i] = cap2 * th;
+          }
+          if (slope != 0.f) {
+#pragma unroll
+            for (int i = 0; i < AT3_BK; ++i) sv[i] = fmaf(slope, (float)(kb + i - pos), sv[i]);
+          }
+        } else if (slope != 0.f) {
+          const float away = (float)(kb - pos);           // exact, like its sum with i
+#pragma unroll
+          for (int i = 0; i < AT3_BK; i += 2) {
+            float d0 = away + (float)i, d1 = away + (float)(i + 1);
+            at3_fma2(d0, d1, d0, d1, slope, 0.f);
+            at3_fma2_into(sv[i], sv[i + 1], sc, d0, d1);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < AT3_BK; i += 2) at3_fma2(sv[i], sv[i + 1], sv[i], sv[i + 1], sc, 0.f);
+        }
+      }
       if (!interior) {
 #pragma unroll
         for (int i = 0; i < AT3_BK; ++i) {
           const int tk = kb + i;
-          const bool keep = row_ok && tk >= lo && tk <= pos && (a.window <= 0 || tk > pos - a.window);
+          const bool keep = row_ok && tk >= lo && tk <= pos && (a.window <= 0 || tk > pos - a.window) &&
+                            (!X || tk >= row_chunk);
           if (!keep) sv[i] = -INFINITY;
         }
       }
@@ -309,7 +360,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
         for (int u = 0; u < 4; ++u) mxs[u] = at3_max3(mxs[u], sv[i + 2 * u], sv[i + 2 * u + 1]);
       }
-      const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * sc;      // sc > 0
+      const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * (X ? 1.f : sc);      // sc > 0
       // move the reference maximum only when some row of the warp has outgrown it by 2^8
       const bool grow = mx > m_ref + 8.f;
       const bool rescale = __any_sync(0xffffffffu, grow);
@@ -324,7 +375,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // The product of the step before is complete: these scores were multiplied after it by
         // the same thread, and the commit behind them (s_full) covers everything it had issued.
 #pragma unroll
-        for (int c = 0; c < D; c += 32) {
+        for (int c = 0; c < DV; c += 32) {
           unsigned v[32];
           tc_load32(tmem_o + c, v);
 #pragma unroll
@@ -344,8 +395,8 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int z0 = max(ctx, kb) - kb, z1 = min(stale_hi, kb + AT3_BK) - kb;
         if (r >= z0 && r < z1) {
 #pragma unroll
-          for (int hf = 0; hf < HALVES; ++hf) {
-            const unsigned row = v_smem + s * TILE_BYTES + hf * AT3_HALF + (unsigned)r * 128;
+          for (int hf = 0; hf < V_HALVES; ++hf) {
+            const unsigned row = v_smem + s * V_BYTES + hf * AT3_HALF + (unsigned)r * 128;
 #pragma unroll
             for (int c = 0; c < 128; c += 16)
               asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(row + c), "r"(0u) : "memory");
@@ -369,7 +420,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
         for (int i = 0; i < 64; i += 2) {
           float a0, a1;
-          at3_fma2(a0, a1, sv[c + i], sv[c + i + 1], sc, neg_mr);           // -inf stays -inf
+          at3_fma2(a0, a1, sv[c + i], sv[c + i + 1], X ? 1.f : sc, neg_mr);           // -inf stays -inf
           const float p0 = fast_exp2(a0), p1 = fast_exp2(a1);               // 2^-inf = 0
           at3_add2(sums[i & 2], sums[(i & 2) + 1], p0, p1);
           __nv_bfloat162 pr = __floats2bfloat162_rn(p0, p1);
@@ -390,24 +441,19 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (!ok && lane == 0) { atomicExch(args.status, AT3_ERR_SOFTMAX); atomicExch(&abort_s, 1); }
     tc_fence_after();
     if (ok && !*(volatile int*)&abort_s) {
+      if (X && a.sink && m_ref != -INFINITY) l += fast_exp2(fminf(a.sink[h0 + t] * AT3_LOG2E - m_ref, 120.f));
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* o = (__nv_bfloat16*)a.out + (size_t)(t0 + q0 + r) * a.nh * D + (size_t)(h0 + t) * D;
+      const size_t at = (size_t)(t0 + q0 + r) * a.nh * DV + (size_t)(h0 + t) * DV;
 #pragma unroll
-      for (int c = 0; c < D; c += 32) {
+      for (int c = 0; c < DV; c += 32) {
         unsigned v[32];
         tc_load32(tmem_o + c, v);
         if (row_ok) {
+          float f[32];
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 pk;
-            __nv_bfloat162 t0v = __floats2bfloat162_rn(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv);
-            __nv_bfloat162 t1v = __floats2bfloat162_rn(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
-            __nv_bfloat162 t2v = __floats2bfloat162_rn(__uint_as_float(v[i + 4]) * inv, __uint_as_float(v[i + 5]) * inv);
-            __nv_bfloat162 t3v = __floats2bfloat162_rn(__uint_as_float(v[i + 6]) * inv, __uint_as_float(v[i + 7]) * inv);
-            pk.x = *reinterpret_cast<unsigned*>(&t0v); pk.y = *reinterpret_cast<unsigned*>(&t1v);
-            pk.z = *reinterpret_cast<unsigned*>(&t2v); pk.w = *reinterpret_cast<unsigned*>(&t3v);
-            *reinterpret_cast<uint4*>(o + c + i) = pk;
-          }
+          for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) * inv;
+          if (X && a.out_f32) store_row32((float*)a.out + at + c, f, 32);
+          else store_row32((__nv_bfloat16*)a.out + at + c, f, 32);
         }
       }
     }
@@ -423,22 +469,32 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 // ---------------------------------------------------------------- host side
 // Registers the kernel is given at launch, times its threads: what the two setmaxnreg numbers
 // must fit into.  0 if the kernel cannot be asked.
-template <int D> static int at3_register_pool() {
+template <int D, int DV, bool X> static int at3_register_pool() {
   static int pool = -1;
   if (pool < 0) {
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, attn_prefill_tc3_kernel<D>) != cudaSuccess) { (void)cudaGetLastError(); pool = 0; }
+    if (cudaFuncGetAttributes(&fa, attn_prefill_tc3_kernel<D, DV, X>) != cudaSuccess) { (void)cudaGetLastError(); pool = 0; }
     else pool = fa.numRegs * AT3_THREADS;
   }
   return pool;
 }
 
+static bool at3_shape(int dtype, int d, int page_size, int nh, int nkv) {
+  return dtype == GG_BF16 && (d == 64 || d == 128) && page_size >= 8 && page_size <= AT3_BK && (page_size & (page_size - 1)) == 0 &&
+         nkv > 0 && nh % nkv == 0 && (nh / nkv) % 2 == 0;
+}
+
 bool attn_tc3_supported(int dtype, int d, int page_size, int nh, int nkv) {
-  if (!(dtype == GG_BF16 && (d == 64 || d == 128) && page_size >= 8 && page_size <= AT3_BK &&
-        (page_size & (page_size - 1)) == 0 && nkv > 0 && nh % nkv == 0 && (nh / nkv) % 2 == 0))
-    return false;
+  if (!at3_shape(dtype, d, page_size, nh, nkv)) return false;
   // a softmax group that asks for more registers than the CTA was given would wait for ever
-  return (d == 128 ? at3_register_pool<128>() : at3_register_pool<64>()) >= AT3_POOL;
+  return (d == 128 ? at3_register_pool<128, 128, false>() : at3_register_pool<64, 64, false>()) >= AT3_POOL;
+}
+
+bool attn_tc3_x_supported(int dtype, int d, int dv, int page_size, int nh, int nkv) {
+  if (!at3_shape(dtype, d, page_size, nh, nkv) || (dv != 64 && dv != 128)) return false;
+  const int pool = d == 128 ? (dv == 128 ? at3_register_pool<128, 128, true>() : at3_register_pool<128, 64, true>())
+                            : (dv == 128 ? at3_register_pool<64, 128, true>() : at3_register_pool<64, 64, true>());
+  return pool >= AT3_POOL;
 }
 
 static int encode3(CUtensorMap* map, const void* ptr, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
@@ -453,13 +509,31 @@ static int encode3(CUtensorMap* map, const void* ptr, int rank, const cuuint64_t
   return GG_OK;
 }
 
-// a.tile_seq / a.tile_q0 list tiles of 128 query rows.  T = rows of the q buffer.
-int attn_prefill_tc3(const AttnArgs& a, int num_tiles, int T, int num_pages, int* status, cudaStream_t stream) {
+template <int D, int DV, bool X>
+static int at3_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const At3Args& args, int num_tiles,
+                      cudaStream_t stream) {
+  const size_t smem = (size_t)(4 * (D / 64) + 2 * (DV / 64)) * AT3_HALF + 1024;   // 2 Q, 2 K, 2 V
+  static bool set = false;
+  if (!set) {
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc3_kernel<D, DV, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "attn_prefill_tc3: %s", cudaGetErrorString(e));
+    set = true;
+  }
+  cudaError_t e = gg_launch(attn_prefill_tc3_kernel<D, DV, X>, dim3(args.a.nh / 2, num_tiles), dim3(AT3_THREADS), smem, stream, map_q,
+                            map_k, map_v, args);
+  if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "attn_prefill_tc3: launch: %s", cudaGetErrorString(e));
+  return gg_check_launch("attn_prefill_tc3");
+}
+
+// a.tile_seq / a.tile_q0 list tiles of 128 query rows.  T = rows of the q buffer.  `x`: with the options of the general path.
+int attn_prefill_tc3(const AttnArgs& a, int num_tiles, int T, int num_pages, int* status, bool x, cudaStream_t stream) {
+  const int dv = x && a.dv > 0 ? a.dv : a.d, nv = x && a.v_share > 1 ? a.nkv / a.v_share : a.nkv;
   GG_REQUIRE(num_tiles >= 0 && num_tiles <= 65535, "attn_prefill_tc3: %d tiles in one launch", num_tiles);
   GG_REQUIRE(status != nullptr, "attn_prefill_tc3: no status word given");
   GG_REQUIRE(a.q_stride % 8 == 0 && ((size_t)a.q % 16) == 0, "attn_prefill_tc3: q rows must be 16-byte aligned");
   GG_REQUIRE((a.nh / a.nkv) % 2 == 0, "attn_prefill_tc3: %d heads per kv head; pairs of heads must share a kv head", a.nh / a.nkv);
-  GG_REQUIRE(attn_tc3_supported(GG_BF16, a.d, a.page_size, a.nh, a.nkv), "attn_prefill_tc3: not for this shape or build");
+  GG_REQUIRE(x ? attn_tc3_x_supported(GG_BF16, a.d, dv, a.page_size, a.nh, a.nkv) : attn_tc3_supported(GG_BF16, a.d, a.page_size, a.nh, a.nkv),
+             "attn_prefill_tc3: not for this shape or build");
   if (num_tiles == 0) return GG_OK;
   CUtensorMap map_q, map_k, map_v;
   {
@@ -469,42 +543,22 @@ int attn_prefill_tc3(const AttnArgs& a, int num_tiles, int T, int num_pages, int
     int rc = encode3(&map_q, a.q, 2, dims, strides, box);
     if (rc) return rc;
   }
-  {
-    const cuuint64_t D = (cuuint64_t)a.d;
-    cuuint64_t dims[4] = {D, (cuuint64_t)a.page_size, (cuuint64_t)a.nkv, (cuuint64_t)num_pages};
-    cuuint64_t strides[3] = {D * 2, (cuuint64_t)a.page_size * D * 2, (cuuint64_t)a.nkv * a.page_size * D * 2};
+  for (int which = 0; which < 2; ++which) {
+    const cuuint64_t D = (cuuint64_t)(which ? dv : a.d), heads = (cuuint64_t)(which ? nv : a.nkv);
+    cuuint64_t dims[4] = {D, (cuuint64_t)a.page_size, heads, (cuuint64_t)num_pages};
+    cuuint64_t strides[3] = {D * 2, (cuuint64_t)a.page_size * D * 2, heads * a.page_size * D * 2};
     cuuint32_t box[4] = {64, (cuuint32_t)a.page_size, 1, 1};
-    int rc = encode3(&map_k, a.kcache, 4, dims, strides, box);
-    if (rc) return rc;
-    rc = encode3(&map_v, a.vcache, 4, dims, strides, box);
+    int rc = encode3(which ? &map_v : &map_k, which ? a.vcache : a.kcache, 4, dims, strides, box);
     if (rc) return rc;
   }
   At3Args args;
   args.a = a;
   args.num_pages = num_pages;
   args.status = status;
-  const size_t halves = (size_t)(a.d / 64);
-  const size_t smem = 6 * halves * AT3_HALF + 1024;   // 2 Q, 2 K, 2 V
-  cudaError_t e;
-  if (a.d == 128) {
-    static bool set = false;
-    if (!set) {
-      e = cudaFuncSetAttribute(attn_prefill_tc3_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "attn_prefill_tc3: %s", cudaGetErrorString(e));
-      set = true;
-    }
-    e = gg_launch(attn_prefill_tc3_kernel<128>, dim3(a.nh / 2, num_tiles), dim3(AT3_THREADS), smem, stream, map_q,
-                  map_k, map_v, args);
-  } else {
-    static bool set = false;
-    if (!set) {
-      e = cudaFuncSetAttribute(attn_prefill_tc3_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "attn_prefill_tc3: %s", cudaGetErrorString(e));
-      set = true;
-    }
-    e = gg_launch(attn_prefill_tc3_kernel<64>, dim3(a.nh / 2, num_tiles), dim3(AT3_THREADS), smem, stream, map_q,
-                  map_k, map_v, args);
-  }
-  if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "attn_prefill_tc3: launch: %s", cudaGetErrorString(e));
-  return gg_check_launch("attn_prefill_tc3");
+  if (!x) return a.d == 128 ? at3_launch<128, 128, false>(map_q, map_k, map_v, args, num_tiles, stream)
+                            : at3_launch<64, 64, false>(map_q, map_k, map_v, args, num_tiles, stream);
+  if (a.d == 128) return dv == 128 ? at3_launch<128, 128, true>(map_q, map_k, map_v, args, num_tiles, stream)
+                                   : at3_launch<128, 64, true>(map_q, map_k, map_v, args, num_tiles, stream);
+  return dv == 128 ? at3_launch<64, 128, true>(map_q, map_k, map_v, args, num_tiles, stream)
+                   : at3_launch<64, 64, true>(map_q, map_k, map_v, args, num_tiles, stream);
 }

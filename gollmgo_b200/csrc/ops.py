@@ -782,7 +782,8 @@ def attn_prefill_x(q: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache:
                    head_bias: Optional[torch.Tensor] = None, dist_bias: Optional[torch.Tensor] = None,
                    dist_bucket: Optional[torch.Tensor] = None, chunk: int = 0,
                    sink: Optional[torch.Tensor] = None, slopes: Optional[torch.Tensor] = None,
-                   temperature=None) -> None:
+                   temperature=None, tile128_seq: Optional[torch.Tensor] = None, tile128_q0: Optional[torch.Tensor] = None,
+                   num_tiles128: int = 0) -> None:
     """Causal attention of prompt portions with keys of size d, values of size dv, ``v_share`` key
     heads to a value head, optional window and capped scores; out [T, nh*dv] in the cache's type or
     float32.  ``tile_*`` list tiles of 16 queries (general kernel, float32 arithmetic), ``tile64_*``
@@ -795,11 +796,19 @@ def attn_prefill_x(q: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache:
     only the keys of its own chunk of that many positions (chunks counted from position 0 of the
     sequence); ``sink`` [nh] float32: exp(sink[h]) is added to the softmax denominator of head h;
     ``slopes`` [nh] float32: slopes[h] * (i - j) is taken off the scaled score; ``temperature`` (coef, every):
-    the query at position p is multiplied by 1 + coef * ln(floor((p + 1) / every) + 1)."""
+    the query at position p is multiplied by 1 + coef * ln(floor((p + 1) / every) + 1).  ``tile128_*`` list tiles of
+    128 queries (tcgen05 kernel: bfloat16, d and dv 64 or 128, even groups of heads, softmax weights without kept keys or a
+    distance table); where given and possible it runs."""
+    global tc_launched
     _attn_extras(nh, head_bias, dist_bias, dist_bucket, sink, slopes)
+    use_tc = tile128_seq is not None and kcache.dtype == torch.bfloat16
+    if use_tc:
+        tc_launched = True
     _check(lib().gg_attn_prefill_x(_p(q), ctypes.c_longlong(q_stride), _p(kcache), _p(vcache), dtype_code(kcache.dtype),
                                    _p(block_tables), bt_stride, _p(cu_q_lens), _p(context_lens), _p(tile_seq),
                                    _p(tile_q0), num_tiles, _p(tile64_seq), _p(tile64_q0), num_tiles64, int(allow_mma),
+                                   _p(tile128_seq if use_tc else None), _p(tile128_q0 if use_tc else None), num_tiles128,
+                                   q.shape[0], kcache.shape[0], _p(tc_status(q.device)) if use_tc else ctypes.c_void_p(0),
                                    _p(out), int(out.dtype == torch.float32 and kcache.dtype != torch.float32),
                                    nh, nkv, d, dv, v_share, page_size, window, ctypes.c_float(scale),
                                    ctypes.c_float(softcap), int(keep_first), int(sigmoid_weights), _p(head_bias),

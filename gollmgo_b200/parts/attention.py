@@ -221,6 +221,8 @@ class Attention:
         if self.general:
             if self._mma_x:
                 need.append(TILES_MMA_X)
+                if ATTN_POLICY == "auto":
+                    need.append(TILES_TC)
             return need
         if self.ctx.act_dtype == torch.bfloat16 and self.d in (64, 128) and ATTN_POLICY != "general":
             need.append(TILES_MMA)
@@ -231,6 +233,15 @@ class Attention:
     def _splits(self, n_dec: int, max_context: int) -> int:
         return decode_splits(n_dec, self._ctas_per_split, self.num_sms, self._cluster_cap,
                              context_tiles(max_context, self.window), self._tile_bytes)
+
+    def long_tiles(self, batch):
+        """The tiles of 128 query rows for a prompt step of the general path that runs on tcgen05 (ops.attn_prefill_x), as its
+        arguments; empty where the mma.sync kernel is the faster one (_few_short_tiles; at least two heads must share a kv
+        head for the other kernel to take the step at all)."""
+        t128 = batch.tiles.get(TILES_TC) if self._mma_x else None
+        if t128 is None or self._few_short_tiles(t128.count, batch):
+            return {}
+        return dict(tile128_seq=t128.seq, tile128_q0=t128.q0, num_tiles128=t128.count)
 
     def _few_short_tiles(self, tiles128: int, batch) -> bool:
         """Prompt portions that leave the tcgen05 kernel's tiles (128 rows of two heads) on fewer
@@ -360,7 +371,7 @@ class Attention:
                                t16.seq, t16.q0, t16.count, out, self.nh, self.nkv, self.d, self.dv, self.v_share,
                                self.ctx.page_size, window, self.scale, self.softcap,
                                t64.seq if t64 else None, t64.q0 if t64 else None, t64.count if t64 else 0,
-                               allow_mma=t64 is not None, **more)
+                               allow_mma=t64 is not None, **more, **self.long_tiles(batch))
         if batch.num_decode:
             n = batch.num_decode
             facts = getattr(batch, "facts", None)

@@ -26,7 +26,7 @@ import torch
 from ..cache import PagedKVNeed
 from ..csrc import ops
 from ..weights import WeightSpec
-from .attention import ATTN_POLICY, TILES_GENERAL, TILES_MMA_X, Attention, context_tiles, decode_splits
+from .attention import ATTN_POLICY, TILES_GENERAL, TILES_MMA_X, TILES_TC, Attention, context_tiles, decode_splits
 from .linear import linear
 from .registry import register_mixer
 
@@ -73,7 +73,8 @@ class NormedAttention(Attention):
         return PagedKVNeed(self.nkv, self.d, self.window, v_heads=self.nv, v_head_dim=self.dv)
 
     def query_tiles(self):
-        return [TILES_GENERAL, TILES_MMA_X] if self._mma_x else [TILES_GENERAL]
+        need = [TILES_GENERAL, TILES_MMA_X] if self._mma_x else [TILES_GENERAL]
+        return need + [TILES_TC] if self._mma_x and ATTN_POLICY == "auto" else need
 
     def _splits(self, n_dec, max_context):
         return decode_splits(n_dec, self._ctas_per_split, self.num_sms, self._cluster_cap,
@@ -145,7 +146,7 @@ class NormedAttention(Attention):
                                t16.seq, t16.q0, t16.count, out, self.nh, self.nkv, self.d, self.dv, 1,
                                self.ctx.page_size, window, self.scale, 0.0,
                                t64.seq if t64 else None, t64.q0 if t64 else None, t64.count if t64 else 0,
-                               allow_mma=t64 is not None, **more)
+                               allow_mma=t64 is not None, **more, **self.long_tiles(batch))
         if batch.num_decode:
             n = batch.num_decode
             facts = getattr(batch, "facts", None)
