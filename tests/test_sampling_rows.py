@@ -1,0 +1,65 @@
+"""The sampling kernel with a row on one multiprocessor (csrc/sampling.cu): every way it finds its thresholds, against
+probabilities in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from gollmgo_b200.csrc import ops
+    return ops
+
+
+def kept_probabilities(row, t, k, p):
+    """Probabilities of the values that top-k and top-p leave (ties at a threshold all stay)."""
+    x = row.double() / t
+    if 0 < k < x.numel():
+        x = x.masked_fill(x < x.topk(k).values[-1], -float("inf"))
+    q = torch.softmax(x, 0)
+    if 0 < p < 1:
+        s, order = q.sort(descending=True)
+        n = int((s.cumsum(0) < p - 1e-12).sum()) + 1
+        q = torch.where(x >= x[order[n - 1]], q, torch.zeros_like(q))
+        q = q / q.sum()
+    return q
+
+
+# vocabulary, rows, spread of the logits, (top_k, top_p) in turn: candidates above the threads' maxima; more than there are
+# threads; a leading byte that fits in shared memory, does not fit (flat logits) or fits only where few rows share it;
+# odd widths (rows that start off a 16-byte border); fewer values than threads; rows whose integer sums need 64 bits
+CASES = [(40000, 40, 2.5, [(50, 0.9), (1024, 0.0), (1025, 0.8), (3000, 0.95), (0, 0.9), (0, 0.0), (1, 0.5)]),
+         (128256, 40, 2.5, [(0, 0.9), (400, 0.8), (0, 0.99), (20000, 0.5)]),
+         (128256, 150, 0.4, [(0, 0.9), (400, 0.8), (0, 0.5)]),
+         (60000, 40, 0.01, [(0, 0.9), (7, 0.9), (2000, 0.9)]),
+         (16389, 60, 2.5, [(0, 0.9), (50, 0.0), (0, 0.0), (50, 0.7)]),
+         (301, 5, 1.0, [(0, 0.9), (300, 0.7), (20, 0.0), (301, 0.4)]),
+         (300000, 38, 1.5, [(0, 0.9), (100, 0.9), (5000, 0.6)])]
+
+
+@pytest.mark.parametrize("V,R,std,ways", CASES)
+def test_tokens_lie_where_the_draw_does(ops, V, R, std, ways):
+    gen = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(R, V, device="cuda", generator=gen) * std
+    logits[1] = torch.round(logits[1] * 4) / 4 + 0.0          # many ties (the kernels order -0 below 0, so there is none of it)
+    logits[2, ::3] = -float("inf")
+    dev = lambda x, dt: torch.tensor(x, dtype=dt, device="cuda")  # noqa: E731
+    temps = [0.7 + 0.1 * (r % 4) for r in range(R)]
+    ks, ps = [ways[r % len(ways)][0] for r in range(R)], [ways[r % len(ways)][1] for r in range(R)]
+    args = (dev(temps, torch.float32), dev(ks, torch.int32), dev(ps, torch.float32), dev(list(range(R)), torch.int64), dev([3] * R, torch.int64))
+    out, again = (torch.empty(R, dtype=torch.int32, device="cuda") for _ in range(2))
+    ops.sample(logits, *args, out)
+    ops.sample(logits, *args, again)
+    assert torch.equal(out, again)
+    mask = (1 << 64) - 1
+    for r in range(R):
+        z = (r + 4 * 0x9E3779B97F4A7C15) & mask
+        z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & mask
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+        u = ((z ^ (z >> 31)) >> 40) / 2.0 ** 24
+        q = kept_probabilities(logits[r], float(torch.tensor(temps[r], dtype=torch.float32)), ks[r], float(torch.tensor(ps[r], dtype=torch.float32)))
+        cum, got = q.cumsum(0), int(out[r])
+        # float32 sums of up to 3e5 weights: the draw may fall on a neighbour within 1e-4 of a border
+        assert q[got] > 0 or ps[r] > 0, (r, got)
+        assert float(cum[got] - q[got]) - 1e-4 <= u <= float(cum[got]) + 1e-4, (r, got)
