@@ -10,6 +10,7 @@ from __future__ import annotations
 
 from typing import List, Sequence
 
+import numpy as np
 import torch
 
 from ..csrc import ops
@@ -52,13 +53,17 @@ class Sampler:
         if all(p.greedy for p in params):
             ops.argmax(logits, out)
         else:
-            dev = self.device
-            temps = torch.tensor([p.temperature for p in params], dtype=torch.float32).to(dev, non_blocking=True)
-            top_k = torch.tensor([p.top_k for p in params], dtype=torch.int32).to(dev, non_blocking=True)
-            top_p = torch.tensor([p.top_p for p in params], dtype=torch.float32).to(dev, non_blocking=True)
-            seeds = torch.tensor([_as_i64(p.seed or 0) for p in params], dtype=torch.int64).to(dev, non_blocking=True)
-            draws = torch.tensor(list(draw_index), dtype=torch.int64).to(dev, non_blocking=True)
-            ops.sample(logits, temps, top_k, top_p, seeds, draws, out)
+            # one buffer, one copy: [seeds | draws] of 64 bits, then [top_k], [temperature], [top_p] of 32
+            host = np.empty(7 * R, dtype=np.int32)
+            wide, f32 = host[:4 * R].view(np.int64), host[5 * R:].view(np.float32)
+            wide[:R] = [_as_i64(p.seed or 0) for p in params]
+            wide[R:] = draw_index
+            host[4 * R:5 * R] = [p.top_k for p in params]
+            f32[:R] = [p.temperature for p in params]
+            f32[R:] = [p.top_p for p in params]
+            dev = torch.from_numpy(host).to(self.device, non_blocking=True)
+            wide, f32 = dev[:4 * R].view(torch.int64), dev[5 * R:].view(torch.float32)
+            ops.sample(logits, f32[:R], dev[4 * R:5 * R], f32[R:], wide[:R], wide[R:], out)
         self._host[slot][:R].copy_(out, non_blocking=True)
         self._events[slot].record()
         return (slot, R)
