@@ -206,7 +206,7 @@ template <int DPT, bool CH, bool DELTA, int NC>
 __global__ void __launch_bounds__(DR_COLS * DR_LANES)
 delta_recur_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
                    float* __restrict__ state, const int* __restrict__ cu_q_lens, const int* __restrict__ context_lens,
-                   const int* __restrict__ state_slots, int G, int H, int d, int dv, float* __restrict__ o_raw) {
+                   const int* __restrict__ state_slots, int G, int H, int d, int dv, int max_len, float* __restrict__ o_raw) {
   extern __shared__ __align__(16) float sm[];
   constexpr int CC = DR_COLS * NC;               // columns of the CTA
   const int b = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CC;
@@ -214,7 +214,7 @@ delta_recur_kernel(const float* __restrict__ qkv, const float* __restrict__ beta
   const int C = 2 * G * d + H * dv;
   const int slot = state_slots[b];
   const int t0 = cu_q_lens[b], qlen = cu_q_lens[b + 1] - t0;
-  if (slot < 0 || qlen <= 0) { pdl_trigger(); return; }
+  if (slot < 0 || qlen <= 0 || qlen > max_len) { pdl_trigger(); return; }
   const int start = context_lens[b] - qlen;
   const int kvh = h / (H / G);
   const int dp = DPT * DR_LANES;                 // d rounded up to what the lanes hold
@@ -528,7 +528,7 @@ extern "C" int gg_delta_prep(const void* x, long long x_stride, int dtype, const
 template <int DPT, bool CH, bool DELTA, int NC>
 static int delta_recur_launch(const float* qkv, const float* beta, const float* decay, float* state,
                               const int* cu_q_lens, const int* context_lens, const int* state_slots, int B, int G, int H,
-                              int d, int dv, float* o_raw, bool long_rows, cudaStream_t stream) {
+                              int d, int dv, int max_len, float* o_raw, bool long_rows, cudaStream_t stream) {
   const int dp = DPT * DR_LANES;
   const size_t smem = (size_t)(2 * DR_STAGE_FLOATS_X(dp, CH, NC) + DR_CHUNK * DR_COLS * NC * DR_LANES) * sizeof(float);
   if (smem > 48 * 1024) {
@@ -540,17 +540,19 @@ static int delta_recur_launch(const float* qkv, const float* beta, const float* 
   // empty machine (measured on a prompt of 2048 tokens with 128 blocks: 857 us launched early, 463 us so).
   if (long_rows)
     gg_launch_after(delta_recur_kernel<DPT, CH, DELTA, NC>, grid, dim3(DR_COLS * DR_LANES), smem, stream, qkv, beta, decay, state,
-                    cu_q_lens, context_lens, state_slots, G, H, d, dv, o_raw);
+                    cu_q_lens, context_lens, state_slots, G, H, d, dv, max_len, o_raw);
   else
     gg_launch(delta_recur_kernel<DPT, CH, DELTA, NC>, grid, dim3(DR_COLS * DR_LANES), smem, stream, qkv, beta, decay, state, cu_q_lens,
-              context_lens, state_slots, G, H, d, dv, o_raw);
+              context_lens, state_slots, G, H, d, dv, max_len, o_raw);
   return gg_check_launch("delta_recur");
 }
 
+// max_len > 0: sequences with more tokens in this step are left alone.
 extern "C" int gg_delta_recur(const float* qkv, const float* beta, const float* decay, float* state,
                               const int* cu_q_lens, const int* context_lens, const int* state_slots, int B, int G, int H,
-                              int d, int dv, int dw, int plain, int T, float* o_raw, cudaStream_t stream) {
-  const bool long_rows = T > 4 * B;              // more than a few tokens a sequence: a step with prompt portions
+                              int d, int dv, int dw, int plain, int max_len, int T, float* o_raw, cudaStream_t stream) {
+  const bool long_rows = T > 4 * B && max_len != 1;
+  if (max_len <= 0) max_len = T;              // more than a few tokens a sequence: a step with prompt portions
   GG_REQUIRE(dw == 1 || dw == d, "delta_recur: a decay per head (1) or per key channel (%d), not %d", d, dw);
   GG_REQUIRE(!plain || dw == 1, "delta_recur: the plain recurrence takes a decay per head");
   GG_REQUIRE(B > 0 && G > 0 && H > 0 && H % G == 0 && d > 0 && dv > 0, "delta_recur: bad sizes B=%d G=%d H=%d d=%d dv=%d", B, G, H, d, dv);
@@ -559,10 +561,10 @@ extern "C" int gg_delta_recur(const float* qkv, const float* beta, const float* 
 #define DR_GO(N)                                                                                                              \
   do {                                                                                                                        \
     if (plain && N <= 16 && dv % (2 * DR_COLS) == 0)                                                                          \
-      return delta_recur_launch<N, false, false, (N <= 16 ? 2 : 1)>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, o_raw, long_rows, stream); \
-    if (plain) return delta_recur_launch<N, false, false, 1>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, o_raw, long_rows, stream); \
-    if (dw > 1) return delta_recur_launch<N, true, true, 1>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, o_raw, long_rows, stream); \
-    return delta_recur_launch<N, false, true, 1>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, o_raw, long_rows, stream); \
+      return delta_recur_launch<N, false, false, (N <= 16 ? 2 : 1)>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, max_len, o_raw, long_rows, stream); \
+    if (plain) return delta_recur_launch<N, false, false, 1>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, max_len, o_raw, long_rows, stream); \
+    if (dw > 1) return delta_recur_launch<N, true, true, 1>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, max_len, o_raw, long_rows, stream); \
+    return delta_recur_launch<N, false, true, 1>(qkv, beta, decay, state, cu_q_lens, context_lens, state_slots, B, G, H, d, dv, max_len, o_raw, long_rows, stream); \
   } while (0)
   if (d <= 16) DR_GO(2);
   if (d <= 32) DR_GO(4);

@@ -957,18 +957,77 @@ def delta_prep(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, 
 
 def delta_recur(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                 cu_q_lens: torch.Tensor, context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int,
-                kv_heads: int, heads: int, d: int, dv: int, o_raw: torch.Tensor, plain: bool = False) -> None:
+                kv_heads: int, heads: int, d: int, dv: int, o_raw: torch.Tensor, plain: bool = False,
+                max_len: int = 0) -> None:
     """The recurrence S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q over every sequence's
     tokens of the step, from and to state [slots, heads, dv, d] float32.  decay [T, heads]: g is a
     number per head; [T, heads * d]: a factor per key channel (row of S).  ``plain``: u = beta v (the
-    write does not look at the state: the recurrence of a state-space layer)."""
+    write does not look at the state: the recurrence of a state-space layer).  ``max_len`` > 0: sequences with more
+    tokens in this step are left alone."""
     _cuda(qkv, beta, decay, state, o_raw)
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, d):
         raise KernelError("delta_recur: state must be float32 [slots, heads, dv, d]")
     dw = decay.shape[-1] // heads
     _check(lib().gg_delta_recur(_p(qkv), _p(beta), _p(decay), _p(state), _p(cu_q_lens), _p(context_lens),
-                                _p(state_slots), num_seqs, kv_heads, heads, d, dv, dw, int(plain), o_raw.shape[0], _p(o_raw),
+                                _p(state_slots), num_seqs, kv_heads, heads, d, dv, dw, int(plain), int(max_len), o_raw.shape[0], _p(o_raw),
                                 _stream()))
+
+
+LINEAR_CHUNK = 128            # tokens of a chunk (csrc/linear_chunks.cu)
+
+
+def linear_chunks_ok(d: int, dv: int) -> bool:
+    """Whether linear_chunks takes keys of d and values of dv."""
+    return d % 8 == 0 and d <= 256 and dv % 4 == 0 and dv <= 256
+
+
+def linear_scratch_floats(num_tokens: int, num_seqs: int, heads: int, d: int, dv: int) -> int:
+    return (num_tokens // LINEAR_CHUNK + num_seqs + 1) * heads * (d * dv + 4)         # a state and a factor per chunk and head
+
+
+def linear_chunks(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
+                  tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
+                  context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, kv_heads: int, heads: int, d: int,
+                  dv: int, o_raw: torch.Tensor) -> bool:
+    """delta_recur(plain=True) over the sequences with more than one token in this step, a chunk of LINEAR_CHUNK tokens at a
+    time (tile_seq, tile_q0: the chunks); the others are left alone.  scratch: float32 of linear_scratch_floats().
+    False, and nothing done, where sizes or addresses are not for these kernels."""
+    _cuda(qkv, beta, decay, state, scratch, o_raw)
+    if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, d) or decay.shape[-1] != heads \
+            or qkv.dtype != torch.float32 or scratch.dtype != torch.float32:
+        raise KernelError("linear_chunks: float32 rows, scratch and state [slots, heads, dv, d], a decay per head")
+    global tc_launched
+    rc = lib().gg_linear_chunks(_p(qkv), _p(beta), _p(decay), _p(state), _p(scratch), ctypes.c_longlong(scratch.numel()), _p(tile_seq),
+                                _p(tile_q0), num_tiles, _p(cu_q_lens), _p(context_lens), _p(state_slots), o_raw.shape[0], num_seqs,
+                                kv_heads, heads, d, dv, _p(o_raw), _p(tc_status(o_raw.device)), _stream())
+    if rc == 3:                                            # GG_ERR_UNSUPPORTED
+        return False
+    _check(rc, 3)
+    tc_launched = True
+    return True
+
+
+def linear_retention(rows: torch.Tensor, log2_decay: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
+                     tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
+                     context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, gate: torch.Tensor, eps: float,
+                     heads: int, d: int, dv: int, out: torch.Tensor) -> bool:
+    """retention_chunks on the kernels of linear_chunks: tiles of LINEAR_CHUNK rows, scratch float32 of
+    linear_scratch_floats().  False, and nothing done, where sizes or addresses are not for these kernels."""
+    global tc_launched
+    _cuda(rows, log2_decay, state, scratch, tile_seq, tile_q0, out)
+    if rows.dtype != torch.float32 or rows.shape[1] != heads * (2 * d + dv) or log2_decay.dtype != torch.float32 \
+            or log2_decay.numel() != heads or state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, d) \
+            or scratch.dtype != torch.float32 or gate.stride(1) != 1 or gate.dtype != out.dtype:
+        raise KernelError("linear_retention: float32 rows, decays, state [slots, heads, dv, d] and scratch; gate of the output's dtype")
+    rc = lib().gg_linear_retention(_p(rows), _p(log2_decay), _p(state), _p(scratch), ctypes.c_longlong(scratch.numel()), _p(tile_seq),
+                                   _p(tile_q0), num_tiles, _p(cu_q_lens), _p(context_lens), _p(state_slots), rows.shape[0], num_seqs,
+                                   _p(gate), ctypes.c_longlong(gate.stride(0)), ctypes.c_float(eps), heads, d, dv,
+                                   dtype_code(out.dtype), _p(out), _p(tc_status(out.device)), _stream())
+    if rc == 3:
+        return False
+    _check(rc, 3)
+    tc_launched = True
+    return True
 
 
 def delta_out(o_raw: torch.Tensor, gate: torch.Tensor, weight: Optional[torch.Tensor], eps: float, heads: int, dv: int,

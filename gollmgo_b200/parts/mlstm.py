@@ -9,7 +9,7 @@ with q = Wq x * d^-1/2, k = Wk x, v = Wv x per head, the log input gate i = cap 
 log forget gate f = logsigmoid(cap tanh((Wf x + bf) / cap)) per head.  Each head's o is divided by its root
 mean square, the heads together are multiplied by a weight and by sigmoid(Wg x), and projected.
 
-The recurrence is the engine's plain linear recurrence (csrc/delta_rule.cu, the form of a state-space layer)
+The recurrence is the engine's plain linear recurrence (parts/linear_recurrence.py)
 with one more value column that is always 1, so that n is a column of S; the gates, the maxima and the
 normaliser are csrc/mlstm.cu.  State per request, in its state slot: S with n in float32
 [heads, dvp, d] (dvp = dv + 1 rounded up to 4) and m [heads].  Nothing is paged.  The gates' product is
@@ -26,6 +26,7 @@ from ..cache import FixedStateNeed
 from ..csrc import ops
 from ..weights import WeightSpec
 from .linear import linear
+from .linear_recurrence import PlainRecurrence
 from .registry import register_mixer
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "i": "i", "f": "f", "gate": "g", "o": "o", "norm": "norm"}
@@ -61,10 +62,14 @@ class MatrixMemory:
         ws.reserve("mlstm_o", T * self.nh * self.dvp, torch.float32)
         ws.reserve("mlstm_y", T * self.nh * self.dv, ctx.act_dtype)
         ws.reserve(self.out_buffer, T * self.hidden, ctx.act_dtype)
+        self.recurrence = PlainRecurrence(ctx, self.nh, self.nh, self.d, self.dvp)
         self.w_proj = self.w_if = self.b_i = self.b_f = self.norm_w = self.w_o = None
 
     def cache_need(self):
         return (FixedStateNeed((self.nh, self.dvp, self.d), "float32"), FixedStateNeed((self.nh,), "float32"))
+
+    def query_tiles(self):
+        return self.recurrence.query_tiles()
 
     def weights(self):
         n, H, qk, vv = self.names, self.hidden, self.nh * self.d, self.nh * self.dv
@@ -101,8 +106,7 @@ class MatrixMemory:
         rows = ws.get("mlstm_rows", T, self.rows_width)
         ops.mlstm_rows(proj, H, self.d, self.dv, self.dvp, self.d ** -0.5, rows)
         o = ws.get("mlstm_o", T, H * self.dvp)
-        ops.delta_recur(rows, beta, decay, state, batch.cu_q_lens, batch.context_lens, batch.state_slots, B,
-                        H, H, self.d, self.dvp, o, plain=True)
+        self.recurrence.run(rows, beta, decay, state, batch, o)
         y = ws.get("mlstm_y", T, H * self.dv)
         ops.mlstm_out(o, m_row, proj[:, self.gate_col:self.gate_col + H * self.dv], self.norm_w, self.eps, self.floor,
                       H, self.dv, self.dvp, y)

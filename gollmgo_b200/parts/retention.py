@@ -27,7 +27,12 @@ from .context import QueryTiles
 from .linear import linear
 from .registry import build_position, register_mixer
 
-CHUNKS = QueryTiles(ops.RETENTION_CHUNK)          # the chunks of prompt portions
+CHUNKS = QueryTiles(ops.RETENTION_CHUNK)          # the chunks of prompt portions: of the packed float32 kernels,
+TC_CHUNKS = QueryTiles(ops.LINEAR_CHUNK)          # and of the tensor-core ones (sizes that linear_chunks_ok names)
+# Steps with so many prompt tokens take the tensor-core kernels (a B200, 16 heads 128 x 256, us for a layer, tensor cores and
+# packed float32: one sequence of 16: 43 and 39, of 65: 61 and 55, of 128: 70 and 72, of 512: 98 and 108, of 4096: 485 and 610;
+# 8 of 16: 57 and 58, of 64: 93 and 122; 32 of 128: 522 and 617).
+TC_FROM = 128
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "gate": "g", "o": "o"}
 
@@ -64,6 +69,9 @@ class Retention:
         self.decays = torch.tensor(self.decay, dtype=torch.float32, device=ctx.device)
         self.log2_decays = torch.tensor([math.log2(g) for g in self.decay], dtype=torch.float32, device=ctx.device)
         self.chunked = self.dv <= ops.RETENTION_MAX_V
+        self.tc = self.chunked and ops.linear_chunks_ok(self.d, self.dv)
+        if self.tc:
+            ws.reserve("linear_states", ops.linear_scratch_floats(T, ctx.max_seqs, self.nh, self.d, self.dv), torch.float32)
         if self.chunked:
             ws.reserve("ret_states", ops.retention_scratch_floats(T, ctx.max_seqs, self.nh, self.d, self.dv), torch.float32)
         else:
@@ -76,7 +84,7 @@ class Retention:
         return FixedStateNeed((self.nh, self.dv, self.d), "float32")
 
     def query_tiles(self):
-        return [CHUNKS] if self.chunked else []
+        return ([CHUNKS] if self.chunked else []) + ([TC_CHUNKS] if self.tc else [])
 
     def weights(self):
         n, H, qk, vv = self.names, self.hidden, self.nh * self.d, self.nh * self.dv
@@ -116,10 +124,17 @@ class Retention:
                 if CHUNKS not in batch.tiles:
                     raise RuntimeError("the step's batch was built without the index list this mixer declares in "
                                        "query_tiles(): give it to the BatchBuilder (query_tiles=...)")
+                seqs = (batch.cu_q_lens, batch.context_lens, batch.state_slots, batch.num_seqs)
+                done, tiles = False, batch.tiles.get(TC_CHUNKS) if self.tc and T - batch.num_decode >= TC_FROM else None
+                if tiles is not None:
+                    scratch = ws.get("linear_states", 1, ops.linear_scratch_floats(T, batch.num_seqs, H, d, dv))
+                    done = ops.linear_retention(rows, self.log2_decays, state, scratch, tiles.seq, tiles.q0, tiles.count, *seqs, gate,
+                                                self.eps, H, d, dv, y)
+            if batch.num_portions and not done:
                 tiles = batch.tiles[CHUNKS]
                 scratch = ws.get("ret_states", 1, ops.retention_scratch_floats(T, batch.num_seqs, H, d, dv))
-                ops.retention_chunks(rows, self.log2_decays, state, scratch, tiles.seq, tiles.q0, tiles.count, batch.cu_q_lens,
-                                     batch.context_lens, batch.state_slots, batch.num_seqs, gate, self.eps, H, d, dv, y)
+                ops.retention_chunks(rows, self.log2_decays, state, scratch, tiles.seq, tiles.q0, tiles.count, *seqs, gate, self.eps, H, d,
+                                     dv, y)
             if batch.num_decode:
                 ops.retention_decode(proj, self.gate_col, batch.positions, table, pairs, self.decays, state, batch.dec_seqs,
                                      batch.num_decode, batch.cu_q_lens, batch.context_lens, batch.state_slots, H, d, dv, kscale,

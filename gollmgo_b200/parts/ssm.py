@@ -11,8 +11,7 @@ weight, and projected back.
 
 State per request, in its state slot: S in float32 [heads, v_head_dim, state] and the last
 taps - 1 inputs of the convolution in float32 [taps - 1, channels].  Nothing is paged.  The
-recurrence is the linear-recurrence kernel of the delta rule without the delta (csrc/delta_rule.cu,
-csrc/ssm.cu); everything between the two products is float32.
+recurrence is the plain linear one (parts/linear_recurrence.py, csrc/ssm.cu); everything between the two products is float32.
 
 params: hidden_size, num_heads, v_head_dim, state, groups, conv (taps), norm_groups, eps, out_buffer,
 names (optional dict: in, conv, conv_bias, dt_bias, A_log, D, norm, o).
@@ -25,6 +24,7 @@ from ..cache import FixedStateNeed
 from ..csrc import ops
 from ..weights import WeightSpec
 from .linear import linear
+from .linear_recurrence import PlainRecurrence
 from .registry import register_mixer
 
 _NAMES = {"in": "in", "conv": "conv", "conv_bias": "conv.b", "dt_bias": "dt_bias", "A_log": "A_log", "D": "D",
@@ -64,6 +64,7 @@ class StateSpaceMixer:
         ws.reserve("ssm_y", T * self.inner, torch.float32)
         ws.reserve("ssm_out", T * self.inner, ctx.act_dtype)
         ws.reserve(self.out_buffer, T * self.hidden, ctx.act_dtype)
+        self.recurrence = PlainRecurrence(ctx, self.groups, self.nh, self.n, self.p)
         self.w_in = self.w_o = self.conv_w = self.conv_b = self.a_log = self.dt_bias = self.d_skip = self.norm_w = None
 
     def cache_need(self):
@@ -71,6 +72,9 @@ class StateSpaceMixer:
         if self.taps > 1:
             need.append(FixedStateNeed((self.taps - 1, self.channels), "float32"))
         return tuple(need)
+
+    def query_tiles(self):
+        return self.recurrence.query_tiles()
 
     def weights(self):
         n = self.names
@@ -109,8 +113,7 @@ class StateSpaceMixer:
                      batch.context_lens, batch.state_slots, B, self.nh, self.p, self.groups, self.n, cbx, dt, decay)
         y = ws.get("ssm_y", T, self.inner)
         # rows [C | B | x] are the recurrence's q, k, v; the step size takes beta's place
-        ops.delta_recur(cbx, dt, decay, state, batch.cu_q_lens, batch.context_lens, batch.state_slots, B,
-                        self.groups, self.nh, self.n, self.p, y, plain=True)
+        self.recurrence.run(cbx, dt, decay, state, batch, y)
         out = ws.get("ssm_out", T, self.inner)
         ops.ssm_out(y, cbx, 2 * self.groups * self.n, proj[:, :self.inner], self.d_skip, self.norm_w, self.eps,
                     self.nh, self.p, self.parts, out)
