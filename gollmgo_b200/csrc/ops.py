@@ -691,14 +691,20 @@ def moe_gather(x: torch.Tensor, order: torch.Tensor, top: int, out: torch.Tensor
 
 def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_group: torch.Tensor, groups: int,
                     gated: bool = False, row_entry: Optional[torch.Tensor] = None,
-                    row_scale: Optional[torch.Tensor] = None, relu2: bool = False) -> None:
+                    row_scale: Optional[torch.Tensor] = None, relu2: bool = False,
+                    clamped: Optional[tuple] = None) -> None:
     """The tcgen05 product (gemm_tc) over groups: rows 128 i .. of x belong to group tile_group[i]
     (< 0: to none, skipped) and are multiplied with that group's matrix w[g] ([groups, N, K]; gated:
     [groups, 2N, K], out = silu(x Wg^T) * (x Wu^T); ``relu2``: out = the square of relu(x W^T)).  bfloat16; rows of x a multiple of 128.  ``row_scale``
-    (gated, float32): the products of row r are multiplied by row_scale[row_entry[r]] before the activation."""
+    (gated, float32): the products of row r are multiplied by row_scale[row_entry[r]] before the activation.  ``clamped``
+    (gated, without row_scale): (limit, alpha, shift) of clamped_gate, which takes silu's place."""
     global tc_launched
     M, K = x.shape
     N = out.shape[1]
+    if clamped is not None and (not gated or row_scale is not None):
+        raise KernelError("gemm_tc_grouped: the clamped activation goes with the gated product without factors on rows")
+    limit, alpha, shift = clamped or (0.0, 0.0, 0.0)
+    mode = 4 if clamped else 2 if gated else 3 if relu2 else 0
     if w.numel() != groups * (2 if gated else 1) * N * K or out.shape[0] != M or not out.is_contiguous() \
             or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise KernelError("gemm_tc_grouped: shapes or dtypes do not fit")
@@ -706,8 +712,9 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_gr
     if row_scale is not None and (row_scale.dtype != torch.float32 or row_entry is None or row_entry.numel() < M):
         raise KernelError("gemm_tc_grouped: float32 factors with a row list as long as x")
     tc_launched = True
-    _check(lib().gg_gemm_tc_grouped(_p(x), ctypes.c_longlong(x.stride(0)), _p(w), _p(out), M, N, K, 2 if gated else 3 if relu2 else 0,
-                                    _p(tile_group), groups, _p(row_entry), _p(row_scale), _p(tc_status(x.device)), _stream()))
+    _check(lib().gg_gemm_tc_grouped(_p(x), ctypes.c_longlong(x.stride(0)), _p(w), _p(out), M, N, K, mode,
+                                    _p(tile_group), groups, _p(row_entry), _p(row_scale), ctypes.c_float(limit), ctypes.c_float(alpha),
+                                    ctypes.c_float(shift), _p(tc_status(x.device)), _stream()))
 
 
 def moe_combine(y: torch.Tensor, place: torch.Tensor, wgt: Optional[torch.Tensor], shared: Optional[torch.Tensor],

@@ -123,7 +123,7 @@ class MixtureOfExperts:
         ws.reserve("moe_in", slots * self.hidden, ctx.act_dtype)
         ws.reserve("moe_act", slots * self.inter, ctx.act_dtype)
         if self.activation == "clamped_swish":
-            ws.reserve("moe_gate_up", slots * 2 * self.inter, ctx.act_dtype)
+            ws.reserve("moe_gate_up", n * 2 * self.inter, ctx.act_dtype)       # (of short steps)
         ws.reserve("moe_rows", slots * self.hidden, ctx.act_dtype)
         ws.reserve("moe_out", T * self.hidden, ctx.act_dtype)
         self.w_router = self.b_router = self.w_gate_up = self.w_down = self.choice_correction = None
@@ -223,13 +223,8 @@ class MixtureOfExperts:
             xin = ws.get("moe_in", slots, self.hidden)
             ops.moe_gather(x, order, self.top, xin)
             a = ws.get("moe_act", slots, self.inter)
-            if self.activation != "clamped_swish":
-                ops.gemm_tc_grouped(xin, self.w_gate_up, a, tiles, E, gated=self.gated, row_entry=order, row_scale=on_input,
-                                    relu2=relu2)
-            else:
-                gu = ws.get("moe_gate_up", slots, 2 * self.inter)
-                ops.gemm_tc_grouped(xin, self.w_gate_up, gu, tiles, E)
-                self._activate(gu, a)
+            ops.gemm_tc_grouped(xin, self.w_gate_up, a, tiles, E, gated=self.gated, row_entry=order, row_scale=on_input, relu2=relu2,
+                                clamped=(self.limit, self.alpha, self.shift) if self.activation == "clamped_swish" else None)
             y = ws.get("moe_rows", slots, self.hidden)
             ops.gemm_tc_grouped(a, self.w_down, y, tiles, E)
         else:
