@@ -41,8 +41,11 @@ def library_file() -> str:
     return build.library_path()
 
 
+_NULL = ctypes.c_void_p(0)            # (made once: a launch may name a dozen tensors that are not there)
+
+
 def _p(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return ctypes.c_void_p(t.data_ptr()) if t is not None else _NULL
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -814,8 +817,8 @@ def attn_prefill_x(q: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache:
     _check(lib().gg_attn_prefill_x(_p(q), ctypes.c_longlong(q_stride), _p(kcache), _p(vcache), dtype_code(kcache.dtype),
                                    _p(block_tables), bt_stride, _p(cu_q_lens), _p(context_lens), _p(tile_seq),
                                    _p(tile_q0), num_tiles, _p(tile64_seq), _p(tile64_q0), num_tiles64, int(allow_mma),
-                                   _p(tile128_seq if use_tc else None), _p(tile128_q0 if use_tc else None), num_tiles128,
-                                   q.shape[0], kcache.shape[0], _p(tc_status(q.device)) if use_tc else ctypes.c_void_p(0),
+                                   _p(tile128_seq) if use_tc else _NULL, _p(tile128_q0) if use_tc else _NULL, num_tiles128,
+                                   q.shape[0], kcache.shape[0], _p(tc_status(q.device)) if use_tc else _NULL,
                                    _p(out), int(out.dtype == torch.float32 and kcache.dtype != torch.float32),
                                    nh, nkv, d, dv, v_share, page_size, window, ctypes.c_float(scale),
                                    ctypes.c_float(softcap), int(keep_first), int(sigmoid_weights), _p(head_bias),

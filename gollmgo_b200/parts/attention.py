@@ -238,7 +238,9 @@ class Attention:
         """The tiles of 128 query rows for a prompt step of the general path that runs on tcgen05 (ops.attn_prefill_x), as its
         arguments; empty where the mma.sync kernel is the faster one (_few_short_tiles; at least two heads must share a kv
         head for the other kernel to take the step at all)."""
-        t128 = batch.tiles.get(TILES_TC) if self._mma_x else None
+        if not self._mma_x:
+            return {}
+        t128 = batch.tiles.get(TILES_TC)
         if t128 is None or self._few_short_tiles(t128.count, batch):
             return {}
         return dict(tile128_seq=t128.seq, tile128_q0=t128.q0, num_tiles128=t128.count)
@@ -251,7 +253,10 @@ class Attention:
         3.84, 128 tokens 4.45 / 4.24, 256 tokens 5.2-5.6 / 5.3-5.4, 512 tokens 8.3-8.5 / 8.6."""
         if tiles128 * ((self.nh + 1) // 2) * 2 > self.num_sms:
             return False
-        return max(s + n for s, n in zip(batch.q_starts, batch.q_lens) if n > 1) <= SHORT_PROMPT_KEYS
+        for s, n in zip(batch.q_starts, batch.q_lens):
+            if n > 1 and s + n > SHORT_PROMPT_KEYS:
+                return False
+        return True
 
     def _flat_step(self, n_dec: int) -> bool:
         """More (token, kv head) pairs than CTAs fit at once: equal ranges of tiles, no slices."""

@@ -30,8 +30,9 @@ class PlainRecurrence:
     def run(self, rows, beta, decay, state, batch, out):
         groups, heads, d, dv = self.sizes
         seqs = (batch.cu_q_lens, batch.context_lens, batch.state_slots, batch.num_seqs)
-        tiles = batch.tiles.get(CHUNKS) if self.chunked and batch.num_portions else None
-        if tiles is not None and max(batch.q_lens) >= CHUNKS_FROM:
+        long = self.chunked and batch.num_portions and max(batch.q_lens) >= CHUNKS_FROM
+        tiles = batch.tiles.get(CHUNKS) if long else None
+        if tiles is not None:
             scratch = self.ctx.workspace.get("linear_states", 1, ops.linear_scratch_floats(out.shape[0], batch.num_seqs, heads, d, dv))
             if ops.linear_chunks(rows, beta, decay, state, scratch, tiles.seq, tiles.q0, tiles.count, *seqs, groups, heads, d, dv, out):
                 if batch.num_decode:
