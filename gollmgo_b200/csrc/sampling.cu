@@ -506,7 +506,9 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
   const float target = u * total;
   if (local > 0.f && target >= before && target < before + local) {
     const unsigned over = __ballot_sync(0xffffffffu, sub > 0.f && target < before + incl);
-    // (rounding can leave none: then the last block with anything in it)
+    // (rounding can leave none: then the last block with anything in it.  A lane's running sum starts from a sum in another
+    // order than the one its neighbour ended with, so a draw can fall between the two: a value without weight, as a masked
+    // one in a row without thresholds, is not taken for it)
     const unsigned some = __ballot_sync(0xffffffffu, sub > 0.f);
     const int b = over ? __ffs(over) - 1 : 31 - __clz(some);
     float cum = before + __shfl_sync(0xffffffffu, incl - sub, b);
@@ -519,7 +521,10 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
       int last = -1;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (!(w[j] < 0.f)) { sum += w[j]; last = at + j; }
+        if (!(w[j] < 0.f)) sum += w[j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (w[j] > 0.f) last = at + j;
       float run = sum;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -530,7 +535,7 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
       int hit = -1;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (!(w[j] < 0.f)) { c += w[j]; if (hit < 0 && target < c) hit = at + j; }
+        if (w[j] > 0.f) { c += w[j]; if (hit < 0 && target < c) hit = at + j; }
       const unsigned hits = __ballot_sync(0xffffffffu, hit >= 0), lasts = __ballot_sync(0xffffffffu, last >= 0);
       if (hits) { pick = __shfl_sync(0xffffffffu, hit, __ffs(hits) - 1); break; }
       if (lasts) pick = __shfl_sync(0xffffffffu, last, 31 - __clz(lasts));
@@ -677,8 +682,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int V, int part, const f
     for (int i = i0; i < i1; ++i) {
       const float x = sc_part[i];
       if (ordered_key(x) >= floor_key) {
-        cum += expf((x - m) * invT);
-        pick = base + i;
+        const float w = expf((x - m) * invT);
+        cum += w;
+        if (w > 0.f) pick = base + i;            // (a draw that rounding carries past the end falls back to a value that can be drawn)
         if (target < cum) break;
       }
     }
