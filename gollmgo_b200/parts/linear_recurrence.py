@@ -16,11 +16,13 @@ CHUNKS_FROM = 256
 
 
 class PlainRecurrence:
-    """Sizes: groups of q and k, heads, keys of d and values of dv."""
+    """Sizes: groups of q and k, heads, keys of d and values of dv.  ``chunks``: whether the chunk form may be used.  Its products
+    of three tf32 parts and sums cut off at 24 bits are 1e-7 to 2e-6 from float64, the walk's 1e-7 to 4e-7: nothing beside the
+    rounding of bfloat16 activations, but a model served in float32 keeps the walk."""
 
-    def __init__(self, ctx, groups, heads, d, dv):
+    def __init__(self, ctx, groups, heads, d, dv, chunks=True):
         self.ctx, self.sizes = ctx, (groups, heads, d, dv)
-        self.chunked = ops.linear_chunks_ok(d, dv)
+        self.chunked = chunks and ops.linear_chunks_ok(d, dv)
         if self.chunked:
             ctx.workspace.reserve("linear_states", ops.linear_scratch_floats(ctx.max_tokens, ctx.max_seqs, heads, d, dv), torch.float32)
 

@@ -13,7 +13,8 @@ The recurrence is the engine's plain linear recurrence (parts/linear_recurrence.
 with one more value column that is always 1, so that n is a column of S; the gates, the maxima and the
 normaliser are csrc/mlstm.cu.  State per request, in its state slot: S with n in float32
 [heads, dvp, d] (dvp = dv + 1 rounded up to 4) and m [heads].  Nothing is paged.  The gates' product is
-summed and left in float32, and so is everything between the projections and the gated rows.
+summed and left in float32, and so is everything between the projections and the gated rows; long portions of bfloat16
+models are multiplied in tf32 parts (csrc/linear_chunks.cu).
 
 params: hidden_size, num_heads, head_dim, v_head_dim, gate_cap (0: none), eps, floor (default 1e-6), out_buffer,
 names (optional dict: q, k, v, i, f, gate, o, norm; the gates' biases are the i, f names + ".b").
@@ -62,7 +63,7 @@ class MatrixMemory:
         ws.reserve("mlstm_o", T * self.nh * self.dvp, torch.float32)
         ws.reserve("mlstm_y", T * self.nh * self.dv, ctx.act_dtype)
         ws.reserve(self.out_buffer, T * self.hidden, ctx.act_dtype)
-        self.recurrence = PlainRecurrence(ctx, self.nh, self.nh, self.d, self.dvp)
+        self.recurrence = PlainRecurrence(ctx, self.nh, self.nh, self.d, self.dvp, chunks=ctx.act_dtype != torch.float32)
         self.w_proj = self.w_if = self.b_i = self.b_f = self.norm_w = self.w_o = None
 
     def cache_need(self):

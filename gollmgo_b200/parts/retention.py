@@ -8,7 +8,8 @@ mean square (no weight), the heads together are multiplied by silu(Wg x) and pro
 
 State per request, in its state slot: S in float32 [heads, dv, d].  Nothing is paged.  Everything between
 the projections and the gated rows is float32 (csrc/retention.cu): single decoded tokens in one kernel, prompt
-portions in chunks whose states follow one another and whose rows are then all made at once.  Heads of more
+portions in chunks whose states follow one another and whose rows are then all made at once; long portions of
+bfloat16 models have those chunks multiplied in tf32 parts on the tensor cores (csrc/linear_chunks.cu).  Heads of more
 than 512 values go token by token through the engine's plain linear recurrence (csrc/delta_rule.cu) instead.
 
 params: hidden_size, num_heads, head_dim, v_head_dim, decay (one number in (0, 1] per head), position
@@ -28,7 +29,7 @@ from .linear import linear
 from .registry import build_position, register_mixer
 
 CHUNKS = QueryTiles(ops.RETENTION_CHUNK)          # the chunks of prompt portions: of the packed float32 kernels,
-TC_CHUNKS = QueryTiles(ops.LINEAR_CHUNK)          # and of the tensor-core ones (sizes that linear_chunks_ok names)
+TC_CHUNKS = QueryTiles(ops.LINEAR_CHUNK)          # and of the tensor-core ones (bfloat16 models, sizes that linear_chunks_ok names)
 # Steps with so many prompt tokens take the tensor-core kernels (a B200, 16 heads 128 x 256, us for a layer, tensor cores and
 # packed float32: one sequence of 16: 43 and 39, of 65: 61 and 55, of 128: 70 and 72, of 512: 98 and 108, of 4096: 485 and 610;
 # 8 of 16: 57 and 58, of 64: 93 and 122; 32 of 128: 522 and 617).
@@ -69,7 +70,7 @@ class Retention:
         self.decays = torch.tensor(self.decay, dtype=torch.float32, device=ctx.device)
         self.log2_decays = torch.tensor([math.log2(g) for g in self.decay], dtype=torch.float32, device=ctx.device)
         self.chunked = self.dv <= ops.RETENTION_MAX_V
-        self.tc = self.chunked and ops.linear_chunks_ok(self.d, self.dv)
+        self.tc = self.chunked and ctx.act_dtype != torch.float32 and ops.linear_chunks_ok(self.d, self.dv)
         if self.tc:
             ws.reserve("linear_states", ops.linear_scratch_floats(T, ctx.max_seqs, self.nh, self.d, self.dv), torch.float32)
         if self.chunked:

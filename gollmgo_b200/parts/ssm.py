@@ -11,7 +11,8 @@ weight, and projected back.
 
 State per request, in its state slot: S in float32 [heads, v_head_dim, state] and the last
 taps - 1 inputs of the convolution in float32 [taps - 1, channels].  Nothing is paged.  The
-recurrence is the plain linear one (parts/linear_recurrence.py, csrc/ssm.cu); everything between the two products is float32.
+recurrence is the plain linear one (parts/linear_recurrence.py, csrc/ssm.cu).  Everything between the two products is held in
+float32; long portions of bfloat16 models are multiplied in tf32 parts (csrc/linear_chunks.cu).
 
 params: hidden_size, num_heads, v_head_dim, state, groups, conv (taps), norm_groups, eps, out_buffer,
 names (optional dict: in, conv, conv_bias, dt_bias, A_log, D, norm, o).
@@ -64,7 +65,7 @@ class StateSpaceMixer:
         ws.reserve("ssm_y", T * self.inner, torch.float32)
         ws.reserve("ssm_out", T * self.inner, ctx.act_dtype)
         ws.reserve(self.out_buffer, T * self.hidden, ctx.act_dtype)
-        self.recurrence = PlainRecurrence(ctx, self.groups, self.nh, self.n, self.p)
+        self.recurrence = PlainRecurrence(ctx, self.groups, self.nh, self.n, self.p, chunks=ctx.act_dtype != torch.float32)
         self.w_in = self.w_o = self.conv_w = self.conv_b = self.a_log = self.dt_bias = self.d_skip = self.norm_w = None
 
     def cache_need(self):
