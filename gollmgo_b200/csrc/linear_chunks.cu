@@ -13,6 +13,9 @@
 // bits count); hi hi + hi lo + lo hi, the term left out and what lo drops are 2^-21 of a product.  hi hi and the small terms
 // have accumulators of their own where tensor memory has the room (the tensor core's sums are cut off, not rounded).  Sums
 // of logarithms are float64 and are subtracted there, so strong decays cost no accuracy.
+// Infinities and NaN reach what they reach token by token: a bad value column, factor or decay the rows from its token on, a
+// bad k those rows in all columns, a bad q its own row, and the state.  There they are NaN, also where the walk would have
+// kept an infinity.  What rounds to infinity at 11 bits (from 2^128 (1 - 2^-12) on; no bfloat16 value does) counts as one.
 // What bounds it: reading rows, splitting and writing both parts to shared memory (every operand arrives as float32 rows and
 // three of them have to be turned), a step of 32 values of k at a time, the next step's reads under way; the products run
 // beside that.  With the products on mma.sync (tf32 there runs at 486 multiply-adds a clock and multiprocessor) every warp
@@ -62,8 +65,11 @@ struct LinearArgs {
 __device__ __forceinline__ size_t lc_place(int first_token, int b) { return (size_t)(first_token / LC_C + b); }
 
 // log2 of a decay.  One of 0 (its exponential underflowed) stays finite, so that differences of sums do, and still
-// wipes out what came before: 2^-2000.
-__device__ __forceinline__ float lc_log2(float g) { return fmaxf(log2f(g), -2000.f); }
+// wipes out what came before: 2^-2000.  NaN stays NaN.
+__device__ __forceinline__ float lc_log2(float g) {
+  const float l = log2f(g);
+  return l < -2000.f ? -2000.f : l;
+}
 
 // What a lane of a warp holds of a chunk's decays and factors: of tokens 4 lane .. 4 lane + 3.
 struct LcTokens { float g[4], b[4]; };
@@ -95,8 +101,10 @@ __device__ __forceinline__ void lc_sums(const LinearArgs& p, const LcTokens& x, 
     const double v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
+  double before = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) before = 0.0;                         // (not incl - s: a NaN would reach the lane's tokens before it)
 #pragma unroll
-  for (int i = 0; i < 4; ++i) L[4 * lane + i] = (incl - s) + a[i];
+  for (int i = 0; i < 4; ++i) L[4 * lane + i] = before + a[i];
 }
 
 __device__ __forceinline__ void lc_split(float x, float& hi, float& lo) {
@@ -154,6 +162,31 @@ template <int R> struct LcAcross {
         const int r = 8 * (warp + 16 * i) + 4 * e;
         v[2 * i + e] = lane < tokens && r < rows ? *reinterpret_cast<const float4*>(s + r) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+  }
+  // A product over tokens gives an earlier token's row a weight of 0 for a later one's value, and 0 times infinity or NaN is
+  // NaN: such values leave the tile here (as 0), and first[r] becomes the first token that had one in column r.  One
+  // multiply-add a value finds them.  Returns whether there was any.
+  __device__ __forceinline__ bool take_out(int token, int* first) {
+    const int warp = threadIdx.x >> 5;
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float z = 0.f;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) { const float4 q = v[2 * i + e]; z = fmaf(q.x, 0.f, z); z = fmaf(q.y, 0.f, z); z = fmaf(q.z, 0.f, z); z = fmaf(q.w, 0.f, z); }
+      if (z == 0.f) continue;
+      any = true;
+      const int r0 = 8 * (warp + 16 * i);
+      auto check = [&](float& x, int r) {
+        if (x * 0.f != 0.f) { atomicMin(first + r, token); x = 0.f; }
+      };
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        check(v[2 * i + e].x, r0 + 4 * e); check(v[2 * i + e].y, r0 + 4 * e + 1);
+        check(v[2 * i + e].z, r0 + 4 * e + 2); check(v[2 * i + e].w, r0 + 4 * e + 3);
+      }
+    }
+    return any;
   }
   // scale(i): the factor of the lane's token in the rows of turn i
   template <typename F> __device__ __forceinline__ void store(unsigned at, unsigned lo_off, F scale) {
@@ -396,6 +429,7 @@ linear_rows_kernel(const LinearArgs p) {
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 3];
   __shared__ double Ls[8][LC_C];
   __shared__ float bs[8][LC_C], fs[8][LC_C];
+  __shared__ int first_s[8][NB], marked_s[8];          // of the heads' columns: the first token with infinity or NaN in v
   __shared__ unsigned tmem_base_s;
   __shared__ int abort_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -408,8 +442,10 @@ linear_rows_kernel(const LinearArgs p) {
     mbar_init(done(0), 1);
     mbar_init(done(1), 1);
     abort_s = 0;
+    for (int h = 0; h < 8; ++h) marked_s[h] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (int e = threadIdx.x; e < 8 * NB; e += LC_THREADS) first_s[e / NB][e % NB] = LC_C;
   if (warp == LC_ISSUER) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -477,6 +513,11 @@ linear_rows_kernel(const LinearArgs p) {
         } else {
 #pragma unroll
           for (int e = 0; e < 32; ++e) o[e] = __uint_as_float(m[e]);
+        }
+        if (*(volatile int*)&marked_s[hh]) {           // rows from such a token on
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (i >= *(volatile int*)&first_s[hh][c0 + e]) o[e] = __int_as_float(0x7fffffff);
         }
       };
       if (!RETENTION) {
@@ -578,6 +619,7 @@ linear_rows_kernel(const LinearArgs p) {
           lc_sts4(to, hi[0], hi[1], hi[2], hi[3]);
           lc_sts4(to + LC_A_BYTES, lo[0], lo[1], lo[2], lo[3]);
         }
+        if (v.take_out(32 * s + lane, first_s[hh])) { *(volatile int*)&marked_s[hh] = 1; __threadfence_block(); }
         v.store(at + 2 * LC_A_BYTES, B_PART, one);
         if (s + 1 < kj) v.load(rv + (size_t)h * dv + (size_t)(32 * (s + 1)) * p.row_stride, p.row_stride, n - 32 * (s + 1), dv);
         ring.give();
