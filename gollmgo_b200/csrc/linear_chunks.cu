@@ -534,8 +534,9 @@ linear_rows_kernel(const LinearArgs p) {
       } else {
         // The rows go through the ring's memory (one head a CTA: every product that read it is done), so that a warp has a
         // row of the result: its sum of squares, its gate and its values side by side.
-        float* tile = reinterpret_cast<float*>(lc_smem_raw);
+        float* tile = reinterpret_cast<float*>(lc_smem_raw + (base - tc_smem(lc_smem_raw)));      // (16-byte accesses)
         constexpr int TP = NB + 4;
+        static_assert(LC_C * TP * sizeof(float) <= STAGES * STAGE, "the rows fit in the ring");
         for (int c0 = (warp >> 2) * 32; c0 < cols; c0 += LC_WORKERS / 4) {
           float o[32];
           value(c0, o);
