@@ -44,10 +44,11 @@ struct LinearArgs {
   const float* decay;          // [T, H]; null: log2_decay
   const float* log2_decay;     // [H]
   float* state;                // [slots, H, dv, d]
-  float* scratch;              // [places][H][dv][d]: P of a chunk, then the state before it
-  float* factor;               // [places][H]: 2^(L_n)
-  const int* tile_seq;         // chunks: sequence and first token of its portion
+  float* scratch;              // [chunks][H][dv][d]: P of a chunk, then the state before it
+  float* factor;               // [chunks][H]: 2^(L_n)
+  const int* tile_seq;         // chunks: sequence and first token of its portion; a sequence's side by side in their order
   const int* tile_q0;
+  int tiles;
   const int* cu_q_lens;
   const int* context_lens;
   const int* state_slots;
@@ -59,10 +60,6 @@ struct LinearArgs {
   void* out;                   // retention: [T, H dv] in the gate's type
   int* status;
 };
-
-// Chunk c of sequence b has this place in the scratch: unique, since a sequence's chunks start 128 tokens apart and the next
-// sequence's first index is at least one higher.  Places needed: T / 128 + B + 1.
-__device__ __forceinline__ size_t lc_place(int first_token, int b) { return (size_t)(first_token / LC_C + b); }
 
 // log2 of a decay.  One of 0 (its exponential underflowed) stays finite, so that differences of sums do, and still
 // wipes out what came before: 2^-2000.  NaN stays NaN.
@@ -302,7 +299,7 @@ linear_products_kernel(const LinearArgs p) {
   const int b = p.tile_seq[blockIdx.x], q0 = p.tile_q0[blockIdx.x], h0 = blockIdx.y * p.heads, m0 = blockIdx.z * 128;
   const int qlen = p.cu_q_lens[b + 1] - p.cu_q_lens[b], t0 = p.cu_q_lens[b] + q0, n = min(LC_C, qlen - q0);
   const int d = p.d, dv = p.dv, cols = p.heads * dv, steps = (n + 31) / 32;
-  const size_t place = lc_place(t0, b);
+  const size_t place = blockIdx.x;
   pdl_trigger();
   pdl_wait();
   // the first step's rows and the decays are on their way together
@@ -383,10 +380,17 @@ linear_products_kernel(const LinearArgs p) {
 // grid (B, H, pieces of 1024 values), 256 threads, four values a thread; four chunks' reads under way.
 __global__ void __launch_bounds__(256)
 linear_scan_kernel(const LinearArgs p) {
+  __shared__ int first_s;
   pdl_trigger();
   const int b = blockIdx.x, h = blockIdx.y;
-  const int slot = p.state_slots[b], t0 = p.cu_q_lens[b], qlen = p.cu_q_lens[b + 1] - t0;
-  if (slot < 0 || qlen <= 1) { pdl_wait(); return; }                  // single tokens go through another kernel
+  const int slot = p.state_slots[b], qlen = p.cu_q_lens[b + 1] - p.cu_q_lens[b];
+  if (threadIdx.x == 0) first_s = -1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < p.tiles; i += 256)                    // the sequence's first chunk
+    if (p.tile_seq[i] == b && p.tile_q0[i] == 0) first_s = i;
+  __syncthreads();
+  const int first = first_s;
+  if (slot < 0 || first < 0) { pdl_wait(); return; }                  // sequences without chunks go through another kernel
   const size_t size = (size_t)p.d * p.dv, at = ((size_t)blockIdx.z * 256 + threadIdx.x) << 2;
   const bool live = at < size;
   float4* st = reinterpret_cast<float4*>(p.state + ((size_t)slot * p.H + h) * size + at);
@@ -395,7 +399,7 @@ linear_scan_kernel(const LinearArgs p) {
   const bool carry = p.context_lens[b] - qlen > 0;
   float4 S = carry ? *st : make_float4(0.f, 0.f, 0.f, 0.f);
   const int chunks = (qlen + LC_C - 1) / LC_C;
-  auto place = [&](int c) { return lc_place(t0 + c * LC_C, b) * p.H + h; };
+  auto place = [&](int c) { return (size_t)(first + c) * p.H + h; };
   for (int c0 = 0; c0 < chunks; c0 += 4) {
     float4 P[4];
     float f[4];
@@ -572,7 +576,7 @@ linear_rows_kernel(const LinearArgs p) {
       const int h = h0 + hh;
       if (BUFS == 1 && hh > 0) epilogue(hh - 1);       // its tensor memory is the next head's
       if (carry) {                                     // what the state before the chunk is worth to each row
-        const float* S = p.scratch + (lc_place(t0, b) * p.H + h) * (size_t)dv * d;
+        const float* S = p.scratch + ((size_t)blockIdx.x * p.H + h) * dv * d;
         LcAlong<128> a;
         LcAlong<NB> v;
         a.load(rq, p.row_stride, n, 0, d);
@@ -662,8 +666,7 @@ linear_rows_kernel(const LinearArgs p) {
 
 // ---------------------------------------------------------------- launchers
 // Floats of scratch: a state and a factor per chunk and head.
-static long long lc_places(int T, int B) { return T / LC_C + B + 1; }
-static long long lc_scratch(int T, int B, int H, int d, int dv) { return lc_places(T, B) * H * ((long long)d * dv + 4); }
+static long long lc_scratch(int tiles, int H, int d, int dv) { return (long long)tiles * H * ((long long)d * dv + 4); }
 
 // Whether the kernels take these sizes and addresses.
 static bool lc_supported(const LinearArgs& p) {
@@ -692,8 +695,9 @@ template <int NB, bool RETENTION, typename TA> static int lc_rows(const LinearAr
   return gg_check_launch("linear_rows");
 }
 
-template <bool RETENTION, typename TA> static int lc_run(LinearArgs p, int num_tiles, int T, cudaStream_t stream) {
-  p.factor = p.scratch + lc_places(T, p.B) * p.H * (long long)p.d * p.dv;
+template <bool RETENTION, typename TA> static int lc_run(LinearArgs p, int num_tiles, cudaStream_t stream) {
+  p.tiles = num_tiles;
+  p.factor = p.scratch + (long long)num_tiles * p.H * p.d * p.dv;
   const int rep = p.H / p.G;
   // the chunks' products: heads of a group side by side, up to 256 columns (eight neighbouring ones are of one head)
   p.heads = 1;
@@ -712,9 +716,9 @@ template <bool RETENTION, typename TA> static int lc_run(LinearArgs p, int num_t
   return lc_rows<256, RETENTION, TA>(p, num_tiles, stream);
 }
 
-// gg_delta_recur's plain recurrence over the sequences with more than one token (their chunks of 128 tokens are the tiles);
-// the others are left alone.  Returns GG_ERR_UNSUPPORTED, and launches nothing, where sizes or addresses are not for these
-// kernels.  Scratch the caller provides: float[(T / 128 + B + 1) * H * (d * dv + 4)].
+// gg_delta_recur's plain recurrence over the sequences whose chunks of 128 tokens are the tiles (all chunks of a sequence, in
+// their order); the others are left alone.  Returns GG_ERR_UNSUPPORTED, and launches nothing, where sizes or addresses are not
+// for these kernels.  Scratch the caller provides: float[num_tiles * H * (d * dv + 4)].
 extern "C" int gg_linear_chunks(const float* qkv, const float* beta, const float* decay, float* state, float* scratch,
                                 long long scratch_floats, const int* tile_seq, const int* tile_q0, int num_tiles,
                                 const int* cu_q_lens, const int* context_lens, const int* state_slots, int T, int B, int G, int H,
@@ -727,9 +731,9 @@ extern "C" int gg_linear_chunks(const float* qkv, const float* beta, const float
   p.cu_q_lens = cu_q_lens; p.context_lens = context_lens; p.state_slots = state_slots;
   p.B = B; p.G = G; p.H = H; p.d = d; p.dv = dv; p.o_raw = o_raw; p.status = status;
   if (!lc_supported(p) || H > 65535) return GG_ERR_UNSUPPORTED;
-  GG_REQUIRE(scratch_floats >= lc_scratch(T, B, H, d, dv), "linear_chunks: scratch of %lld values is too small", scratch_floats);
+  GG_REQUIRE(scratch_floats >= lc_scratch(num_tiles, H, d, dv), "linear_chunks: scratch of %lld values is too small", scratch_floats);
   if (num_tiles == 0) return GG_OK;
-  return lc_run<false, float>(p, num_tiles, T, stream);
+  return lc_run<false, float>(p, num_tiles, stream);
 }
 
 // Retention's prompt portions (see retention.cu): rows of gg_retention_rows, one fixed decay a head, unit norm and gate.
@@ -747,7 +751,7 @@ extern "C" int gg_linear_retention(const float* rows, const float* log2_decay, f
   p.gate = gate; p.gate_stride = gate_stride; p.eps = eps; p.out = out; p.status = status;
   if (!lc_supported(p) || (dtype != GG_F32 && dtype != GG_BF16) || gate_stride % 4 || ((size_t)gate % 16) || ((size_t)out % 16) || H > 65535)
     return GG_ERR_UNSUPPORTED;
-  GG_REQUIRE(scratch_floats >= lc_scratch(T, B, H, d, dv), "linear_retention: scratch of %lld values is too small", scratch_floats);
+  GG_REQUIRE(scratch_floats >= lc_scratch(num_tiles, H, d, dv), "linear_retention: scratch of %lld values is too small", scratch_floats);
   if (num_tiles == 0) return GG_OK;
-  return dtype == GG_F32 ? lc_run<true, float>(p, num_tiles, T, stream) : lc_run<true, __nv_bfloat16>(p, num_tiles, T, stream);
+  return dtype == GG_F32 ? lc_run<true, float>(p, num_tiles, stream) : lc_run<true, __nv_bfloat16>(p, num_tiles, stream);
 }

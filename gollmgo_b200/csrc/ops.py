@@ -992,6 +992,7 @@ def linear_chunks_ok(d: int, dv: int) -> bool:
 
 
 def linear_scratch_floats(num_tokens: int, num_seqs: int, heads: int, d: int, dv: int) -> int:
+    """Room for the chunks of num_seqs portions of num_tokens together, however long each is."""
     return (num_tokens // LINEAR_CHUNK + num_seqs + 1) * heads * (d * dv + 4)         # a state and a factor per chunk and head
 
 
@@ -999,8 +1000,8 @@ def linear_chunks(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, st
                   tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
                   context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, kv_heads: int, heads: int, d: int,
                   dv: int, o_raw: torch.Tensor) -> bool:
-    """delta_recur(plain=True) over the sequences with more than one token in this step, a chunk of LINEAR_CHUNK tokens at a
-    time (tile_seq, tile_q0: the chunks); the others are left alone.  scratch: float32 of linear_scratch_floats().
+    """delta_recur(plain=True) over the sequences whose chunks of LINEAR_CHUNK tokens tile_seq and tile_q0 list (all chunks of a
+    sequence, side by side in their order); the others are left alone.  scratch: float32 of linear_scratch_floats().
     False, and nothing done, where sizes or addresses are not for these kernels."""
     _cuda(qkv, beta, decay, state, scratch, o_raw)
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, d) or decay.shape[-1] != heads \
@@ -1021,8 +1022,8 @@ def linear_retention(rows: torch.Tensor, log2_decay: torch.Tensor, state: torch.
                      tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
                      context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, gate: torch.Tensor, eps: float,
                      heads: int, d: int, dv: int, out: torch.Tensor) -> bool:
-    """retention_chunks on the kernels of linear_chunks: tiles of LINEAR_CHUNK rows, scratch float32 of
-    linear_scratch_floats().  False, and nothing done, where sizes or addresses are not for these kernels."""
+    """retention_chunks on the kernels of linear_chunks, over the sequences that the tiles of LINEAR_CHUNK rows name (as there);
+    scratch float32 of linear_scratch_floats().  False, and nothing done, where sizes or addresses are not for these kernels."""
     global tc_launched
     _cuda(rows, log2_decay, state, scratch, tile_seq, tile_q0, out)
     if rows.dtype != torch.float32 or rows.shape[1] != heads * (2 * d + dv) or log2_decay.dtype != torch.float32 \
@@ -1320,10 +1321,11 @@ def retention_scratch_floats(tokens: int, seqs: int, heads: int, d: int, dv: int
 def retention_chunks(rows: torch.Tensor, log2_decay: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
                      tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
                      context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, gate: torch.Tensor, eps: float,
-                     heads: int, d: int, dv: int, out: torch.Tensor) -> None:
+                     heads: int, d: int, dv: int, out: torch.Tensor, max_len: int = 0) -> None:
     """The tokens of prompt portions: S <- g S + k v^T, o = S^T q, out = o / sqrt(mean(o^2) + eps) * silu(gate), from
     retention_rows' rows and from and to state [slots, heads, dv, d]; tiles of RETENTION_CHUNK rows (tile_seq, tile_q0)
-    are the chunks.  gate: a column view [T, heads*dv]; scratch float32 of retention_scratch_floats()."""
+    are the chunks.  gate: a column view [T, heads*dv]; scratch float32 of retention_scratch_floats().  ``max_len`` > 0: portions
+    of more tokens are left alone."""
     _cuda(rows, log2_decay, state, scratch, tile_seq, tile_q0, out)
     T = rows.shape[0]
     if rows.dtype != torch.float32 or rows.shape[1] != heads * (2 * d + dv) or log2_decay.dtype != torch.float32 \
@@ -1331,10 +1333,10 @@ def retention_chunks(rows: torch.Tensor, log2_decay: torch.Tensor, state: torch.
             or scratch.dtype != torch.float32 or gate.stride(1) != 1 or gate.dtype != out.dtype:
         raise KernelError("retention_chunks: float32 rows, decays, state [slots, heads, dv, d] and scratch; gate of the output's dtype")
     _check(lib().gg_retention_states(_p(rows), _p(log2_decay), _p(state), _p(scratch), ctypes.c_longlong(scratch.numel()),
-                                     _p(cu_q_lens), _p(context_lens), _p(state_slots), T, num_seqs, heads, d, dv, _stream()))
+                                     _p(cu_q_lens), _p(context_lens), _p(state_slots), T, num_seqs, heads, d, dv, int(max_len), _stream()))
     _check(lib().gg_retention_chunks(_p(rows), _p(log2_decay), _p(scratch), _p(tile_seq), _p(tile_q0), num_tiles,
                                      _p(cu_q_lens), _p(context_lens), _p(gate), ctypes.c_longlong(gate.stride(0)),
-                                     ctypes.c_float(eps), heads, d, dv, dtype_code(out.dtype), _p(out), _stream()))
+                                     ctypes.c_float(eps), heads, d, dv, int(max_len), dtype_code(out.dtype), _p(out), _stream()))
 
 
 def retention_decode(proj: torch.Tensor, gate_col: int, positions: torch.Tensor, inv_freq: Optional[torch.Tensor],

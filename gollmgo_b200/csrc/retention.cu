@@ -15,6 +15,7 @@
 // Everything is float32 arithmetic from the projection's values to y (also the products inside a chunk); angles are
 // formed and reduced in float64.  Powers of g are 2^(n log2 g).
 #include "common.cuh"
+#include <climits>
 
 __device__ __forceinline__ void rotation_of(double pos, double inv_freq, float* c, float* s) {
   const double two_pi = 6.283185307179586476925286766559;
@@ -173,13 +174,13 @@ __device__ __forceinline__ float2 ret_mul2(float2 a, float2 b) {
 __global__ void __launch_bounds__(256)
 retention_states_kernel(const float* __restrict__ rows, const float* __restrict__ log2_decay, float* __restrict__ state,
                         float* __restrict__ scratch, const int* __restrict__ cu_q_lens, const int* __restrict__ context_lens,
-                        const int* __restrict__ state_slots, int H, int d, int dv, int vec) {
+                        const int* __restrict__ state_slots, int H, int d, int dv, int max_len, int vec) {
   extern __shared__ __align__(16) float sm[];        // two stages of k [64][64], v [64][64]
   __shared__ float wj[2][RET_C];
   const int b = blockIdx.x, h = blockIdx.y;
   const int slot = state_slots[b];
   const int t0 = cu_q_lens[b], qlen = cu_q_lens[b + 1] - t0;
-  if (slot < 0 || qlen <= 1) return;                 // single tokens go through the decode kernel
+  if (slot < 0 || qlen <= 1 || qlen > max_len) return;                 // single tokens go through the decode kernel
   const int vt = (dv + RET_ST - 1) / RET_ST;
   const int r0 = (blockIdx.z / vt) * RET_ST, c0 = (blockIdx.z % vt) * RET_ST;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1)
 retention_chunks_kernel(const float* __restrict__ rows, const float* __restrict__ log2_decay, const float* __restrict__ scratch,
                         const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, const int* __restrict__ cu_q_lens,
                         const int* __restrict__ context_lens, const TA* __restrict__ gate, long long gate_stride, float eps,
-                        int H, int d, int dv, int vec, int vec_io, TA* __restrict__ out) {
+                        int H, int d, int dv, int max_len, int vec, int vec_io, TA* __restrict__ out) {
   constexpr int VP = NV * 128;
   extern __shared__ __align__(16) float sm[];
   float* Qt = sm;                                    // [d][64]: q transposed
@@ -320,6 +321,7 @@ retention_chunks_kernel(const float* __restrict__ rows, const float* __restrict_
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = tile_seq[blockIdx.x], q0 = tile_q0[blockIdx.x], h = blockIdx.y;
   const int t0 = cu_q_lens[b], qlen = cu_q_lens[b + 1] - t0;
+  if (qlen > max_len) return;
   const int n = min(RET_C, qlen - q0);
   const bool carry = context_lens[b] - qlen + q0 > 0;
   const float l2 = log2_decay[h];
@@ -650,9 +652,10 @@ retention_decode_kernel(const TA* __restrict__ x, long long x_stride, int gate_c
 
 // ---------------------------------------------------------------- launchers
 // Scratch the caller provides: float[(T / 64 + B + 1) * H * d * dv].  rows: gg_retention_rows' output.
+// max_len > 0 (here and below): portions of more tokens are left alone.
 extern "C" int gg_retention_states(const float* rows, const float* log2_decay, float* state, float* scratch,
                                    long long scratch_floats, const int* cu_q_lens, const int* context_lens,
-                                   const int* state_slots, int T, int B, int H, int d, int dv, cudaStream_t stream) {
+                                   const int* state_slots, int T, int B, int H, int d, int dv, int max_len, cudaStream_t stream) {
   GG_REQUIRE(T >= 0 && B > 0 && H > 0 && d > 0 && dv > 0, "retention_states: bad sizes T=%d B=%d H=%d d=%d dv=%d", T, B, H, d, dv);
   GG_REQUIRE(rows && log2_decay && state && scratch, "retention_states: a pointer is null");
   GG_REQUIRE(scratch_floats >= (long long)(T / RET_C + B + 1) * H * d * dv, "retention_states: scratch of %lld values is too small", scratch_floats);
@@ -664,14 +667,14 @@ extern "C" int gg_retention_states(const float* rows, const float* log2_decay, f
   if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "retention_states: %s", cudaGetErrorString(e));
   const int vec = d % 4 == 0 && dv % 4 == 0 && ((size_t)rows % 16) == 0 && ((size_t)scratch % 16) == 0 && ((size_t)state % 16) == 0;
   gg_launch_after(retention_states_kernel, dim3(B, H, tiles), dim3(256), smem, stream, rows, log2_decay, state, scratch, cu_q_lens,
-                  context_lens, state_slots, H, d, dv, vec);
+                  context_lens, state_slots, H, d, dv, max_len > 0 ? max_len : T, vec);
   return gg_check_launch("retention_states");
 }
 
 extern "C" int gg_retention_chunks(const float* rows, const float* log2_decay, const float* scratch, const int* tile_seq,
                                    const int* tile_q0, int num_tiles, const int* cu_q_lens, const int* context_lens,
-                                   const void* gate, long long gate_stride, float eps, int H, int d, int dv, int dtype,
-                                   void* out, cudaStream_t stream) {
+                                   const void* gate, long long gate_stride, float eps, int H, int d, int dv, int max_len,
+                                   int dtype, void* out, cudaStream_t stream) {
   GG_REQUIRE(num_tiles >= 0 && H > 0 && H <= 65535 && d > 0 && d <= 256 && dv > 0 && dv <= 512,
              "retention_chunks: bad sizes tiles=%d H=%d d=%d (at most 256) dv=%d (at most 512)", num_tiles, H, d, dv);
   GG_REQUIRE(rows && log2_decay && scratch && gate && out && gate_stride >= (long long)H * dv, "retention_chunks: bad arguments");
@@ -686,7 +689,7 @@ extern "C" int gg_retention_chunks(const float* rows, const float* log2_decay, c
     cudaError_t e = cudaFuncSetAttribute(retention_chunks_kernel<TA, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "retention_chunks: %s", cudaGetErrorString(e));                         \
     gg_launch(retention_chunks_kernel<TA, NV>, dim3(num_tiles, H), dim3(256), smem, stream, rows, log2_decay, scratch, tile_seq, \
-              tile_q0, cu_q_lens, context_lens, (const TA*)gate, gate_stride, eps, H, d, dv, vec, vec_io, (TA*)out);                  \
+              tile_q0, cu_q_lens, context_lens, (const TA*)gate, gate_stride, eps, H, d, dv, max_len > 0 ? max_len : INT_MAX, vec, vec_io, (TA*)out); \
   } while (0)
 #define RET_GO_NV(TA) do { if (NVv == 1) RET_GO(TA, 1); else if (NVv == 2) RET_GO(TA, 2); else RET_GO(TA, 4); } while (0)
   if (dtype == GG_F32) RET_GO_NV(float);

@@ -14,10 +14,11 @@ class QueryTiles:
     """An index list a mixer asks the batch builder for: the query rows of every prompt
     portion (a sequence with more than one token in the step) cut into tiles of ``height``
     rows, as (sequence, first row) pairs; ``most_keys_first`` orders them by how many keys
-    they attend to, longest first.  A mixer names the lists it wants in ``query_tiles()``;
+    they attend to, longest first; ``at_least``: only portions of so many rows (0: all).  A mixer names the lists it wants in ``query_tiles()``;
     the step's batch then holds each under ``batch.tiles[that QueryTiles]``."""
     height: int
     most_keys_first: bool = False
+    at_least: int = 0
 
 
 @dataclass(frozen=True)

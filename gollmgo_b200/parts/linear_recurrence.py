@@ -1,6 +1,6 @@
-"""The plain linear recurrence S <- g S + k (beta v)^T, o = S^T q over a step's sequences, for the mixers built on it: prompt
-portions in chunks as tensor-core products (csrc/linear_chunks.cu), short portions and single decoded tokens token by token
-(csrc/delta_rule.cu)."""
+"""The plain linear recurrence S <- g S + k (beta v)^T, o = S^T q over a step's sequences, for the mixers built on it: long prompt
+portions in chunks as tensor-core products (csrc/linear_chunks.cu), short ones and single decoded tokens token by token
+(csrc/delta_rule.cu).  A portion's own length decides, so its sums do not depend on what else is in the step."""
 from __future__ import annotations
 
 import torch
@@ -8,11 +8,16 @@ import torch
 from ..csrc import ops
 from .context import QueryTiles
 
-CHUNKS = QueryTiles(ops.LINEAR_CHUNK)
-# Steps whose longest portion has so many tokens take the chunk form; below, its three kernels cost more than the walk (a B200,
-# 64 heads of 64 with a state of 128, us for a layer, chunks and walk: one sequence of 128: 68 and 55, of 224: 75 and 76, of 256:
-# 77 and 82, of 2048: 274 and 485; 32 of 128 after a context: 668 and 631, of 256: 1081 and 1226).
-CHUNKS_FROM = 256
+# Portions of so many tokens take the chunk form: its three kernels, and the state that each chunk writes and reads, cost
+# more than a shorter walk.  Steps of one portion, and of sixteen after a context (a B200, us for a layer, chunks / walk):
+#   128 keys: 64 heads of 64      192: 74 / 70   256: 78 / 82    512: 111 / 140    16 x 256: 578 / 612   32 x 128: 678 / 616
+#             128 heads of 64     192: 132 / 126 256: 142 / 146  512: 192 / 242    16 x 256: 1432 / 1477 32 x 128: 1673 / 1506
+#             16 heads of 132     192: 69 / 60   256: 77 / 72    320: 82 / 86      16 x 256: 462 / 628   32 x 128: 496 / 630
+#             32 heads of 132     192: 109 / 113 256: 119 / 131  512: 156 / 217    16 x 256: 1074 / 1414
+#   64 keys:  64 heads of 64      256: 77 / 72   384: 93 / 93    512: 102 / 115    16 x 256: 502 / 464   8 x 512: 492 / 473
+# (64 keys: the walk's cost goes with the keys, a chunk's with its rows.)
+def chunks_from(d):
+    return 256 if d > 64 else 512
 
 
 class PlainRecurrence:
@@ -22,22 +27,25 @@ class PlainRecurrence:
 
     def __init__(self, ctx, groups, heads, d, dv, chunks=True):
         self.ctx, self.sizes = ctx, (groups, heads, d, dv)
-        self.chunked = chunks and ops.linear_chunks_ok(d, dv)
-        if self.chunked:
-            ctx.workspace.reserve("linear_states", ops.linear_scratch_floats(ctx.max_tokens, ctx.max_seqs, heads, d, dv), torch.float32)
+        self.limit = chunks_from(d)
+        self.chunks = QueryTiles(ops.LINEAR_CHUNK, at_least=self.limit) if chunks and ops.linear_chunks_ok(d, dv) else None
+        if self.chunks is not None:
+            T = ctx.max_tokens
+            ctx.workspace.reserve("linear_states", ops.linear_scratch_floats(T, T // self.limit, heads, d, dv), torch.float32)
 
     def query_tiles(self):
-        return [CHUNKS] if self.chunked else []
+        return [self.chunks] if self.chunks is not None else []
 
     def run(self, rows, beta, decay, state, batch, out):
         groups, heads, d, dv = self.sizes
         seqs = (batch.cu_q_lens, batch.context_lens, batch.state_slots, batch.num_seqs)
-        long = self.chunked and batch.num_portions and max(batch.q_lens) >= CHUNKS_FROM
-        tiles = batch.tiles.get(CHUNKS) if long else None
-        if tiles is not None:
-            scratch = self.ctx.workspace.get("linear_states", 1, ops.linear_scratch_floats(out.shape[0], batch.num_seqs, heads, d, dv))
+        tiles = batch.tiles.get(self.chunks) if self.chunks is not None and batch.num_portions else None
+        max_len = 0
+        if tiles is not None and tiles.count:
+            T = out.shape[0]
+            scratch = self.ctx.workspace.get("linear_states", 1, ops.linear_scratch_floats(T, T // self.limit, heads, d, dv))
             if ops.linear_chunks(rows, beta, decay, state, scratch, tiles.seq, tiles.q0, tiles.count, *seqs, groups, heads, d, dv, out):
-                if batch.num_decode:
-                    ops.delta_recur(rows, beta, decay, state, *seqs, groups, heads, d, dv, out, plain=True, max_len=1)
-                return
-        ops.delta_recur(rows, beta, decay, state, *seqs, groups, heads, d, dv, out, plain=True)
+                if min(batch.q_lens) >= self.limit:
+                    return
+                max_len = self.limit - 1
+        ops.delta_recur(rows, beta, decay, state, *seqs, groups, heads, d, dv, out, plain=True, max_len=max_len)

@@ -121,19 +121,20 @@ def test_retention_against_float64(ops, H, d, dv, dtype):
 
 @pytest.mark.parametrize("lens,chunked", [([255, 1, 3], False), ([256, 1, 3], True), ([1, 1], False)])
 def test_mixers_recurrence_takes_chunks_for_long_portions(ops, monkeypatch, lens, chunked):
-    """PlainRecurrence: the longest portion decides; single tokens of the same step are walked."""
+    """PlainRecurrence: a portion's own length decides; short portions and single tokens of the same step are walked."""
     from types import SimpleNamespace
     from gollmgo_b200.parts import linear_recurrence as L
     from gollmgo_b200.parts.context import Workspace
-    G, H, d, dv, T, B = 1, 2, 16, 8, sum(lens), len(lens)
+    G, H, d, dv, T, B = 1, 2, 128, 8, sum(lens), len(lens)
     ws = Workspace(torch.device("cuda"))
     rec = L.PlainRecurrence(SimpleNamespace(workspace=ws, max_tokens=T, max_seqs=B), G, H, d, dv)
+    need, = rec.query_tiles()
     rows, beta, decay = (torch.rand(T, w, device="cuda") for w in (2 * G * d + H * dv, H, H))
     state, cu, ctx = torch.rand(B, H, dv, d, device="cuda"), i32([sum(lens[:b]) for b in range(B + 1)]), i32([n + 2 for n in lens])
-    tiles = [(b, x) for b, n in enumerate(lens) if n > 1 for x in range(0, n, 128)]
+    tiles = [(b, x) for b, n in enumerate(lens) if n > 1 and n >= need.at_least for x in range(0, n, 128)]
     batch = SimpleNamespace(cu_q_lens=cu, context_lens=ctx, state_slots=i32(list(range(B))), num_seqs=B, q_lens=lens,
                             num_portions=sum(n > 1 for n in lens), num_decode=sum(n == 1 for n in lens),
-                            tiles={L.CHUNKS: SimpleNamespace(seq=i32([t[0] for t in tiles]), q0=i32([t[1] for t in tiles]), count=len(tiles))})
+                            tiles={need: SimpleNamespace(seq=i32([t[0] for t in tiles]), q0=i32([t[1] for t in tiles]), count=len(tiles))})
     calls, real = [], ops.linear_chunks
     monkeypatch.setattr(ops, "linear_chunks", lambda *a: calls.append(1) or real(*a))
     got, want = [(state.clone(), torch.full((T, H * dv), float("nan"), device="cuda")) for _ in range(2)]
@@ -142,3 +143,5 @@ def test_mixers_recurrence_takes_chunks_for_long_portions(ops, monkeypatch, lens
     assert bool(calls) == chunked
     for a, b in zip(got, want):                            # (both within the bound above of float64)
         assert float((a - b).norm() / b.norm()) < (8e-6 if chunked else 1e-12)
+    walked = [b for b, n in enumerate(lens) if n < need.at_least]
+    assert torch.equal(got[0][walked], want[0][walked]) and torch.equal(got[1][lens[0]:], want[1][lens[0]:])

@@ -26,3 +26,81 @@ def chunk_lists(part):
 def test_models_in_float32_keep_float32_products(kind):
     assert chunk_lists(mixer(kind, torch.bfloat16)[0])
     assert not chunk_lists(mixer(kind, torch.float32)[0])
+
+
+@pytest.mark.parametrize("kind", sorted(MIXERS))
+def test_a_portion_s_own_length_decides(kind):
+    from gollmgo_b200.cache import CacheManager
+    from gollmgo_b200.engine import BatchBuilder, StepEntry
+    part, _ = mixer(kind, torch.bfloat16)
+    need, = chunk_lists(part)
+    assert need.at_least > 1
+    lens = [need.at_least, 1, need.at_least - 1, 2, need.at_least + 129]
+    cm = CacheManager([part.cache_need()], 16, 8, len(lens), dtype=torch.bfloat16, device="cpu")
+    for i in range(len(lens)):
+        cm.admit(i)
+    batch = BatchBuilder(cm, "cpu", query_tiles=part.query_tiles()).build([StepEntry(i, [0] * n, [0]) for i, n in enumerate(lens)])
+    tiles = batch.tiles[need]
+    want = [(b, q) for b in (0, 4) for q in range(0, lens[b], ops.LINEAR_CHUNK)]
+    assert tiles.count == len(want) and list(zip(tiles.seq.tolist(), tiles.q0.tolist()))[:tiles.count] == want
+
+
+@pytest.mark.parametrize("kind", ["mamba2", "mlstm"])
+def test_scratch_is_for_chunks_of_long_portions(kind):
+    """The states of the chunks that a step can hold, however many sequences a step may have."""
+    few, many = (mixer(kind, torch.bfloat16, max_seqs=n)[1].workspace._want["linear_states"][0] for n in (1, 256))
+    assert few == many
+    part, ctx = mixer(kind, torch.bfloat16, max_tokens=4096)
+    _, heads, d, dv = part.recurrence.sizes
+    limit = part.recurrence.limit
+    worst = max(n // p * -(-p // ops.LINEAR_CHUNK) for n in (4096,) for p in range(limit, 4097))
+    assert worst <= ctx.workspace._want["linear_states"][0] // (heads * (d * dv + 4)) <= 4096 // 128 + 4096 // 256 + 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", sorted(MIXERS))
+def test_long_short_and_single_portions_hand_one_state_on(kind):
+    """The layer as it chooses beside the same layer without the chunk form, over steps that mix both with decoded tokens."""
+    from gollmgo_b200 import parts
+    from gollmgo_b200.cache import CacheManager
+    from gollmgo_b200.engine import BatchBuilder, StepEntry
+    parts.set_matmul_precision()
+    steps = [[300, 40, 1, 130], [1, 280, 129, 2], [1, 1, 1, 1], [600, 1, 20, 300], [2, 255, 256, 1]]
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    weights, sides, calls = {}, [], []
+    for chunks in (True, False):
+        part, ctx = mixer(kind, torch.bfloat16, "cuda")
+        for n, s in part.weights().items():
+            if n not in weights:
+                w = torch.randn(*s.shape, device="cuda", generator=gen) * (s.shape[-1] ** -0.5 if len(s.shape) > 1 else 0.1)
+                weights[n] = (w + (4.0 if n == "f.b" else -4.0 if n == "dt_bias" else 1.0 if n in ("norm", "D") else 0.0)).bfloat16()
+        part.load(weights.__getitem__)
+        if not chunks:
+            if kind == "retention":
+                part.tc = False
+            else:
+                part.recurrence.chunks = None
+        cm = CacheManager([part.cache_need()], 16, 8, 4, dtype=torch.bfloat16, device="cuda")
+        for i in range(4):
+            cm.admit(i)
+        view = cm.cache_view(0, part.cache_need())
+        sides.append((part, BatchBuilder(cm, "cuda", query_tiles=part.query_tiles()), view))
+    name = "linear_retention" if kind == "retention" else "linear_chunks"
+    real = getattr(ops, name)
+    for lens in steps:
+        x = torch.randn(sum(lens), 64, device="cuda", generator=gen).bfloat16()
+        got = []
+        for part, builder, view in sides:
+            setattr(ops, name, lambda *a, **k: calls.append(lens) or real(*a, **k))
+            try:
+                y = part.forward(x, builder.build([StepEntry(i, [0] * n, [0]) for i, n in enumerate(lens)]), view)
+            finally:
+                setattr(ops, name, real)
+            got.append([y.float()] + [t.clone() for t in (view if isinstance(view, tuple) else (view,))])
+        # what the rows' products differ by flips a bfloat16 rounding here and there (2^-9 of a value, for a few of the values);
+        # the states are float32 on both sides, each within 4e-6 of float64
+        assert float((got[0][0] - got[1][0]).norm() / got[1][0].norm()) < 2e-3
+        for a, b in zip(got[0][1:], got[1][1:]):
+            assert float((a.float() - b.float()).norm() / b.float().norm()) < 2e-5
+    assert int(ops.tc_status("cuda")[0]) == 0
+    assert calls == [lens for lens in steps if max(lens) >= chunk_lists(sides[0][0])[0].at_least]
