@@ -346,9 +346,10 @@ extern "C" int gg_rope_kv_write_x(void* qkv, long long row_stride, int act_dtype
   GG_REQUIRE(row_stride >= (long long)(nh + nkv) * d + (long long)nv * dv, "rope_kv_write_x: rows of %lld values are too short", row_stride);
   GG_REQUIRE(!write_cache || (kcache && vcache && slot_mapping), "rope_kv_write_x: cache write without cache or slots");
   if (T == 0) return GG_OK;
-  if (rot == 0) inv_freq = nullptr;
   const size_t smem = (size_t)(rot > 0 ? rot : 2) * sizeof(float);
   GG_REQUIRE(smem <= 48 * 1024, "rope_kv_write_x: rotary width %d too large", rot);
+  if (!inv_freq) rot = 0;                                // without a table every value passes
+  if (rot == 0) inv_freq = nullptr;
   if (act_dtype == GG_BF16 && !(interleaved && rot) && d % 8 == 0 && dv % 8 == 0 && rot % 16 == 0 && row_stride % 8 == 0 && ((size_t)qkv % 16) == 0 &&
       (!write_cache || (((size_t)kcache % 16) == 0 && ((size_t)vcache % 16) == 0))) {
     gg_launch(rope_kv_write_x_vec_kernel, dim3(T), dim3(256), smem, stream, (__nv_bfloat16*)qkv, row_stride, positions, slot_mapping,
