@@ -108,7 +108,7 @@ delta_prep_vec_kernel(const TA* __restrict__ x, long long x_stride, const float*
   const int lanes = d >> 2;                              // of one q or k head: 8, 16 or 32
   const float scale = c < G * d ? rsqrtf((float)d) : 1.f;
   conv_tokens<TAPS>(x, x_stride, conv_w, (const float*)nullptr, conv_state, cu_q_lens, context_lens, state_slots, B, C,
-                    live ? c : 0, ta, tb, single && live, [&](int t, float4 y) {
+                    live ? c : 0, ta, tb, single, live, [&](int t, float4 y) {
     float ss = y.x * y.x + y.y * y.y + (y.z * y.z + y.w * y.w);
     for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float f = unit ? rsqrtf(ss + 1e-6f) * scale : 1.f;

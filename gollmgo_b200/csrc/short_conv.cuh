@@ -22,15 +22,16 @@ __device__ __forceinline__ int seq_of_token(const int* __restrict__ cu, int B, i
 }
 
 // Channels c .. c + 3 of tokens [ta, tb) of x (rows of x_stride values, whose channel 0 is x[0]); emit(t, y) gets the
-// four results of token t (all threads of a warp call it together for the same t).  conv_state [slots, TAPS - 1, C] holds
-// the inputs before each sequence's first token of the step.  `single` (as many tokens as sequences, [ta, tb) one token): the
+// four results of token t: all threads of a warp call it together for the same t, since the lanes of a head sum among
+// themselves, so threads without channels of their own (live = false) go the same way and only store nothing.  conv_state
+// [slots, TAPS - 1, C] holds the inputs before each sequence's first token of the step.  `single` (as many tokens as sequences, [ta, tb) one token): the
 // thread that reads a sequence's window is the only one that does, so it also moves the window on.
 template <int TAPS, typename TA, typename Emit>
 __device__ __forceinline__ void conv_tokens(const TA* __restrict__ x, long long x_stride, const float* __restrict__ conv_w,
                                             const float* __restrict__ conv_b, float* conv_state,
                                             const int* __restrict__ cu, const int* __restrict__ context_lens,
                                             const int* __restrict__ state_slots, int B, int C, int c, int ta, int tb,
-                                            bool single, Emit emit) {
+                                            bool single, bool live, Emit emit) {
   float w[TAPS * 4];
   float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), win[TAPS - 1];
 #pragma unroll
@@ -42,7 +43,7 @@ __device__ __forceinline__ void conv_tokens(const TA* __restrict__ x, long long 
   pdl_wait();
   const TA* xc = x + c;
   int b = seq_of_token(cu, B, ta);
-  for (int t = ta; t < tb; ++b) {
+  for (int t = ta; t < tb && b < B; ++b) {            // (rows behind the last sequence have no window)
     const int t0 = cu[b], t1 = cu[b + 1], slot = state_slots[b];
     const bool carried = slot >= 0 && context_lens[b] - (t1 - t0) > 0;
     float* st = conv_state + (size_t)(carried ? slot : 0) * (TAPS - 1) * C + c;
@@ -80,7 +81,7 @@ __device__ __forceinline__ void conv_tokens(const TA* __restrict__ x, long long 
       }
       t = min(te, t + 4);
     }
-    if (single && slot >= 0) {
+    if (single && live && slot >= 0) {
       float* to = conv_state + (size_t)slot * (TAPS - 1) * C + c;
 #pragma unroll
       for (int s = 0; s < TAPS - 1; ++s) store4(to + (size_t)s * C, win[s]);

@@ -95,7 +95,7 @@ ssm_prep_vec_kernel(const TA* __restrict__ proj, long long stride, const float* 
   const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) << 2;
   if (c >= Cc) return;
   const int dst = c < inner ? 2 * GN + c : (c < inner + GN ? GN + (c - inner) : c - inner - GN);    // rows [C | B | x]
-  conv_tokens<TAPS>(proj + inner, stride, conv_w, conv_b, conv_state, cu_q_lens, context_lens, state_slots, B, Cc, c, ta, tb, single,
+  conv_tokens<TAPS>(proj + inner, stride, conv_w, conv_b, conv_state, cu_q_lens, context_lens, state_slots, B, Cc, c, ta, tb, single, true,
                     [&](int t, float4 y) { store4(cbx + (size_t)t * Cc + dst, y); });
 }
 

@@ -31,8 +31,10 @@ def near(got, want, tol):
     assert err <= tol, f"{err:.2e}"
 
 
-# (tokens of each sequence, tokens it had before): around the eight tokens of a block; a step of single tokens
-STEPS = [([1, 7, 8, 9, 2, 17, 30], [0, 5, 0, 2, 1, 0, 3]), ([1] * 11, [0, 1, 2, 3, 9, 0, 5, 40, 1, 0, 2]), ([64], [0]), ([1, 33], [4, 0])]
+# (tokens of each sequence, tokens it had before): around the tokens of a block; a step of single tokens; as many tokens as
+# sequences, though some have two and some none
+STEPS = [([1, 7, 8, 9, 2, 17, 30], [0, 5, 0, 2, 1, 0, 3]), ([1] * 11, [0, 1, 2, 3, 9, 0, 5, 40, 1, 0, 2]), ([64], [0]), ([1, 33], [4, 0]),
+         ([2, 0, 1], [3, 4, 0])]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
@@ -88,6 +90,25 @@ def test_delta_and_ssm_prep(ops, dtype, taps, step):
         near(dt, step_size, 5e-6)
         near(decay, torch.exp(-torch.exp(a_log.double()) * step_size), 5e-6)
         near(state, after, 1e-7)
+
+
+@pytest.mark.parametrize("lens", [[5, 20], [1, 1, 1]])
+def test_rows_behind_the_last_sequence_change_nothing(ops, lens):
+    """More rows than the sequences have tokens: the sequences' rows and windows are as without them."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    G, H, d, dv, T, B, more = 1, 3, 32, 4, sum(lens), len(lens), 19
+    C = 2 * G * d + H * dv
+    x, w = torch.randn(T + more, C, device="cuda", generator=gen), torch.randn(C, 4, device="cuda", generator=gen)
+    zb, za, a_log, dt_b = (torch.randn(*s, device="cuda", generator=gen) for s in ((T + more, H), (T + more, H), (H,), (H,)))
+    cu, ctx, slots = i32([sum(lens[:b]) for b in range(B + 1)]), i32([n + 3 for n in lens]), i32(list(range(B)))
+    start = torch.randn(B, 3, C, device="cuda", generator=gen)
+    got = []
+    for rows in (T, T + more):
+        state, out, beta, decay = start.clone(), *(torch.empty(rows, n, device="cuda") for n in (C, H, H))
+        ops.delta_prep(x[:rows], w, state, zb[:rows], za[:rows], a_log, dt_b, cu, ctx, slots, B, G, H, d, dv, out, beta, decay)
+        got.append((out[:T], beta[:T], decay[:T], state))
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=1e-6, atol=1e-6)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
