@@ -25,6 +25,22 @@ def _as_i64(x: int) -> int:
     return x - (1 << 64) if x >> 63 else x
 
 
+def pack(params: Sequence[SamplingParams], draw_index: Sequence[int], R: int) -> np.ndarray:
+    """What a step of R rows hands to the device, in one buffer for one copy: [seeds | draws] of 64 bits, then [top_k],
+    [temperature], [top_p] of 32.  Entries beyond the rows are passed over."""
+    params, draws = list(params)[:R], list(draw_index)[:R]
+    if len(params) < R or len(draws) < R:
+        raise ValueError(f"{R} rows to sample, parameters for {len(params)} and draws for {len(draws)}")
+    host = np.empty(7 * R, dtype=np.int32)
+    wide, f32 = host[:4 * R].view(np.int64), host[5 * R:].view(np.float32)
+    wide[:R] = [_as_i64(p.seed or 0) for p in params]
+    wide[R:] = draws
+    host[4 * R:5 * R] = [p.top_k for p in params]
+    f32[:R] = [p.temperature for p in params]
+    f32[R:] = [p.top_p for p in params]
+    return host
+
+
 class Sampler:
     """Samples on the device into ``tokens`` (a buffer the next step can read from
     directly) and copies the result to one of two pinned host buffers; ``wait``
@@ -53,15 +69,7 @@ class Sampler:
         if all(p.greedy for p in params):
             ops.argmax(logits, out)
         else:
-            # one buffer, one copy: [seeds | draws] of 64 bits, then [top_k], [temperature], [top_p] of 32
-            host = np.empty(7 * R, dtype=np.int32)
-            wide, f32 = host[:4 * R].view(np.int64), host[5 * R:].view(np.float32)
-            wide[:R] = [_as_i64(p.seed or 0) for p in params]
-            wide[R:] = draw_index
-            host[4 * R:5 * R] = [p.top_k for p in params]
-            f32[:R] = [p.temperature for p in params]
-            f32[R:] = [p.top_p for p in params]
-            dev = torch.from_numpy(host).to(self.device, non_blocking=True)
+            dev = torch.from_numpy(pack(params, draw_index, R)).to(self.device, non_blocking=True)
             wide, f32 = dev[:4 * R].view(torch.int64), dev[5 * R:].view(torch.float32)
             ops.sample(logits, f32[:R], dev[4 * R:5 * R], f32[R:], wide[:R], wide[R:], out)
         self._host[slot][:R].copy_(out, non_blocking=True)
