@@ -214,7 +214,7 @@ delta_recur_kernel(const float* __restrict__ qkv, const float* __restrict__ beta
   const int C = 2 * G * d + H * dv;
   const int slot = state_slots[b];
   const int t0 = cu_q_lens[b], qlen = cu_q_lens[b + 1] - t0;
-  if (slot < 0 || qlen <= 0 || qlen > max_len) { pdl_trigger(); return; }
+  if (slot < 0 || qlen <= 0 || qlen > max_len) { pdl_trigger(); pdl_wait(); return; }      // (the grid is not done before the one ahead of it)
   const int start = context_lens[b] - qlen;
   const int kvh = h / (H / G);
   const int dp = DPT * DR_LANES;                 // d rounded up to what the lanes hold
@@ -547,12 +547,12 @@ static int delta_recur_launch(const float* qkv, const float* beta, const float* 
   return gg_check_launch("delta_recur");
 }
 
-// max_len > 0: sequences with more tokens in this step are left alone.
+// max_len > 0: sequences with more tokens in this step are left alone; 0: none is.
 extern "C" int gg_delta_recur(const float* qkv, const float* beta, const float* decay, float* state,
                               const int* cu_q_lens, const int* context_lens, const int* state_slots, int B, int G, int H,
                               int d, int dv, int dw, int plain, int max_len, int T, float* o_raw, cudaStream_t stream) {
-  const bool long_rows = T > 4 * B && max_len != 1;
-  if (max_len <= 0) max_len = T;              // more than a few tokens a sequence: a step with prompt portions
+  const bool long_rows = T > 4 * B && max_len != 1;       // more than a few tokens a sequence: a step with prompt portions
+  if (max_len <= 0) max_len = T;
   GG_REQUIRE(dw == 1 || dw == d, "delta_recur: a decay per head (1) or per key channel (%d), not %d", d, dw);
   GG_REQUIRE(!plain || dw == 1, "delta_recur: the plain recurrence takes a decay per head");
   GG_REQUIRE(B > 0 && G > 0 && H > 0 && H % G == 0 && d > 0 && dv > 0, "delta_recur: bad sizes B=%d G=%d H=%d d=%d dv=%d", B, G, H, d, dv);
