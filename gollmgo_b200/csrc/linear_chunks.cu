@@ -295,12 +295,12 @@ linear_products_kernel(const LinearArgs p) {
   if (warp == LC_ISSUER) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_trigger();                                     // (not before: a kernel behind could take the tensor memory and wait for this one)
   }
   const int b = p.tile_seq[blockIdx.x], q0 = p.tile_q0[blockIdx.x], h0 = blockIdx.y * p.heads, m0 = blockIdx.z * 128;
   const int qlen = p.cu_q_lens[b + 1] - p.cu_q_lens[b], t0 = p.cu_q_lens[b] + q0, n = min(LC_C, qlen - q0);
   const int d = p.d, dv = p.dv, cols = p.heads * dv, steps = (n + 31) / 32;
   const size_t place = blockIdx.x;
-  pdl_trigger();
   pdl_wait();
   // the first step's rows and the decays are on their way together
   const float* kb = p.rows + (size_t)t0 * p.row_stride + p.k_col + (size_t)(h0 / (p.H / p.G)) * d + m0;
@@ -453,12 +453,12 @@ linear_rows_kernel(const LinearArgs p) {
   if (warp == LC_ISSUER) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_trigger();                                     // (not before: a kernel behind could take the tensor memory and wait for this one)
   }
   const int b = p.tile_seq[blockIdx.x], q0 = p.tile_q0[blockIdx.x], h0 = blockIdx.y * p.heads;
   const int qlen = p.cu_q_lens[b + 1] - p.cu_q_lens[b], t0 = p.cu_q_lens[b] + q0, n = min(LC_C, qlen - q0);
   const bool carry = p.context_lens[b] - qlen + q0 > 0;
   const int d = p.d, dv = p.dv, kd = (d + 31) / 32, kj = (n + 31) / 32;
-  pdl_trigger();
   pdl_wait();
   LcTokens tokens;
   if (warp < p.heads) tokens = lc_tokens(p, t0, n, h0 + warp);       // (at most eight heads; used below)
