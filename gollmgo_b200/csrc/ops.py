@@ -783,6 +783,9 @@ def rope_kv_write_x(qkv: torch.Tensor, positions: torch.Tensor, slot_mapping: Op
 ATTN_MMA_X_MAX_DIST = 16384
 
 
+_NO_TILES = (_NULL, _NULL, 0, 0, 0, _NULL)
+
+
 def attn_prefill_x(q: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache: torch.Tensor,
                    block_tables: torch.Tensor, bt_stride: int, cu_q_lens: torch.Tensor, context_lens: torch.Tensor,
                    tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, out: torch.Tensor, nh: int, nkv: int,
@@ -814,11 +817,10 @@ def attn_prefill_x(q: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache:
     use_tc = tile128_seq is not None and kcache.dtype == torch.bfloat16
     if use_tc:
         tc_launched = True
+    long = (_p(tile128_seq), _p(tile128_q0), num_tiles128, q.shape[0], kcache.shape[0], _p(tc_status(q.device))) if use_tc else _NO_TILES
     _check(lib().gg_attn_prefill_x(_p(q), ctypes.c_longlong(q_stride), _p(kcache), _p(vcache), dtype_code(kcache.dtype),
                                    _p(block_tables), bt_stride, _p(cu_q_lens), _p(context_lens), _p(tile_seq),
-                                   _p(tile_q0), num_tiles, _p(tile64_seq), _p(tile64_q0), num_tiles64, int(allow_mma),
-                                   _p(tile128_seq) if use_tc else _NULL, _p(tile128_q0) if use_tc else _NULL, num_tiles128,
-                                   q.shape[0], kcache.shape[0], _p(tc_status(q.device)) if use_tc else _NULL,
+                                   _p(tile_q0), num_tiles, _p(tile64_seq), _p(tile64_q0), num_tiles64, int(allow_mma), *long,
                                    _p(out), int(out.dtype == torch.float32 and kcache.dtype != torch.float32),
                                    nh, nkv, d, dv, v_share, page_size, window, ctypes.c_float(scale),
                                    ctypes.c_float(softcap), int(keep_first), int(sigmoid_weights), _p(head_bias),
@@ -832,12 +834,19 @@ def attn_mma_x_chunk_sink() -> bool:
     return bool(lib().gg_attn_mma_x_chunk_sink())
 
 
+_NO_TEMPERATURE = (ctypes.c_float(0.0), ctypes.c_float(0.0))
+
+
 def _temperature(temperature):
-    coef, every = temperature or (0.0, 0.0)
+    if not temperature:
+        return _NO_TEMPERATURE
+    coef, every = temperature
     return ctypes.c_float(coef), ctypes.c_float(every)
 
 
 def _attn_extras(nh, head_bias, dist_bias, dist_bucket, sink=None, slopes=None) -> None:
+    if head_bias is None and dist_bias is None and sink is None and slopes is None and dist_bucket is None:
+        return
     _cuda(head_bias, dist_bias, dist_bucket, sink, slopes)
     if slopes is not None and (slopes.dtype != torch.float32 or slopes.numel() != nh):
         raise KernelError("attention: the slopes are float32 [heads]")

@@ -20,6 +20,9 @@ class QueryTiles:
     most_keys_first: bool = False
     at_least: int = 0
 
+    def __hash__(self):          # (a layer asks for its lists several times a step: the generated one builds a tuple each time)
+        return self.height
+
 
 @dataclass(frozen=True)
 class StepFacts:
