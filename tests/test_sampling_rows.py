@@ -27,7 +27,7 @@ def kept_probabilities(row, t, k, p):
 
 
 # vocabulary, rows, spread of the logits, (top_k, top_p) in turn: candidates above the threads' maxima; more than there are
-# threads; a leading byte that fits in shared memory, does not fit (flat logits) or fits only where few rows share it;
+# threads; a leading byte that fits in shared memory or does not (flat logits);
 # odd widths (rows that start off a 16-byte border); fewer values than threads; rows whose integer sums need 64 bits
 CASES = [(40000, 40, 2.5, [(50, 0.9), (1024, 0.0), (1025, 0.8), (3000, 0.95), (0, 0.9), (0, 0.0), (1, 0.5)]),
          (128256, 40, 2.5, [(0, 0.9), (400, 0.8), (0, 0.99), (20000, 0.5)]),
