@@ -273,8 +273,9 @@ class BatchBuilder:
         T = sum(q_lens)
         portions = [b for b in range(B) if q_lens[b] > 1]
         tile_lists = []
+        most_keys = max((q_starts[b] + q_lens[b] for b in portions), default=0)
         for need in self.query_tiles:
-            tl = [(b, q0) for b in portions if q_lens[b] >= need.at_least for q0 in range(0, q_lens[b], need.height)]
+            tl = [] if most_keys <= need.beyond_keys else [(b, q0) for b in portions if q_lens[b] >= need.at_least for q0 in range(0, q_lens[b], need.height)]
             if need.most_keys_first:
                 tl.sort(key=lambda t: -(q_starts[t[0]] + t[1]))
             tile_lists.append(tl)

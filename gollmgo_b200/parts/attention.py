@@ -40,6 +40,11 @@ TILES_GENERAL, TILES_MMA, TILES_TC = QueryTiles(16), QueryTiles(64), QueryTiles(
 # the mma.sync kernel of the general path (values of another size, capped scores): its tiles differ in
 # length by the causal mask alone, so the long ones go first and the short ones fill the end of the launch
 TILES_MMA_X = QueryTiles(64, most_keys_first=True)
+# ... and its tiles on tcgen05: only where some portion sees more than 144 keys, since a second step of 128 keys that is nearly
+# empty is not worth the kernel's start.  A layer on a B200, us, tcgen05 / mma.sync, 32 heads of 128 with a cap: 8 x 32 tokens
+# 57 / 39, 32 x 64 194 / 157, 32 x 128 307 / 318, 32 x 32 after 100 179 / 137, 8 x 160 128 / 135, 32 x 160 418 / 441; 16 heads:
+# 16 x 64 54 / 37, 16 x 96 60 / 59, 32 x 128 126 / 124, 8 x 160 52 / 58
+TILES_TC_X = QueryTiles(128, most_keys_first=True, beyond_keys=144)
 FORCED_SPLITS = int(os.environ.get("GOLLMGO_B200_DECODE_SPLITS", "0"))   # for measurements: this count, whatever the batch
 CTAS_PER_SM = 3            # decode attention CTAs resident on one SM (csrc/attention_mma.cu)
 TILE_KEYS = 64             # keys of one tile of the decode kernels
@@ -222,7 +227,7 @@ class Attention:
             if self._mma_x:
                 need.append(TILES_MMA_X)
                 if ATTN_POLICY == "auto":
-                    need.append(TILES_TC)
+                    need.append(TILES_TC_X)
             return need
         if self.ctx.act_dtype == torch.bfloat16 and self.d in (64, 128) and ATTN_POLICY != "general":
             need.append(TILES_MMA)
@@ -236,12 +241,13 @@ class Attention:
 
     def long_tiles(self, batch):
         """The tiles of 128 query rows for a prompt step of the general path that runs on tcgen05 (ops.attn_prefill_x), as its
-        arguments; empty where the mma.sync kernel is the faster one (_few_short_tiles; at least two heads must share a kv
-        head for the other kernel to take the step at all)."""
-        if not self._mma_x:
-            return {}
-        t128 = batch.tiles.get(TILES_TC)
-        if t128 is None or self._few_short_tiles(t128.count, batch):
+        arguments; empty where the mma.sync kernel is the faster one: few keys (TILES_TC_X), or few tiles of no more than 256
+        keys, where the plain attention's line lies (_few_short_tiles; with options, us, tcgen05 / mma.sync: 32 heads, one
+        portion of 192 tokens 51 / 49, 256 55 / 57, 384 62 / 72, two of 160 62 / 56, 32 after 200 54 / 47; 16 heads: 33 / 35,
+        35 / 41, 39 / 53, 35 / 37, 35 / 39).  At least two heads must share a kv head for the other kernel to take the step
+        at all."""
+        t128 = batch.tiles.get(TILES_TC_X) if self._mma_x else None
+        if t128 is None or not t128.count or self._few_short_tiles(t128.count, batch):
             return {}
         return dict(tile128_seq=t128.seq, tile128_q0=t128.q0, num_tiles128=t128.count)
 

@@ -14,11 +14,13 @@ class QueryTiles:
     """An index list a mixer asks the batch builder for: the query rows of every prompt
     portion (a sequence with more than one token in the step) cut into tiles of ``height``
     rows, as (sequence, first row) pairs; ``most_keys_first`` orders them by how many keys
-    they attend to, longest first; ``at_least``: only portions of so many rows (0: all).  A mixer names the lists it wants in ``query_tiles()``;
+    they attend to, longest first; ``at_least``: only portions of so many rows (0: all);
+    ``beyond_keys``: no tiles unless some portion attends to more keys than that.  A mixer names the lists it wants in ``query_tiles()``;
     the step's batch then holds each under ``batch.tiles[that QueryTiles]``."""
     height: int
     most_keys_first: bool = False
     at_least: int = 0
+    beyond_keys: int = 0
 
     def __hash__(self):          # (a layer asks for its lists several times a step: the generated one builds a tuple each time)
         return self.height

@@ -26,7 +26,7 @@ import torch
 from ..cache import PagedKVNeed
 from ..csrc import ops
 from ..weights import WeightSpec
-from .attention import ATTN_POLICY, TILES_GENERAL, TILES_MMA_X, TILES_TC, Attention, context_tiles, decode_splits
+from .attention import ATTN_POLICY, TILES_GENERAL, TILES_MMA_X, TILES_TC_X, Attention, context_tiles, decode_splits
 from .linear import linear
 from .registry import register_mixer
 
@@ -74,7 +74,7 @@ class NormedAttention(Attention):
 
     def query_tiles(self):
         need = [TILES_GENERAL, TILES_MMA_X] if self._mma_x else [TILES_GENERAL]
-        return need + [TILES_TC] if self._mma_x and ATTN_POLICY == "auto" else need
+        return need + [TILES_TC_X] if self._mma_x and ATTN_POLICY == "auto" else need
 
     def _splits(self, n_dec, max_context):
         return decode_splits(n_dec, self._ctas_per_split, self.num_sms, self._cluster_cap,
