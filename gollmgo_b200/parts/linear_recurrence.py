@@ -15,9 +15,10 @@ from .context import QueryTiles
 #             16 heads of 132     192: 69 / 60   256: 77 / 72    320: 82 / 86      16 x 256: 462 / 628   32 x 128: 496 / 630
 #             32 heads of 132     192: 109 / 113 256: 119 / 131  512: 156 / 217    16 x 256: 1074 / 1414
 #   64 keys:  64 heads of 64      256: 77 / 72   384: 93 / 93    512: 102 / 115    16 x 256: 502 / 464   8 x 512: 492 / 473
-# (64 keys: the walk's cost goes with the keys, a chunk's with its rows.)
+# (64 keys: the walk's cost goes with the keys, a chunk's with its rows.  A line at 512 there would leave the portions below it
+# walking alone behind the chunks of a longer one: 364 + 218 + 582 + 436 tokens 296, all in chunks 231, all walking 328.)
 def chunks_from(d):
-    return 256 if d > 64 else 512
+    return 256 if d > 64 else 384
 
 
 class PlainRecurrence:
