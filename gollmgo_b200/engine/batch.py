@@ -39,10 +39,10 @@ class StepEntry:
 
 class TileList:
     """One QueryTiles list of a step on the device: tile i covers rows q0[i] .. q0[i] + height
-    of sequence seq[i] (``count`` tiles)."""
+    of sequence seq[i] (``count`` tiles); ``left_out``: how many portions of the step it does not list."""
 
-    def __init__(self, need: QueryTiles, seq: torch.Tensor, q0: torch.Tensor, count: int):
-        self.need, self.seq, self.q0, self.count = need, seq, q0, count
+    def __init__(self, need: QueryTiles, seq: torch.Tensor, q0: torch.Tensor, count: int, left_out: int = 0):
+        self.need, self.seq, self.q0, self.count, self.left_out = need, seq, q0, count, left_out
 
 
 class StepBatch:
@@ -273,9 +273,11 @@ class BatchBuilder:
         T = sum(q_lens)
         portions = [b for b in range(B) if q_lens[b] > 1]
         tile_lists = []
-        most_keys = max((q_starts[b] + q_lens[b] for b in portions), default=0)
+        left_out = []
         for need in self.query_tiles:
-            tl = [] if most_keys <= need.beyond_keys else [(b, q0) for b in portions if q_lens[b] >= need.at_least for q0 in range(0, q_lens[b], need.height)]
+            chosen = need.chosen(portions, q_lens, q_starts)
+            left_out.append(len(portions) - len(chosen))
+            tl = [(b, q0) for b in chosen for q0 in range(0, q_lens[b], need.height)]
             if need.most_keys_first:
                 tl.sort(key=lambda t: -(q_starts[t[0]] + t[1]))
             tile_lists.append(tl)
@@ -369,7 +371,7 @@ class BatchBuilder:
         sb.token_src = v(lay.token_src, Tp) if (has_src or static_dev is not None) else None
         sb.cu_q_lens, sb.context_lens = v(lay.cu_q_lens, Bp + 1), v(lay.context_lens, Bp)
         sb.state_slots, sb.logit_rows = v(lay.state_slots, Bp), v(lay.logit_rows, R)[:R]
-        sb.tiles = {need: TileList(need, v(lay.tile_seq[i], counts[i]), v(lay.tile_q0[i], counts[i]), counts[i])
+        sb.tiles = {need: TileList(need, v(lay.tile_seq[i], counts[i]), v(lay.tile_q0[i], counts[i]), counts[i], left_out[i])
                     for i, need in enumerate(self.query_tiles)}
         sb.dec_seqs = v(lay.dec_seqs, nd)
         sb.slot_mapping = [v(o, Tp) for o in lay.slot_mapping]

@@ -25,6 +25,12 @@ class QueryTiles:
     def __hash__(self):          # (a layer asks for its lists several times a step: the generated one builds a tuple each time)
         return self.height
 
+    def chosen(self, portions, q_lens, q_starts):
+        """Those of the step's ``portions`` (sequences, of q_lens rows behind q_starts cached ones) whose tiles are listed."""
+        if self.beyond_keys and max((q_starts[b] + q_lens[b] for b in portions), default=0) <= self.beyond_keys:
+            return []
+        return [b for b in portions if q_lens[b] >= self.at_least] if self.at_least else portions
+
 
 @dataclass(frozen=True)
 class StepFacts:

@@ -26,18 +26,18 @@ from ..csrc import ops
 from ..weights import WeightSpec
 from .context import QueryTiles
 from .linear import linear
+from .linear_recurrence import ChunkTiles
 from .registry import build_position, register_mixer
 
-# Portions of so many tokens take the tensor-core kernels (bfloat16 models, sizes that linear_chunks_ok names).  A portion's own
-# length decides, so its sums do not depend on what else is in the step.  Us for a layer on a B200, tensor cores / packed
+# Portions of so many tokens take the tensor-core kernels (bfloat16 models, sizes that linear_chunks_ok names), and so do all of a
+# step that has so many together in few or well-filled chunks (ChunkTiles).  Us for a layer on a B200, tensor cores / packed
 # float32, steps of one portion, and of several after a context:
 #   16 heads 128 x 256    64: 55 / 53   128: 70 / 72    256: 85 / 86    512: 99 / 109    8 x 64: 95 / 121   8 x 128: 137 / 183
 #                         64 x 2: 581 / 261   32 x 16: 300 / 204   32 x 64: 444 / 366   32 x 128: 633 / 616   20 x 192: 541 / 582
 #   16 heads 128 x 128    64: 40 / 39   128: 50 / 52    256: 59 / 60    512: 69 / 79     8 x 64: 64 / 74    8 x 128: 91 / 117
 #   32 heads 128 x 256    64: 99 / 98   128: 116 / 121  256: 136 / 146  512: 171 / 225   32 x 64: 1076 / 842   32 x 128: 1594 / 1564
 TC_FROM = 128
-CHUNKS = QueryTiles(ops.RETENTION_CHUNK)          # the chunks of prompt portions: of the packed float32 kernels (which pass over
-TC_CHUNKS = QueryTiles(ops.LINEAR_CHUNK, at_least=TC_FROM)         # those of longer portions), and of the tensor-core ones
+CHUNKS = QueryTiles(ops.RETENTION_CHUNK)          # the chunks of prompt portions, of the packed float32 kernels
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "gate": "g", "o": "o"}
 
@@ -76,6 +76,7 @@ class Retention:
         self.chunked = self.dv <= ops.RETENTION_MAX_V
         self.tc = self.chunked and ctx.act_dtype != torch.float32 and ops.linear_chunks_ok(self.d, self.dv)
         if self.tc:                                  # (the one scratch: the two forms of a step follow one another)
+            self.tc_chunks = ChunkTiles(ops.LINEAR_CHUNK, at_least=TC_FROM, rows=TC_FROM, most=T // ops.LINEAR_CHUNK + T // TC_FROM)
             ws.reserve("ret_states", ops.linear_scratch_floats(T, T // TC_FROM, self.nh, self.d, self.dv), torch.float32)
         if self.chunked:
             ws.reserve("ret_states", ops.retention_scratch_floats(T, ctx.max_seqs, self.nh, self.d, self.dv), torch.float32)
@@ -89,7 +90,7 @@ class Retention:
         return FixedStateNeed((self.nh, self.dv, self.d), "float32")
 
     def query_tiles(self):
-        return ([CHUNKS] if self.chunked else []) + ([TC_CHUNKS] if self.tc else [])
+        return ([CHUNKS] if self.chunked else []) + ([self.tc_chunks] if self.tc else [])
 
     def weights(self):
         n, H, qk, vv = self.names, self.hidden, self.nh * self.d, self.nh * self.dv
@@ -130,13 +131,14 @@ class Retention:
                     raise RuntimeError("the step's batch was built without the index list this mixer declares in "
                                        "query_tiles(): give it to the BatchBuilder (query_tiles=...)")
                 seqs = (batch.cu_q_lens, batch.context_lens, batch.state_slots, batch.num_seqs)
-                tiles, max_len = batch.tiles.get(TC_CHUNKS) if self.tc else None, 0
+                tiles, max_len = batch.tiles.get(self.tc_chunks) if self.tc else None, 0
                 if tiles is not None and tiles.count:
-                    scratch = ws.get("ret_states", 1, ops.linear_scratch_floats(T, T // TC_FROM, H, d, dv))
+                    most = self.ctx.max_tokens
+                    scratch = ws.get("ret_states", 1, ops.linear_scratch_floats(most, most // TC_FROM, H, d, dv))
                     if ops.linear_retention(rows, self.log2_decays, state, scratch, tiles.seq, tiles.q0, tiles.count, *seqs, gate,
                                             self.eps, H, d, dv, y):
                         max_len = TC_FROM - 1
-                if max_len == 0 or any(1 < n <= max_len for n in batch.q_lens):
+                if max_len == 0 or tiles.left_out:
                     tiles = batch.tiles[CHUNKS]
                     scratch = ws.get("ret_states", 1, ops.retention_scratch_floats(T, batch.num_seqs, H, d, dv))
                     ops.retention_chunks(rows, self.log2_decays, state, scratch, tiles.seq, tiles.q0, tiles.count, *seqs, gate, self.eps,

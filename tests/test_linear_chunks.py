@@ -134,7 +134,8 @@ def test_mixers_recurrence_takes_chunks_for_long_portions(ops, monkeypatch, lens
     tiles = [(b, x) for b, n in enumerate(lens) if n > 1 and n >= need.at_least for x in range(0, n, 128)]
     batch = SimpleNamespace(cu_q_lens=cu, context_lens=ctx, state_slots=i32(list(range(B))), num_seqs=B, q_lens=lens,
                             num_portions=sum(n > 1 for n in lens), num_decode=sum(n == 1 for n in lens),
-                            tiles={need: SimpleNamespace(seq=i32([t[0] for t in tiles]), q0=i32([t[1] for t in tiles]), count=len(tiles))})
+                            tiles={need: SimpleNamespace(seq=i32([t[0] for t in tiles]), q0=i32([t[1] for t in tiles]), count=len(tiles),
+                                                   left_out=sum(1 < n < need.at_least for n in lens))})
     calls, real = [], ops.linear_chunks
     monkeypatch.setattr(ops, "linear_chunks", lambda *a: calls.append(1) or real(*a))
     got, want = [(state.clone(), torch.full((T, H * dv), float("nan"), device="cuda")) for _ in range(2)]

@@ -28,21 +28,54 @@ def test_models_in_float32_keep_float32_products(kind):
     assert not chunk_lists(mixer(kind, torch.float32)[0])
 
 
-@pytest.mark.parametrize("kind", sorted(MIXERS))
-def test_a_portion_s_own_length_decides(kind):
+def listed(part, lens):
+    """The sequences whose chunks a step of these portions lists, all of their chunks in order; and the portions it leaves out."""
     from gollmgo_b200.cache import CacheManager
     from gollmgo_b200.engine import BatchBuilder, StepEntry
-    part, _ = mixer(kind, torch.bfloat16)
     need, = chunk_lists(part)
-    assert need.at_least > 1
-    lens = [need.at_least, 1, need.at_least - 1, 2, need.at_least + 129]
     cm = CacheManager([part.cache_need()], 16, 8, len(lens), dtype=torch.bfloat16, device="cpu")
     for i in range(len(lens)):
         cm.admit(i)
     batch = BatchBuilder(cm, "cpu", query_tiles=part.query_tiles()).build([StepEntry(i, [0] * n, [0]) for i, n in enumerate(lens)])
     tiles = batch.tiles[need]
-    want = [(b, q) for b in (0, 4) for q in range(0, lens[b], ops.LINEAR_CHUNK)]
-    assert tiles.count == len(want) and list(zip(tiles.seq.tolist(), tiles.q0.tolist()))[:tiles.count] == want
+    seqs = sorted(set(tiles.seq.tolist()[:tiles.count]))
+    assert list(zip(tiles.seq.tolist(), tiles.q0.tolist()))[:tiles.count] == [(b, q) for b in seqs for q in range(0, lens[b], ops.LINEAR_CHUNK)]
+    assert tiles.left_out == sum(n > 1 for n in lens) - len(seqs)
+    return seqs
+
+
+@pytest.mark.parametrize("kind", sorted(MIXERS))
+def test_long_portions_and_few_short_ones_beside_them(kind):
+    part, _ = mixer(kind, torch.bfloat16, max_seqs=64)
+    L = chunk_lists(part)[0].at_least
+    assert listed(part, [L, 1, L - 1, 2, L + 129]) == [0, 2, 3, 4]                   # few chunks: the short ones beside the long
+    assert listed(part, [L] + [8] * 40) == [0]                                       # many nearly empty ones: on their own
+    assert listed(part, [1, L] + [100] * 9) == list(range(1, 11))                    # many well-filled ones
+    assert listed(part, [L] + [40] * 9 + [L]) == [0, 10]
+    assert listed(part, [1, 1]) == [] and listed(part, [20, 30, 1]) == []
+    # portions that are only long together: retention alone
+    assert listed(part, [L - 1, L - 1]) == ([0, 1] if kind == "retention" else [])
+    assert listed(part, [16] * 20) == []
+
+
+@pytest.mark.parametrize("kind", sorted(MIXERS))
+def test_chunks_fit_in_the_scratch_whatever_the_step(kind):
+    import random
+    rng = random.Random(5)
+    part, ctx = mixer(kind, torch.bfloat16, max_tokens=1024, max_seqs=64)
+    need, = chunk_lists(part)
+    name = "ret_states" if kind == "retention" else "linear_states"
+    heads, d, dv = (part.nh, part.d, part.dv) if kind == "retention" else part.recurrence.sizes[1:]
+    room = ctx.workspace._want[name][0] // (heads * (d * dv + 4))
+    for _ in range(3000):
+        lens, left = [], 1024
+        while left > 1 and len(lens) < 64:
+            n = min(left, rng.choice([2, 5, 20, 64, 65, 129, 130, 257, need.at_least, need.at_least + 1, rng.randint(2, 600)]))
+            if n > 1:
+                lens.append(n)
+            left -= n
+        chosen = need.chosen(list(range(len(lens))), lens, [0] * len(lens))
+        assert sum(-(-lens[b] // ops.LINEAR_CHUNK) for b in chosen) <= room
 
 
 @pytest.mark.parametrize("kind", ["mamba2", "mlstm"])
@@ -65,7 +98,8 @@ def test_long_short_and_single_portions_hand_one_state_on(kind):
     from gollmgo_b200.cache import CacheManager
     from gollmgo_b200.engine import BatchBuilder, StepEntry
     parts.set_matmul_precision()
-    steps = [[300, 40, 1, 130], [1, 280, 129, 2], [1, 1, 1, 1], [600, 1, 20, 300], [2, 255, 256, 1]]
+    # all in chunks; divided; single tokens; divided; all in chunks
+    steps = [[300, 40, 1, 130, 1, 1, 1, 1], [300, 8, 8, 8, 8, 8, 8, 1], [1] * 8, [2, 600, 1, 20, 300, 2, 2, 2], [2, 255, 256, 1, 1, 1, 1, 1]]
     gen = torch.Generator(device="cuda").manual_seed(7)
     weights, sides, calls = {}, [], []
     for chunks in (True, False):
@@ -80,8 +114,8 @@ def test_long_short_and_single_portions_hand_one_state_on(kind):
                 part.tc = False
             else:
                 part.recurrence.chunks = None
-        cm = CacheManager([part.cache_need()], 16, 8, 4, dtype=torch.bfloat16, device="cuda")
-        for i in range(4):
+        cm = CacheManager([part.cache_need()], 16, 8, 8, dtype=torch.bfloat16, device="cuda")
+        for i in range(8):
             cm.admit(i)
         view = cm.cache_view(0, part.cache_need())
         sides.append((part, BatchBuilder(cm, "cuda", query_tiles=part.query_tiles()), view))
@@ -103,4 +137,4 @@ def test_long_short_and_single_portions_hand_one_state_on(kind):
         for a, b in zip(got[0][1:], got[1][1:]):
             assert float((a.float() - b.float()).norm() / b.float().norm()) < 2e-5
     assert int(ops.tc_status("cuda")[0]) == 0
-    assert calls == [lens for lens in steps if max(lens) >= chunk_lists(sides[0][0])[0].at_least]
+    assert calls == [lens for lens in steps if max(lens) > 255]
