@@ -244,21 +244,29 @@ class Attention:
         arguments; empty where the mma.sync kernel is the faster one: few keys (TILES_TC_X), or few tiles of no more than 256
         keys, where the plain attention's line lies (_few_short_tiles; with options, us, tcgen05 / mma.sync: 32 heads, one
         portion of 192 tokens 51 / 49, 256 55 / 57, 384 62 / 72, two of 160 62 / 56, 32 after 200 54 / 47; 16 heads: 33 / 35,
-        35 / 41, 39 / 53, 35 / 37, 35 / 39).  At least two heads must share a kv head for the other kernel to take the step
-        at all."""
+        35 / 41, 39 / 53, 35 / 37, 35 / 39).  A window or chunk of fewer than 128 keys leaves either of the kernel's steps of
+        128 half empty (32 heads, window 64: one portion of 2048 179 / 174, of 300 66 / 50; window 128: 181 / 193, 66 / 52;
+        window 256: 184 / 229, 65 / 62; chunks of 64: 207 / 200, 72 / 56).  At least two heads must share a kv head for the
+        other kernel to take the step at all."""
         t128 = batch.tiles.get(TILES_TC_X) if self._mma_x else None
-        if t128 is None or not t128.count or self._few_short_tiles(t128.count, batch):
+        if t128 is None or not t128.count:
+            return {}
+        reach = min(x for x in (self.window, getattr(self, "chunk", 0), 1 << 30) if x)
+        if reach < 128 or self._few_short_tiles(t128.count, batch, reach):
             return {}
         return dict(tile128_seq=t128.seq, tile128_q0=t128.q0, num_tiles128=t128.count)
 
-    def _few_short_tiles(self, tiles128: int, batch) -> bool:
+    def _few_short_tiles(self, tiles128: int, batch, reach: int = 1 << 30) -> bool:
         """Prompt portions that leave the tcgen05 kernel's tiles (128 rows of two heads) on fewer
         than half of the SMs, with at most 256 keys each: the mma.sync kernel's tiles of 64 rows
         of one head spread the same work over four times the CTAs and start faster.  Measured on
         whole prompt steps of the Llama-3.1-8B shape (ms, tcgen05 / mma.sync): 64 tokens 4.10 /
-        3.84, 128 tokens 4.45 / 4.24, 256 tokens 5.2-5.6 / 5.3-5.4, 512 tokens 8.3-8.5 / 8.6."""
+        3.84, 128 tokens 4.45 / 4.24, 256 tokens 5.2-5.6 / 5.3-5.4, 512 tokens 8.3-8.5 / 8.6.
+        ``reach``: no query attends to more keys than that."""
         if tiles128 * ((self.nh + 1) // 2) * 2 > self.num_sms:
             return False
+        if reach <= SHORT_PROMPT_KEYS:
+            return True
         for s, n in zip(batch.q_starts, batch.q_lens):
             if n > 1 and s + n > SHORT_PROMPT_KEYS:
                 return False

@@ -42,5 +42,15 @@ def test_lists_of_one_height_are_lists_of_their_own():
 def test_many_short_portions_with_options_stay_on_mma(lens, held, tc):
     batch = step(lens, held, [TILES_TC_X])
     layer = Attention.__new__(Attention)
-    layer._mma_x, layer.nh, layer.num_sms = True, 32, 148
+    layer._mma_x, layer.nh, layer.num_sms, layer.window = True, 32, 148, None
+    assert bool(layer.long_tiles(batch)) == tc
+
+
+@pytest.mark.parametrize("window,chunk,lens,tc", [(64, 0, [2048], False), (128, 0, [2048], True), (128, 0, [300], False), (257, 0, [300], True),
+                                                  (None, 64, [2048], False), (None, 512, [300], True), (1024, 0, [2048], True),
+                                                  (1024, 100, [2048], False), (0, 0, [300], True)])
+def test_short_windows_and_chunks_stay_on_mma(window, chunk, lens, tc):
+    batch = step(lens, [0] * len(lens), [TILES_TC_X])
+    layer = Attention.__new__(Attention)
+    layer._mma_x, layer.nh, layer.num_sms, layer.window, layer.chunk = True, 32, 148, window, chunk
     assert bool(layer.long_tiles(batch)) == tc
