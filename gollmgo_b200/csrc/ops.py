@@ -49,6 +49,8 @@ def _p(t: Optional[torch.Tensor]):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+# (torch.cuda.current_device() also asks whether CUDA is up, which it is where there are CUDA tensors)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _stream():
@@ -56,7 +58,7 @@ def _stream():
     capture runs on a stream of its own).  The raw accessor costs a tenth of building a
     torch.cuda.Stream object, which matters at a few hundred launches per prompt step."""
     if _raw_stream is not None:
-        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+        return ctypes.c_void_p(_raw_stream(_current_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
