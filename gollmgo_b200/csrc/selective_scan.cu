@@ -10,9 +10,11 @@
 //   scan_run    the recurrence over every sequence's tokens of the step, from the products' rows to the gated rows;
 //               moves the convolution's window on
 //   scan_step   the same for steps of single tokens
-// A channel's N states lie in L neighbouring lanes, K each.  The exponentials bound the long form: N a token and
-// channel at 16 a clock and multiprocessor; the chain from token to token is one multiply-add, so blocks of channels
-// walk the whole sequence and nothing is cut along time.  A2 = A log2(e), so that exp is exp2 of one product.
+// A channel's N states lie in L neighbouring lanes, K each.  What bounds the long form (4096 channels of 16 states, 105 clocks a
+// token and multiprocessor, one walking warp on each scheduler): shared memory first (56 wavefronts a token: a lane reads its
+// step size and input, four values of B and four of C), then the exponentials (32 clocks), and too few warps to hide either's
+// latency.  The chain from token to token is one multiply-add; blocks of channels walk the whole sequence and nothing is cut
+// along time.  A2 = A log2(e), so that exp is exp2 of one product.
 #include "common.cuh"
 
 #define SC_THREADS 128
