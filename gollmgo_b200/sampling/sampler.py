@@ -28,9 +28,11 @@ def _as_i64(x: int) -> int:
 def pack(params: Sequence[SamplingParams], draw_index: Sequence[int], R: int) -> np.ndarray:
     """What a step of R rows hands to the device, in one buffer for one copy: [seeds | draws] of 64 bits, then [top_k],
     [temperature], [top_p] of 32.  Entries beyond the rows are passed over."""
-    params, draws = list(params)[:R], list(draw_index)[:R]
-    if len(params) < R or len(draws) < R:
-        raise ValueError(f"{R} rows to sample, parameters for {len(params)} and draws for {len(draws)}")
+    draws = draw_index
+    if type(params) is not list or type(draws) is not list or len(params) != R or len(draws) != R:
+        params, draws = list(params)[:R], list(draws)[:R]
+        if len(params) < R or len(draws) < R:
+            raise ValueError(f"{R} rows to sample, parameters for {len(params)} and draws for {len(draws)}")
     host = np.empty(7 * R, dtype=np.int32)
     wide, f32 = host[:4 * R].view(np.int64), host[5 * R:].view(np.float32)
     wide[:R] = [_as_i64(p.seed or 0) for p in params]
