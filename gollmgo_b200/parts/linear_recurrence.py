@@ -40,9 +40,10 @@ class ChunkTiles(QueryTiles):
     def chosen(self, portions, q_lens, q_starts):
         lens = [q_lens[b] for b in portions]
         total = sum(lens)
-        if total >= self.rows and max(lens, default=0) >= self.longest:
+        longest = max(lens, default=0)
+        if total >= self.rows and longest >= self.longest:
             tiles = sum(-(-n // self.height) for n in lens)
-            if tiles <= self.most and (tiles <= FEW_CHUNKS or total >= FILLED * tiles):
+            if tiles <= self.most and (tiles <= FEW_CHUNKS or (longest >= self.at_least and total >= FILLED * tiles)):
                 return portions
         return super().chosen(portions, q_lens, q_starts)
 
@@ -63,7 +64,9 @@ class PlainRecurrence:
         self.limit, self.chunks = chunks_from(d), None
         if chunks and ops.linear_chunks_ok(d, dv):
             T = ctx.max_tokens
-            self.chunks = ChunkTiles(ops.LINEAR_CHUNK, at_least=self.limit, longest=self.limit, most=T // ops.LINEAR_CHUNK + T // self.limit)
+            # (64 keys: 203 + 121 + 323 tokens all in chunks 128 us, walked 133; 16 x 256 divided by the line above)
+            self.chunks = ChunkTiles(ops.LINEAR_CHUNK, at_least=self.limit, longest=256, rows=0 if d > 64 else 512,
+                                     most=T // ops.LINEAR_CHUNK + T // self.limit)
             ctx.workspace.reserve("linear_states", ops.linear_scratch_floats(T, T // self.limit, heads, d, dv), torch.float32)
 
     def query_tiles(self):

@@ -58,6 +58,14 @@ def test_long_portions_and_few_short_ones_beside_them(kind):
     assert listed(part, [16] * 20) == []
 
 
+def test_keys_of_64_take_chunks_later():
+    from gollmgo_b200.parts.linear_recurrence import PlainRecurrence
+    need, = PlainRecurrence(BuildContext(torch.bfloat16, "cpu", max_tokens=4096, max_seqs=64, page_size=16), 1, 2, 64, 64).query_tiles()
+    pick = lambda lens: need.chosen(list(range(len(lens))), lens, [0] * len(lens))  # noqa: E731
+    assert pick([383]) == [] and pick([384]) == [0] and pick([256, 255]) == [] and pick([256, 256]) == [0, 1]
+    assert pick([203, 121, 323]) == [0, 1, 2] and pick([256] * 16) == [] and pick([384] + [256] * 8) == list(range(9))
+
+
 @pytest.mark.parametrize("kind", sorted(MIXERS))
 def test_chunks_fit_in_the_scratch_whatever_the_step(kind):
     import random
