@@ -161,29 +161,28 @@ template <int R> struct LcAcross {
       }
   }
   // A product over tokens gives an earlier token's row a weight of 0 for a later one's value, and 0 times infinity or NaN is
-  // NaN: such values leave the tile here (as 0), and first[r] becomes the first token that had one in column r.  One
+  // NaN: after the store such values leave the tile (as 0), and first[r] becomes the first token that had one in column r.  One
   // multiply-add a value finds them.  Returns whether there was any.
-  __device__ __forceinline__ bool take_out(int token, int* first) {
-    const int warp = threadIdx.x >> 5;
-    bool any = false;
+  __device__ __forceinline__ bool take_out(unsigned at, unsigned lo_off, int token, int* first) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float z = 0.f;
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      float z = 0.f;
+    for (int i = 0; i < 2 * N; ++i) { z = fmaf(v[i].x, 0.f, z); z = fmaf(v[i].y, 0.f, z); z = fmaf(v[i].z, 0.f, z); z = fmaf(v[i].w, 0.f, z); }
+    if (z == 0.f) return false;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) { const float4 q = v[2 * i + e]; z = fmaf(q.x, 0.f, z); z = fmaf(q.y, 0.f, z); z = fmaf(q.z, 0.f, z); z = fmaf(q.w, 0.f, z); }
-      if (z == 0.f) continue;
-      any = true;
-      const int r0 = 8 * (warp + 16 * i);
-      auto check = [&](float& x, int r) {
-        if (x * 0.f != 0.f) { atomicMin(first + r, token); x = 0.f; }
+    for (int i = 0; i < 2 * N; ++i) {
+      auto check = [&](float x, int e) {
+        const int r = 8 * (warp + 16 * (i >> 1)) + e;
+        if (x * 0.f == 0.f) return;
+        atomicMin(first + r, token);
+        const unsigned to = at + r * 128 + (((lane >> 2) ^ e) << 4) + ((lane & 3) << 2);
+        lc_sts(to, 0.f);
+        lc_sts(to + lo_off, 0.f);
       };
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        check(v[2 * i + e].x, r0 + 4 * e); check(v[2 * i + e].y, r0 + 4 * e + 1);
-        check(v[2 * i + e].z, r0 + 4 * e + 2); check(v[2 * i + e].w, r0 + 4 * e + 3);
-      }
+      const int e = 4 * (i & 1);
+      check(v[i].x, e); check(v[i].y, e + 1); check(v[i].z, e + 2); check(v[i].w, e + 3);
     }
-    return any;
+    return true;
   }
   // scale(i): the factor of the lane's token in the rows of turn i
   template <typename F> __device__ __forceinline__ void store(unsigned at, unsigned lo_off, F scale) {
@@ -449,7 +448,7 @@ linear_rows_kernel(const LinearArgs p) {
     for (int h = 0; h < 8; ++h) marked_s[h] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int e = threadIdx.x; e < 8 * NB; e += LC_THREADS) first_s[e / NB][e % NB] = LC_C;
+  for (int e = threadIdx.x; e < p.heads * NB; e += LC_THREADS) first_s[e / NB][e % NB] = LC_C;
   if (warp == LC_ISSUER) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_base_s)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -624,8 +623,8 @@ linear_rows_kernel(const LinearArgs p) {
           lc_sts4(to, hi[0], hi[1], hi[2], hi[3]);
           lc_sts4(to + LC_A_BYTES, lo[0], lo[1], lo[2], lo[3]);
         }
-        if (v.take_out(32 * s + lane, first_s[hh])) { *(volatile int*)&marked_s[hh] = 1; __threadfence_block(); }
         v.store(at + 2 * LC_A_BYTES, B_PART, one);
+        if (v.take_out(at + 2 * LC_A_BYTES, B_PART, 32 * s + lane, first_s[hh])) { *(volatile int*)&marked_s[hh] = 1; __threadfence_block(); }
         if (s + 1 < kj) v.load(rv + (size_t)h * dv + (size_t)(32 * (s + 1)) * p.row_stride, p.row_stride, n - 32 * (s + 1), dv);
         ring.give();
       }
