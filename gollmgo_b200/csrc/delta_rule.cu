@@ -493,7 +493,7 @@ extern "C" int gg_delta_prep(const void* x, long long x_stride, int dtype, const
                    ((size_t)x % 16) == 0 && ((size_t)conv_w % 16) == 0 && ((size_t)conv_state % 16) == 0 && ((size_t)qkv_out % 16) == 0 &&
                    (C / 4 + CONV_THREADS - 1) / CONV_THREADS < 65535;
   if (vec) {
-    const int single = T == B, per = T > 4 * B ? CONV_TOKENS : 1;
+    const int single = T == B, per = conv_tokens_a_block(T, B, (C / 4 + CONV_THREADS - 1) / CONV_THREADS);
     const dim3 vgrid((T + per - 1) / per, (C / 4 + CONV_THREADS - 1) / CONV_THREADS + 1);
 #define DP_GO(TA, TAPS)                                                                                                          \
   gg_launch(delta_prep_vec_kernel<TA, TAPS>, vgrid, dim3(CONV_THREADS), 0, stream, (const TA*)x, x_stride, conv_w, conv_state, zb, \

@@ -179,7 +179,7 @@ extern "C" int gg_ssm_prep(const void* proj, long long stride, int dtype, const 
   const int GN = G * N;
   if (taps >= 2 && taps <= 4 && inner % 4 == 0 && GN % 4 == 0 && stride % 4 == 0 && ((size_t)proj % 16) == 0 && ((size_t)conv_w % 16) == 0 &&
       (!conv_b || ((size_t)conv_b % 16) == 0) && ((size_t)conv_state % 16) == 0 && ((size_t)cbx % 16) == 0 && Cc / 4 / CONV_THREADS < 65000) {
-    const int single = T == B, per = T > 4 * B ? CONV_TOKENS : 1;
+    const int single = T == B, per = conv_tokens_a_block(T, B, (Cc / 4 + CONV_THREADS - 1) / CONV_THREADS);
     const dim3 vgrid((T + per - 1) / per, (Cc / 4 + CONV_THREADS - 1) / CONV_THREADS + 1);
 #define SP_GO(TA, TAPS)                                                                                                              \
   gg_launch(ssm_prep_vec_kernel<TA, TAPS>, vgrid, dim3(CONV_THREADS), 0, stream, (const TA*)proj, stride, conv_w, conv_b, conv_state, a_log, \

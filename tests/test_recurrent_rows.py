@@ -34,7 +34,9 @@ def near(got, want, tol):
 # (tokens of each sequence, tokens it had before): around the tokens of a block; a step of single tokens; as many tokens as
 # sequences, though some have two and some none
 STEPS = [([1, 7, 8, 9, 2, 17, 30], [0, 5, 0, 2, 1, 0, 3]), ([1] * 11, [0, 1, 2, 3, 9, 0, 5, 40, 1, 0, 2]), ([64], [0]), ([1, 33], [4, 0]),
-         ([2, 0, 1], [3, 4, 0])]
+         ([2, 0, 1], [3, 4, 0]),
+         # as many tokens as blocks of four, eight and sixteen take (two blocks a multiprocessor of one group of channels)
+         ([1290, 3, 17], [0, 2, 0]), ([2480, 9], [5, 0]), ([4750, 33, 16], [1, 0, 7])]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
