@@ -25,6 +25,7 @@
 // float32 232.  Slower: reads two steps ahead (registers spill: rows 130 and 117); groups of four warps with a step each
 // (rows 112); two issuers (no change).
 // All waits on barriers are bounded; one that runs out sets *status and the CTA winds down.
+#include "delta_chunks.cuh"
 #include "tc_common.cuh"
 
 #define LC_C 128               // tokens of a chunk
@@ -37,9 +38,11 @@
 enum { LC_ERR_EMPTY = 81, LC_ERR_FULL = 82, LC_ERR_DONE = 83 };
 
 struct LinearArgs {
-  const float* rows;           // [T, row_stride]: q of group g at q_col + g d, k at k_col + g d, v of head h at v_col + h dv
+  const float* rows;           // [T, row_stride]: q of group g at q_col + g d, k at k_col + g d
   long long row_stride;
-  int q_col, k_col, v_col;
+  int q_col, k_col;
+  const float* values;         // [T, values_stride]: v of head h at h dv
+  long long values_stride;
   const float* beta;           // [T, H]; null: 1
   const float* decay;          // [T, H]; null: log2_decay
   const float* log2_decay;     // [H]
@@ -303,12 +306,12 @@ linear_products_kernel(const LinearArgs p) {
   pdl_wait();
   // the first step's rows and the decays are on their way together
   const float* kb = p.rows + (size_t)t0 * p.row_stride + p.k_col + (size_t)(h0 / (p.H / p.G)) * d + m0;
-  const float* vb = p.rows + (size_t)t0 * p.row_stride + p.v_col + (size_t)h0 * dv;
+  const float* vb = p.values + (size_t)t0 * p.values_stride + (size_t)h0 * dv;
   LcAcross<128> a;
   LcAcross<NB> v;
   if (warp < LC_ISSUER) {
     a.load(kb, p.row_stride, n, d - m0);
-    v.load(vb, p.row_stride, n, cols);
+    v.load(vb, p.values_stride, n, cols);
   }
   if (warp < p.heads) {                                // (at most eight heads)
     lc_sums(p, lc_tokens(p, t0, n, h0 + warp), n, h0 + warp, Ls[warp], ws[warp]);
@@ -336,7 +339,7 @@ linear_products_kernel(const LinearArgs p) {
       v.store(at + 2 * LC_A_BYTES, B_PART, [&](int i) { return wv[i][32 * s]; });
       if (s + 1 < steps) {
         a.load(kb + (size_t)(32 * (s + 1)) * p.row_stride, p.row_stride, n - 32 * (s + 1), d - m0);
-        v.load(vb + (size_t)(32 * (s + 1)) * p.row_stride, p.row_stride, n - 32 * (s + 1), cols);
+        v.load(vb + (size_t)(32 * (s + 1)) * p.values_stride, p.values_stride, n - 32 * (s + 1), cols);
       }
       ring.give();
     }
@@ -474,7 +477,7 @@ linear_rows_kernel(const LinearArgs p) {
     const float* rq = p.rows + (size_t)t0 * p.row_stride + (size_t)(h0 / (p.H / p.G)) * d;
     const float* rk = rq + p.k_col;
     rq += p.q_col;
-    const float* rv = p.rows + (size_t)t0 * p.row_stride + p.v_col;
+    const float* rv = p.values + (size_t)t0 * p.values_stride;
     auto one = [](int) { return 1.f; };
     {                                                  // the chunk's products q_i . k_j
       LcAlong<128> a, k;
@@ -594,7 +597,7 @@ linear_rows_kernel(const LinearArgs p) {
       }
       if (hh == 0) ring.ok = ring.ok && lc_wait_done(scored, 0, p, &abort_s);
       LcAcross<NB> v;                                  // and the chunk's own tokens
-      v.load(rv + (size_t)h * dv, p.row_stride, n, dv);
+      v.load(rv + (size_t)h * dv, p.values_stride, n, dv);
       const double Li = Ls[hh][i];
       for (int s = 0; s < kj && ring.ok; ++s) {
         // this thread's eight scores of the step: row i, keys 32 s + 8 (warp / 4) ..
@@ -625,7 +628,7 @@ linear_rows_kernel(const LinearArgs p) {
         }
         v.store(at + 2 * LC_A_BYTES, B_PART, one);
         if (v.take_out(at + 2 * LC_A_BYTES, B_PART, 32 * s + lane, first_s[hh])) { *(volatile int*)&marked_s[hh] = 1; __threadfence_block(); }
-        if (s + 1 < kj) v.load(rv + (size_t)h * dv + (size_t)(32 * (s + 1)) * p.row_stride, p.row_stride, n - 32 * (s + 1), dv);
+        if (s + 1 < kj) v.load(rv + (size_t)h * dv + (size_t)(32 * (s + 1)) * p.values_stride, p.values_stride, n - 32 * (s + 1), dv);
         ring.give();
       }
       if (BUFS == 2 && hh > 0) epilogue(hh - 1);
@@ -671,7 +674,7 @@ static long long lc_scratch(int tiles, int H, int d, int dv) { return (long long
 static bool lc_supported(const LinearArgs& p) {
   auto on16 = [](const void* q) { return ((size_t)q % 16) == 0; };
   return p.d % 8 == 0 && p.d <= 256 && p.dv % 4 == 0 && p.dv <= 256 && p.row_stride % 4 == 0 && p.q_col % 4 == 0 && p.k_col % 4 == 0 &&
-         p.v_col % 4 == 0 && on16(p.rows) && on16(p.scratch) && on16(p.state) && (!p.o_raw || on16(p.o_raw)) && p.status;
+         p.values_stride % 4 == 0 && on16(p.values) && on16(p.rows) && on16(p.scratch) && on16(p.state) && (!p.o_raw || on16(p.o_raw)) && p.status;
 }
 
 template <typename K> static int lc_smem(K kernel, size_t bytes) {
@@ -694,6 +697,15 @@ template <int NB, bool RETENTION, typename TA> static int lc_rows(const LinearAr
   return gg_check_launch("linear_rows");
 }
 
+// The rows: a CTA takes as many heads of a group as leave a CTA for every multiprocessor and two for most.
+template <bool RETENTION, typename TA> static int lc_all_rows(LinearArgs p, int num_tiles, cudaStream_t stream) {
+  p.heads = 1;
+  while (p.heads < 8 && p.H / p.G % (2 * p.heads) == 0 && (long long)num_tiles * (p.H / (2 * p.heads)) >= 3 * 148 / 2) p.heads *= 2;
+  if (p.dv <= 64) return lc_rows<64, RETENTION, TA>(p, num_tiles, stream);
+  if (p.dv <= 128) return lc_rows<128, RETENTION, TA>(p, num_tiles, stream);
+  return lc_rows<256, RETENTION, TA>(p, num_tiles, stream);
+}
+
 template <bool RETENTION, typename TA> static int lc_run(LinearArgs p, int num_tiles, cudaStream_t stream) {
   p.tiles = num_tiles;
   p.factor = p.scratch + (long long)num_tiles * p.H * p.d * p.dv;
@@ -707,13 +719,20 @@ template <bool RETENTION, typename TA> static int lc_run(LinearArgs p, int num_t
   gg_launch(linear_scan_kernel, dim3(p.B, p.H, (p.d * p.dv / 4 + 255) / 256), dim3(256), 0, stream, p);
   rc = gg_check_launch("linear_scan");
   if (rc) return rc;
-  // the rows: a CTA takes as many heads of a group as leave a CTA for every multiprocessor and two for most
-  p.heads = 1;
-  while (p.heads < 8 && rep % (2 * p.heads) == 0 && (long long)num_tiles * (p.H / (2 * p.heads)) >= 3 * 148 / 2) p.heads *= 2;
-  if (p.dv <= 64) return lc_rows<64, RETENTION, TA>(p, num_tiles, stream);
-  if (p.dv <= 128) return lc_rows<128, RETENTION, TA>(p, num_tiles, stream);
-  return lc_rows<256, RETENTION, TA>(p, num_tiles, stream);
+  return lc_all_rows<RETENTION, TA>(p, num_tiles, stream);
 }
+
+// The delta rule's rows (delta_chunks.cu): what its tokens write stands in the result's place.
+static LinearArgs lc_of_delta(const DeltaChunkArgs& c) {
+  LinearArgs p = {};
+  p.rows = c.rows; p.row_stride = c.row_stride; p.q_col = 0; p.k_col = c.k_col; p.values = c.o_raw; p.values_stride = (long long)c.H * c.dv;
+  p.decay = c.decay; p.state = c.state; p.scratch = c.scratch; p.tile_seq = c.tile_seq; p.tile_q0 = c.tile_q0; p.tiles = c.tiles;
+  p.cu_q_lens = c.cu_q_lens; p.context_lens = c.context_lens; p.state_slots = c.state_slots;
+  p.B = c.B; p.G = c.G; p.H = c.H; p.d = c.d; p.dv = c.dv; p.o_raw = c.o_raw; p.status = c.status;
+  return p;
+}
+bool delta_rows_supported(const DeltaChunkArgs& p) { return lc_supported(lc_of_delta(p)); }
+int delta_rows(const DeltaChunkArgs& p, cudaStream_t stream) { return lc_all_rows<false, float>(lc_of_delta(p), p.tiles, stream); }
 
 // gg_delta_recur's plain recurrence over the sequences whose chunks of 128 tokens are the tiles (all chunks of a sequence, in
 // their order); the others are left alone.  Returns GG_ERR_UNSUPPORTED, and launches nothing, where sizes or addresses are not
@@ -725,7 +744,7 @@ extern "C" int gg_linear_chunks(const float* qkv, const float* beta, const float
   GG_REQUIRE(T >= 0 && B > 0 && G > 0 && H > 0 && H % G == 0 && d > 0 && dv > 0 && num_tiles >= 0, "linear_chunks: bad sizes T=%d B=%d G=%d H=%d d=%d dv=%d", T, B, G, H, d, dv);
   GG_REQUIRE(qkv && beta && decay && state && scratch && o_raw && status, "linear_chunks: a pointer is null");
   LinearArgs p = {};
-  p.rows = qkv; p.row_stride = 2ll * G * d + (long long)H * dv; p.q_col = 0; p.k_col = G * d; p.v_col = 2 * G * d;
+  p.rows = qkv; p.row_stride = 2ll * G * d + (long long)H * dv; p.q_col = 0; p.k_col = G * d; p.values = qkv + 2 * G * d; p.values_stride = p.row_stride;
   p.beta = beta; p.decay = decay; p.state = state; p.scratch = scratch; p.tile_seq = tile_seq; p.tile_q0 = tile_q0;
   p.cu_q_lens = cu_q_lens; p.context_lens = context_lens; p.state_slots = state_slots;
   p.B = B; p.G = G; p.H = H; p.d = d; p.dv = dv; p.o_raw = o_raw; p.status = status;
@@ -743,7 +762,7 @@ extern "C" int gg_linear_retention(const float* rows, const float* log2_decay, f
   GG_REQUIRE(T >= 0 && B > 0 && H > 0 && d > 0 && dv > 0 && num_tiles >= 0, "linear_retention: bad sizes T=%d B=%d H=%d d=%d dv=%d", T, B, H, d, dv);
   GG_REQUIRE(rows && log2_decay && state && scratch && gate && out && status && gate_stride >= (long long)H * dv, "linear_retention: bad arguments");
   LinearArgs p = {};
-  p.rows = rows; p.row_stride = (long long)H * (2 * d + dv); p.q_col = 0; p.k_col = H * d; p.v_col = 2 * H * d;
+  p.rows = rows; p.row_stride = (long long)H * (2 * d + dv); p.q_col = 0; p.k_col = H * d; p.values = rows + 2 * H * d; p.values_stride = p.row_stride;
   p.log2_decay = log2_decay; p.state = state; p.scratch = scratch; p.tile_seq = tile_seq; p.tile_q0 = tile_q0;
   p.cu_q_lens = cu_q_lens; p.context_lens = context_lens; p.state_slots = state_slots;
   p.B = B; p.G = H; p.H = H; p.d = d; p.dv = dv;

@@ -1029,6 +1029,40 @@ def linear_chunks(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, st
     return True
 
 
+def delta_chunks_ok(d: int, dv: int) -> bool:
+    """Whether delta_chunks takes keys of d and values of dv."""
+    return d % 32 == 0 and d <= 128 and dv % 16 == 0 and dv <= 256
+
+
+def delta_solved_floats(num_tokens: int, num_seqs: int, kv_heads: int, heads: int, d: int) -> int:
+    """Size of delta_chunks' second scratch for a step of num_tokens in num_seqs portions: solved keys per head, keys, a factor per
+    token and head."""
+    return (num_tokens // LINEAR_CHUNK + num_seqs + 1) * LINEAR_CHUNK * (heads + kv_heads) * (64 if d <= 64 else 128) + num_tokens * heads
+
+
+def delta_chunks(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
+                 solved: torch.Tensor, tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
+                 context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, kv_heads: int, heads: int, d: int,
+                 dv: int, o_raw: torch.Tensor) -> bool:
+    """delta_recur (a decay per head) over the sequences whose chunks of LINEAR_CHUNK tokens tile_seq and tile_q0 list, as
+    linear_chunks does for the plain recurrence.  scratch: float32 of linear_scratch_floats(); solved: of delta_solved_floats().
+    False, and nothing done, where sizes or addresses are not for these kernels."""
+    _cuda(qkv, beta, decay, state, scratch, solved, o_raw)
+    if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, d) or decay.shape[-1] != heads \
+            or qkv.dtype != torch.float32 or scratch.dtype != torch.float32 or solved.dtype != torch.float32:
+        raise KernelError("delta_chunks: float32 rows, scratch and state [slots, heads, dv, d], a decay per head")
+    global tc_launched
+    rc = lib().gg_delta_chunks(_p(qkv), _p(beta), _p(decay), _p(state), _p(scratch), ctypes.c_longlong(scratch.numel()), _p(solved),
+                               ctypes.c_longlong(solved.numel()), _p(tile_seq), _p(tile_q0), num_tiles, _p(cu_q_lens), _p(context_lens),
+                               _p(state_slots), o_raw.shape[0], num_seqs, kv_heads, heads, d, dv, _p(o_raw), _p(tc_status(o_raw.device)),
+                               _stream())
+    if rc == 3:                                            # GG_ERR_UNSUPPORTED
+        return False
+    _check(rc, 3)
+    tc_launched = True
+    return True
+
+
 def linear_retention(rows: torch.Tensor, log2_decay: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
                      tile_seq: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, cu_q_lens: torch.Tensor,
                      context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, gate: torch.Tensor, eps: float,

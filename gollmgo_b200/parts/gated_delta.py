@@ -10,7 +10,8 @@ square per head, multiplied by a weight shared by the heads and by silu(Wg x), a
 
 State per request, in its state slot: S in float32 [heads, dv, d] and the last taps - 1 inputs
 of the convolution in float32 [taps - 1, channels].  Nothing is paged.  Everything between the
-projections and the output projection is float32 (csrc/delta_rule.cu).
+projections and the output projection is float32 (csrc/delta_rule.cu; long prompt portions with a decay per
+head in chunks, csrc/delta_chunks.cu).
 
 Variants, all parameters: ``decay="channel"``: g is a factor per head and key channel (a row of S,
 ``dt_bias`` then [heads * head_dim]) instead of one per head; ``a_rank`` / ``gate_rank``: the
@@ -31,7 +32,17 @@ from ..cache import FixedStateNeed
 from ..csrc import ops
 from ..weights import WeightSpec
 from .linear import linear
+from .linear_recurrence import ChunkTiles
 from .registry import register_mixer
+
+# Portions of so many tokens take the chunk form (csrc/delta_chunks.cu): its three kernels take some 45 us however short they are,
+# the walk as long as its longest portion.  A B200, us, chunks / walk, values of 128 (16 heads on 4, 32 on 8; 16 on 4 with 64 keys):
+#   128 keys: 192: 58 / 43, 62 / 55   256: 62 / 55, 66 / 70   512: 77 / 102, 87 / 133   8 x 256: 158 / 190, 269 / 356   16 x 64: 126 / 98
+#   64 keys:  256: 52 / 43            512: 64 / 78            8 x 256: 124 / 113
+# A few short portions beside a long one: 256 + 3 x 30: 72 / 108; many: 256 + 30 x 8: 214 / 119 (ChunkTiles divides those).
+def chunks_from(d):
+    return 320 if d > 64 else 384
+
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "beta": "b", "a": "a", "gate": "g", "o": "o", "A_log": "A_log",
           "dt_bias": "dt_bias", "norm": "norm", "a1": "a1", "a2": "a2", "g1": "g1", "g2": "g2"}
@@ -76,6 +87,15 @@ class GatedDeltaRule:
         ws.reserve("delta_o", T * self.nh * self.dv, torch.float32)
         ws.reserve("delta_y", T * self.nh * self.dv, ctx.act_dtype)
         ws.reserve(self.out_buffer, T * self.hidden, ctx.act_dtype)
+        # (the chunks' rows are products of three tf32 parts: a model served in float32 keeps the walk)
+        self.chunks = None
+        if self.dw == 1 and ctx.act_dtype != torch.float32 and ops.delta_chunks_ok(self.d, self.dv):
+            limit = chunks_from(self.d)
+            self.chunks = ChunkTiles(ops.LINEAR_CHUNK, at_least=limit, longest=limit, most=T // ops.LINEAR_CHUNK + T // limit)
+            self.scratch = (ops.linear_scratch_floats(T, T // limit, self.nh, self.d, self.dv),
+                            ops.delta_solved_floats(T, T // limit, self.nkv, self.nh, self.d))
+            ws.reserve("linear_states", self.scratch[0], torch.float32)
+            ws.reserve("delta_solved", self.scratch[1], torch.float32)
         self.w_proj = self.w_ba = self.w_o = self.w_a2 = self.w_g2 = None
         self.conv_w = self.a_log = self.dt_bias = self.norm_w = None
 
@@ -156,6 +176,22 @@ class GatedDeltaRule:
         self.dt_bias = get(n["dt_bias"]).float().contiguous()
         self.norm_w = get(n["norm"]).float().contiguous()
 
+    def query_tiles(self):
+        return [self.chunks] if self.chunks is not None else []
+
+    def _recur(self, qkv, beta, decay, state, batch, o):
+        B, H, d, dv = batch.num_seqs, self.nh, self.d, self.dv
+        tiles, max_len = batch.tiles.get(self.chunks) if self.chunks is not None else None, 0
+        if tiles is not None and tiles.count:
+            states, solved = (self.ctx.workspace.get(n, 1, size) for n, size in zip(("linear_states", "delta_solved"), self.scratch))
+            if ops.delta_chunks(qkv, beta, decay, state, states, solved, tiles.seq, tiles.q0, tiles.count, batch.cu_q_lens,
+                                batch.context_lens, batch.state_slots, B, self.nkv, H, d, dv, o):
+                if not tiles.left_out and not batch.num_decode:
+                    return
+                max_len = self.chunks.at_least - 1 if tiles.left_out else 1
+        ops.delta_recur(qkv, beta, decay, state, batch.cu_q_lens, batch.context_lens, batch.state_slots, B, self.nkv, H, d, dv, o,
+                        max_len=max_len)
+
     def forward(self, x, batch, cache, writes_cache=True, then=None):
         T = x.shape[0]
         ws = self.ctx.workspace
@@ -177,8 +213,7 @@ class GatedDeltaRule:
         ops.delta_prep(proj, self.conv_w, conv_state, zb, za, self.a_log, self.dt_bias, batch.cu_q_lens, batch.context_lens,
                        batch.state_slots, B, self.nkv, self.nh, self.d, self.dv, qkv, beta, decay)
         o = ws.get("delta_o", T, self.nh * self.dv)
-        ops.delta_recur(qkv, beta, decay, state, batch.cu_q_lens, batch.context_lens, batch.state_slots, B,
-                        self.nkv, self.nh, self.d, self.dv, o)
+        self._recur(qkv, beta, decay, state, batch, o)
         y = ws.get("delta_y", T, self.nh * self.dv)
         if self.gate_rank:
             gate = linear(proj[:, self.gate_col:self.a_col if self.a_rank else self.proj_width], self.w_g2,
