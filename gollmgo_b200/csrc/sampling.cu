@@ -27,41 +27,37 @@ __device__ __forceinline__ float uniform_draw(unsigned long long seed, unsigned 
   return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
-// First index of the maximum of row[0..V).  own: the maximum of this thread's values.
-__device__ int block_argmax(const float* row, int V, float* red_f, int* red_i, float* max_out, float* own = nullptr) {
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  if ((((size_t)row) & 15) == 0) {
-    // four values per load, eight loads on their way; within a thread indices only grow, so ">" keeps the first maximum
-    const int V4 = V >> 2;
-    const float4* row4 = reinterpret_cast<const float4*>(row);
-    for (int i0 = threadIdx.x; i0 < V4; i0 += 8 * blockDim.x) {
-      float4 v[8];
+// Which values of a row a thread has: four neighbouring ones from 4 start on, every 4 stride further.  Two blocks that share a row
+// have the threads of one twice as large between them.  AHEAD: how many pairs of loads are on their way beside the pair at hand.
+template <int AHEAD = 1> struct Walk { int start, stride; };
+
+// f(i, v, there) for every four values v at row[4 i] that are this thread's, by whole warps (there: inside the row).  A pass runs its
+// loop a few times only and the code of an unrolled one comes from L2 too: two loads a turn and the next ones on their way take 20
+// thousand clocks of 128 k values with exponentials, sixteen loads a turn 42.
+template <int AHEAD, typename F> __device__ __forceinline__ void each_four(const float* row, int V4, const Walk<AHEAD> walk, F&& f) {
+  const float4* row4 = reinterpret_cast<const float4*>(row);
+  const int lane = threadIdx.x & 31, step = 2 * walk.stride;
+  float4 v[AHEAD + 1][2];
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (i0 + u * (int)blockDim.x < V4) v[u] = row4[i0 + u * blockDim.x];
+  for (int a = 0; a <= AHEAD; ++a)
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = i0 + u * blockDim.x;
-        if (i < V4) {
-          if (v[u].x > best) { best = v[u].x; bi = 4 * i; }
-          if (v[u].y > best) { best = v[u].y; bi = 4 * i + 1; }
-          if (v[u].z > best) { best = v[u].z; bi = 4 * i + 2; }
-          if (v[u].w > best) { best = v[u].w; bi = 4 * i + 3; }
-        }
-      }
-    }
-    for (int i = (V4 << 2) + threadIdx.x; i < V; i += blockDim.x) {
-      const float v = row[i];
-      if (v > best || (v == best && i < bi)) { best = v; bi = i; }
-    }
-  } else {
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float v = row[i];
-      if (v > best || (v == best && i < bi)) { best = v; bi = i; }
-    }
+    for (int u = 0; u < 2; ++u)
+      if (walk.start + a * step + u * walk.stride < V4) v[a][u] = row4[walk.start + a * step + u * walk.stride];
+#pragma unroll 1
+  for (int i = walk.start; i - lane < V4; i += step) {
+    const float4 c[2] = {v[0][0], v[0][1]};
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a) { v[a][0] = v[a + 1][0]; v[a][1] = v[a + 1][1]; }
+    const int n = i + (AHEAD + 1) * step;
+    if (n < V4) v[AHEAD][0] = row4[n];
+    if (n + walk.stride < V4) v[AHEAD][1] = row4[n + walk.stride];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) f(i + u * walk.stride, c[u], i + u * walk.stride < V4);
   }
-  if (own) *own = best;
+}
+
+// Of the threads' maxima and their first indices the block's.
+__device__ __forceinline__ int first_of_block(float best, int bi, float* red_f, int* red_i, float* max_out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -86,8 +82,40 @@ __device__ int block_argmax(const float* row, int V, float* red_f, int* red_i, f
   }
   __syncthreads();
   if (max_out) *max_out = red_f[32];
-  return red_i[32] == 0x7fffffff ? 0 : red_i[32];
+  return red_i[32];
 }
+
+// First index of the maximum of row[0..V) (0x7fffffff: none above -infinity).  own: the maximum of this thread's values.
+template <int AHEAD = 1>
+__device__ int block_argmax(const float* row, int V, float* red_f, int* red_i, float* max_out, float* own = nullptr,
+                            const Walk<AHEAD> walk = {(int)threadIdx.x, (int)blockDim.x}) {
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  if ((((size_t)row) & 15) == 0) {
+    // within a thread indices only grow, so ">" keeps the first maximum
+    const int V4 = V >> 2;
+    each_four(row, V4, walk, [&](int i, const float4& v, bool there) {
+      if (there) {
+        if (v.x > best) { best = v.x; bi = 4 * i; }
+        if (v.y > best) { best = v.y; bi = 4 * i + 1; }
+        if (v.z > best) { best = v.z; bi = 4 * i + 2; }
+        if (v.w > best) { best = v.w; bi = 4 * i + 3; }
+      }
+    });
+    for (int i = (V4 << 2) + walk.start; i < V; i += walk.stride) {
+      const float v = row[i];
+      if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+    }
+  } else {
+    for (int i = walk.start; i < V; i += walk.stride) {
+      const float v = row[i];
+      if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+    }
+  }
+  if (own) *own = best;
+  return first_of_block(best, bi, red_f, red_i, max_out);
+}
+__device__ __forceinline__ int first_if_none(int i) { return i == 0x7fffffff ? 0 : i; }
 
 __global__ void argmax_kernel(const float* __restrict__ logits, int V, int* __restrict__ out) {
   __shared__ float red_f[33];
@@ -95,7 +123,7 @@ __global__ void argmax_kernel(const float* __restrict__ logits, int V, int* __re
   pdl_trigger();
   pdl_wait();
   const int r = blockIdx.x;
-  const int idx = block_argmax(logits + (size_t)r * V, V, red_f, red_i, nullptr);
+  const int idx = first_if_none(block_argmax(logits + (size_t)r * V, V, red_f, red_i, nullptr));
   if (threadIdx.x == 0) out[r] = idx;
 }
 
@@ -147,74 +175,97 @@ template <typename T> __device__ __forceinline__ T sc_load(const T* local, unsig
   return out;
 }
 
-// f(x) for every value of row[0..V): four a load where the start allows it, eight loads on their way before the first is
-// used (one at a time a pass over 128 k values is a chain of 31 trips to L2 a thread).
-template <typename F> __device__ __forceinline__ void each_value(const float* row, int V, F&& f) {
+// f(x) for the values of row[0..V) that are this thread's.
+template <int AHEAD, typename F> __device__ __forceinline__ void each_value(const float* row, int V, const Walk<AHEAD> walk, F&& f) {
   const int V4 = (((size_t)row) & 15) == 0 ? V >> 2 : 0;
-  const float4* row4 = reinterpret_cast<const float4*>(row);
-  for (int i0 = threadIdx.x; i0 < V4; i0 += 8 * blockDim.x) {
-    float4 v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (i0 + u * (int)blockDim.x < V4) v[u] = row4[i0 + u * blockDim.x];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (i0 + u * (int)blockDim.x < V4) { f(v[u].x); f(v[u].y); f(v[u].z); f(v[u].w); }
-  }
-  for (int i = (V4 << 2) + threadIdx.x; i < V; i += blockDim.x) f(row[i]);
+  each_four(row, V4, walk, [&](int, const float4& v, bool there) {
+    if (there) { f(v.x); f(v.y); f(v.z); f(v.w); }
+  });
+  for (int i = (V4 << 2) + walk.start; i < V; i += walk.stride) f(row[i]);
 }
 
-// The values of row[0..V) with keys in [lo, hi] to keep[0..room), in no particular order; *n = how many there are (also
-// those beyond the room).  A thread counts its share of 32 values, a warp adds its lanes' counts to *n at once.
-__device__ void collect(const float* row, int V, float* keep, int room, int* n, unsigned lo, unsigned hi) {
+// The values of row[0..V) with keys in [lo, hi] that are this block's to keep[0..room), in no particular order; *n = how many there
+// are (also those beyond the room).  A warp adds the hits of four values a lane to *n at once, then writes them value by value: the
+// lanes that hit write side by side (each lane writing its own hits in a row met a bank eight times over: 41 us of a row with 27 k
+// hits among 128 k).
+template <int AHEAD>
+__device__ void collect(const float* row, int V, const Walk<AHEAD> walk, float* keep, int room, int* n, unsigned lo, unsigned hi) {
   if (threadIdx.x == 0) *n = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
   const int V4 = (((size_t)row) & 15) == 0 ? V >> 2 : 0;
-  const float4* row4 = reinterpret_cast<const float4*>(row);
   auto in = [&](float x) { const unsigned k = ordered_key(x); return k >= lo && k <= hi; };
-  auto place = [&](int count) {                          // called by whole warps
-    int incl = count;
+  const int first = walk.start - lane;                   // (the warp's; lanes are neighbours)
+  each_four(row, V4, walk, [&](int, const float4& v, bool there) {
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    unsigned m[4], all = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
+    for (int j = 0; j < 4; ++j) { m[j] = __ballot_sync(0xffffffffu, there && in(f[j])); all |= m[j]; }
+    if (!all) return;
     int at = 0;
-    if (lane == 31) at = atomicAdd(n, incl);
-    return __shfl_sync(0xffffffffu, at, 31) + incl - count;
-  };
-  for (int b = 0; b < V4; b += 8 * blockDim.x) {
-    float4 v[8];
-    int count = 0;
+    if (lane == 0) at = atomicAdd(n, __popc(m[0]) + __popc(m[1]) + (__popc(m[2]) + __popc(m[3])));
+    at = __shfl_sync(0xffffffffu, at, 0);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int i = b + u * (int)blockDim.x + (int)threadIdx.x;
-      if (i < V4) v[u] = row4[i];
+    for (int j = 0; j < 4; ++j) {
+      const int to = at + __popc(m[j] & below);
+      if ((m[j] >> lane & 1u) && to < room) keep[to] = f[j];
+      at += __popc(m[j]);
     }
-    unsigned hits = 0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (b + u * (int)blockDim.x + (int)threadIdx.x < V4)
-        hits |= ((unsigned)in(v[u].x) | (unsigned)in(v[u].y) << 1 | (unsigned)in(v[u].z) << 2 | (unsigned)in(v[u].w) << 3) << (4 * u);
-    count = __popc(hits);
-    if (!__any_sync(0xffffffffu, count)) continue;
-    int at = place(count);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const float f[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (hits >> (4 * u + j) & 1u) { if (at < room) keep[at] = f[j]; ++at; }
-    }
-  }
-  for (int b = V4 << 2; b < V; b += blockDim.x) {
-    const int i = b + (int)threadIdx.x;
+  });
+  for (int b = (V4 << 2) + first; b < V; b += walk.stride) {
+    const int i = b + lane;
     const bool hit = i < V && in(row[i]);
-    const int at = place(hit);
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    int at = 0;
+    if (lane == 0 && m) at = atomicAdd(n, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & below);
     if (hit && at < room) keep[at] = row[i];
   }
   __syncthreads();
+}
+
+// ---- a row shared by the two blocks of a cluster (sample_kernel<2>): each has half of the threads that one block alone has, does what
+// those do, and tells the other what they found, so that every sum is formed from the same numbers in the same order.  What is told
+// goes to the other's copy, one of two in turn: a copy is written again only after a further cluster barrier.
+struct PairPub {
+  float f[2][4][32];
+  int i[2][2];
+  unsigned long long bins[2][256];
+};
+__device__ __forceinline__ unsigned pair_addr(const void* local) {        // of the same variable in the other block
+  unsigned v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(sc_rank() ^ 1u));
+  return v;
+}
+__device__ __forceinline__ void pair_tell(float* to, float v) {
+  *to = v;
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(pair_addr(to)), "f"(v) : "memory");
+}
+__device__ __forceinline__ void pair_tell(int* mine, int* others, int v) {
+  *mine = v;
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(pair_addr(others)), "r"(v) : "memory");
+}
+// block_sum of N values over both blocks' 32 warps
+template <int N> __device__ __forceinline__ void pair_sums(float (&v)[N], PairPub* pub, int& par) {
+  const int lane = threadIdx.x & 31, slot = sc_rank() * (blockDim.x >> 5) + (threadIdx.x >> 5);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    v[j] = warp_sum(v[j]);
+    if (lane == 0) pair_tell(&pub->f[par][j][slot], v[j]);
+  }
+  sc_barrier();
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = warp_sum(pub->f[par][j][lane]);
+  par ^= 1;
+}
+// the sum of both blocks' v (of thread 0); *mine: this block's
+__device__ __forceinline__ int pair_count(int v, PairPub* pub, int& par) {
+  if (threadIdx.x == 0) pair_tell(&pub->i[par][0], &pub->i[par][1], v);
+  sc_barrier();
+  const int s = pub->i[par][0] + pub->i[par][1];
+  par ^= 1;
+  return s;
 }
 
 // Sums of weights in fixed point (40 fraction bits) in bins of shared memory.  A 64-bit atomic on shared memory is a loop
@@ -223,11 +274,14 @@ __device__ void collect(const float* row, int V, float* keep, int room, int* n, 
 #define FX_ONE 1099511627776.f           // 2^40
 #define FX_PIECES 3
 __device__ __forceinline__ unsigned long long fixed_weight(float w) { return (unsigned long long)(w * FX_ONE); }
+__device__ __forceinline__ void add_bin(unsigned* bin, unsigned v) {      // (bin is in shared memory: no generic address to resolve)
+  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bin)), "r"(v) : "memory");
+}
 __device__ __forceinline__ void add_fixed(unsigned* bins, int stride, int bin, unsigned long long w) {
 #pragma unroll
   for (int k = 0; k < FX_PIECES; ++k) {
     const unsigned piece = (unsigned)(w >> (14 * k)) & (k + 1 < FX_PIECES ? 0x3fffu : 0xffffffffu);
-    if (piece) atomicAdd(bins + k * stride + bin, piece);
+    if (piece) add_bin(bins + k * stride + bin, piece);
   }
 }
 __device__ __forceinline__ unsigned long long fixed_sum(const unsigned* bins, int stride, int bin) {
@@ -278,18 +332,21 @@ __device__ __forceinline__ void pick_bin(float* hist, float above, float target)
   }
 }
 
-// CL: row is this CTA's part of the row and the histogram of a pass is the sum over the
-// cluster's CTAs in rank order, the same in every CTA, so every CTA descends alike.
+// MODE 1: row is this CTA's part of the row and the histogram of a pass is the sum over the
+// cluster's CTAs in rank order, the same in every CTA, so every CTA descends alike.  MODE 2: the two blocks of a pair walk the row
+// (or their own lists of what is left of it) together.  last: the lowest bit of the byte it ends with.
 // bins: FX_PIECES * 256 integers, 8-byte aligned.  unordered: row is a copy whose order differs from run to run, so the
 // float32 sums of the first pass are left out.  sum_of_all: target is share times the sum of all weights, which the first
-// pass makes too.  keep, keep_n: where given (room for keep_room values; not CL), what is left of the row once
+// pass makes too.  keep, keep_n: where given (room for keep_room values; not MODE 1), what is left of the row once
 // the leading byte is known is copied there, and the lower bytes' passes read the copy.
-template <bool MASS, bool CL>
+template <bool MASS, int MODE, int AHEAD = 1>
 __device__ unsigned int radix_threshold(const float* row, int V, float m, float invT,
                                         unsigned int floor_key, float target, float* hist,
                                         float* red, unsigned* bins, ClusterPub* pub = nullptr,
                                         float* keep = nullptr, int* keep_n = nullptr, int keep_room = 0, const bool sum_of_all = false,
-                                        float share = 0.f, const bool unordered = false) {
+                                        float share = 0.f, const bool unordered = false,
+                                        Walk<AHEAD> walk = {(int)threadIdx.x, (int)blockDim.x}, PairPub* pair = nullptr, int* turn = nullptr, const int last = 0) {
+  constexpr bool CL = MODE == 1;
   const int warp = threadIdx.x >> 5;
   unsigned int prefix = 0, pmask = 0;
   float above = 0.f;       // weight of keys strictly above the current prefix range
@@ -317,20 +374,33 @@ __device__ unsigned int radix_threshold(const float* row, int V, float m, float 
     // the weight of the values from the lower border of each of the three bins on
     const unsigned b0 = (unsigned)top << 24, b1 = (unsigned)max(top - 1, 0) << 24, b2 = (unsigned)max(top - 2, 0) << 24;
     float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, all = 0.f;
-    each_value(row, V, [&](float x) {
+    each_value(row, V, walk, [&](float x) {
+      // (without branches: a value's chain of steps then runs beside its neighbours'; adding 0 changes no sum)
       const unsigned int k = ordered_key(x);
-      if (k >= floor_key && (sum_of_all || k >= b2)) {
-        const float w = MASS ? expf((x - m) * invT) : 1.f;
-        if (k >= b0) acc0 += w;
-        if (k >= b1) acc1 += w;
-        if (k >= b2) acc2 += w;
+      if (MASS) {
+        const float e = expf((x - m) * invT);
+        const float w = k < floor_key ? 0.f : e;
+        acc0 += k >= b0 ? w : 0.f;
+        acc1 += k >= b1 ? w : 0.f;
+        acc2 += k >= b2 ? w : 0.f;
         all += w;
+      } else if (k >= floor_key && k >= b2) {           // (few do)
+        if (k >= b0) acc0 += 1.f;
+        if (k >= b1) acc1 += 1.f;
+        acc2 += 1.f;
       }
     });
-    if (sum_of_all) target = share * block_sum(all, red);       // the target is a share of the sum
-    acc0 = block_sum(acc0, red);
-    acc1 = block_sum(acc1, red);
-    acc2 = block_sum(acc2, red);
+    if constexpr (MODE == 2) {
+      float v[4] = {acc0, acc1, acc2, all};
+      pair_sums(v, pair, *turn);
+      acc0 = v[0]; acc1 = v[1]; acc2 = v[2];
+      if (sum_of_all) target = share * v[3];
+    } else {
+      if (sum_of_all) target = share * block_sum(all, red);     // the target is a share of the sum
+      acc0 = block_sum(acc0, red);
+      acc1 = block_sum(acc1, red);
+      acc2 = block_sum(acc2, red);
+    }
     if (threadIdx.x == 0) { hist[0] = acc0; hist[1] = acc1; hist[2] = acc2; }
     __syncthreads();
     exchange(3);
@@ -345,30 +415,53 @@ __device__ unsigned int radix_threshold(const float* row, int V, float m, float 
     }
     __syncthreads();                           // hist is written again below
   }
-  for (int shift = full ? 24 : 16; shift >= 0; shift -= 8) {
+  for (int shift = full ? 24 : 16; shift >= last; shift -= 8) {
     const bool wide = MASS && V > FX_MAX_VALUES;
     unsigned long long* bins64 = reinterpret_cast<unsigned long long*>(bins);
     if (!CL && keep && pmask == 255u << 24 && shift == 16) {
       // the values that share the threshold's leading byte (their order is as they come: the sums are integers)
-      collect(row, V, keep, keep_room, keep_n, max(floor_key, prefix), prefix | 0xffffffu);
-      if (*keep_n <= keep_room) { row = keep; V = *keep_n; }
+      collect(row, V, walk, keep, keep_room, keep_n, max(floor_key, prefix), prefix | 0xffffffu);
+      int left = *keep_n;
+      if constexpr (MODE == 2) left = pair_count(left, pair, *turn);
+      if (left <= keep_room) {
+        row = keep;
+        V = *keep_n;
+        if constexpr (MODE == 2) walk = {(int)threadIdx.x, (int)blockDim.x};
+      }
       __syncthreads();
     }
     for (int i = threadIdx.x; i < FX_PIECES * 256; i += blockDim.x) bins[i] = 0u;
     __syncthreads();
-    each_value(row, V, [&](float x) {
+    each_value(row, V, walk, [&](float x) {
       const unsigned int k = ordered_key(x);
       if (k >= floor_key && (k & pmask) == prefix) {
         if (wide) atomicAdd(bins64 + ((k >> shift) & 255u), fixed_weight(expf((x - m) * invT)));
         else if (MASS) add_fixed(bins, 256, (k >> shift) & 255u, fixed_weight(expf((x - m) * invT)));
-        else atomicAdd(bins + ((k >> shift) & 255u), 1u);
+        else add_bin(bins + ((k >> shift) & 255u), 1u);
       }
     });
     __syncthreads();
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
-      hist[i] = MASS ? (float)(wide ? bins64[i] : fixed_sum(bins, 256, i)) * (1.f / FX_ONE) : (float)bins[i];
-    __syncthreads();
-    exchange(256);
+    if constexpr (MODE == 2) {
+      const int par = *turn;
+      unsigned long long own = 0;
+      const int i = threadIdx.x;                       // (512 threads)
+      if (i < 256) {
+        own = !MASS ? bins[i] : wide ? bins64[i] : fixed_sum(bins, 256, i);
+        asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(pair_addr(&pair->bins[par][i])), "l"(own) : "memory");
+      }
+      sc_barrier();
+      if (i < 256) {
+        own += pair->bins[par][i];
+        hist[i] = MASS ? (float)own * (1.f / FX_ONE) : (float)own;
+      }
+      __syncthreads();
+      *turn = par ^ 1;
+    } else {
+      for (int i = threadIdx.x; i < 256; i += blockDim.x)
+        hist[i] = MASS ? (float)(wide ? bins64[i] : fixed_sum(bins, 256, i)) * (1.f / FX_ONE) : (float)bins[i];
+      __syncthreads();
+      exchange(256);
+    }
     if (warp == 0) pick_bin(hist, above, target);
     __syncthreads();
     above = hist[256];
@@ -384,13 +477,17 @@ __device__ unsigned int radix_threshold(const float* row, int V, float m, float 
 // wide steps, so the row is walked as few times as possible: the maximum; the values that can be among the top_k largest
 // (those above the k-th largest of the threads' own maxima, some hundreds), or one pass for the sum and the leading byte
 // of top_p and one that copies the values of that byte to shared memory (`room` of them; what does not fit is walked where
-// it is); the sums in index order.  64 rows of 128 k: 48 us with top_k, 55 with both, 96 with top_p alone (thirteen passes,
-// one load in flight and 64-bit atomics took 181 for rows of all kinds).
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// it is); the sums in index order.  What bounds it: the chain of passes, each a few turns of a loop by 16 or 32 warps, whose code
+// arrives from L2 too (each_four).  128 k values, 148 rows: 49 us with top_k, 96 with top_p alone (before loops of two loads: 55, 117).
+// BLOCKS = 2: the row on two multiprocessors, each with half of the threads (PairPub); the same numbers in the same order.  64 rows:
+// 40 us with top_k, 66 with top_p alone, 28 without either, where one multiprocessor a row took 50, 114 and 36.
+template <int BLOCKS>
+__global__ void __launch_bounds__(SAMPLE_THREADS / BLOCKS)
 sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const unsigned long long* __restrict__ seeds,
               const unsigned long long* __restrict__ draw_index, int* __restrict__ out, int room) {
+  constexpr int THREADS = SAMPLE_THREADS / BLOCKS, AHEAD = BLOCKS == 2 ? 3 : 1, MODE = BLOCKS == 2 ? 2 : 0;
   extern __shared__ __align__(16) float keep[];          // [room]
   __shared__ float red_f[33];
   __shared__ int red_i[33];
@@ -398,36 +495,76 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
   __shared__ __align__(8) unsigned bins[FX_PIECES * 256];
   __shared__ float scan[SAMPLE_THREADS / 32 + 1];
   __shared__ int keep_n;
-  __shared__ int found;
+  __shared__ int found, other_found;
   __shared__ unsigned long long sum64;
+  __shared__ PairPub pub_s;
+  PairPub* pub = &pub_s;
+  int turn = 0;
+  const int rank = BLOCKS == 2 ? (int)sc_rank() : 0, tid = rank * THREADS + threadIdx.x;       // the thread's place in the row
+  const Walk<AHEAD> walk = {tid, SAMPLE_THREADS};
+  const Walk<AHEAD> local = {(int)threadIdx.x, THREADS};
   pdl_trigger();
+  if constexpr (BLOCKS == 2) sc_barrier();               // the other block's memory is there
   pdl_wait();
-  const int r = blockIdx.x;
+  const int r = BLOCKS == 2 ? blockIdx.y : blockIdx.x;
   const float* row = logits + (size_t)r * V;
   const float T = temperature[r];
   float m, own;
-  const int amax = block_argmax(row, V, red_f, red_i, &m, &own);
+  int amax = block_argmax(row, V, red_f, red_i, &m, &own, walk);
+  if constexpr (BLOCKS == 2) {
+    float* f = &pub->f[0][0][0];
+    if (threadIdx.x == 0) {
+      pair_tell(f + rank, m);
+      asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(pair_addr(&pub->i[0][1])), "r"(amax) : "memory");
+    }
+    sc_barrier();
+    const float om = f[rank ^ 1];
+    const int oi = pub->i[0][1];
+    if (om > m || (om == m && oi < amax)) amax = oi;
+    m = fmaxf(m, om);                                    // (a NaN is never a maximum here)
+    turn = 1;
+  }
+  amax = first_if_none(amax);
   if (T <= 1e-9f) {
-    if (threadIdx.x == 0) out[r] = amax;
+    if (tid == 0) out[r] = amax;
     return;
   }
   const float invT = 1.f / T;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = tid >> 5;
   unsigned int floor_key = 0;
   const int k = top_k ? top_k[r] : 0;
   const float p = top_p ? top_p[r] : 0.f;
   bool kept = false;                                     // keep[0 .. keep_n) holds every value that can still be drawn
+  int kept_n = 0;
   if (k > 0 && k < V) {
     if (k <= SAMPLE_THREADS && room >= SAMPLE_THREADS) {
-      keep[threadIdx.x] = own;
+      keep[tid] = own;
+      if constexpr (BLOCKS == 2) {
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(pair_addr(keep + tid)), "f"(own) : "memory");
+        sc_barrier();
+        turn ^= 1;
+      } else {
+        __syncthreads();
+      }
+      // (sixteen bits of it: what they leave in below the k-th largest is gone with the threshold itself)
+      const unsigned pivot = radix_threshold<false, 0, AHEAD>(keep, SAMPLE_THREADS, m, invT, 0u, (float)k, hist, red_f, bins, nullptr, nullptr,
+                                                              nullptr, 0, false, 0.f, false, local, nullptr, nullptr, 16);
       __syncthreads();
-      const unsigned pivot = radix_threshold<false, false>(keep, SAMPLE_THREADS, m, invT, 0u, (float)k, hist, red_f, bins);
-      __syncthreads();
-      collect(row, V, keep, room, &keep_n, pivot, 0xffffffffu);          // at least k values: k threads have one
-      kept = keep_n <= room;
+      if constexpr (BLOCKS == 2) sc_barrier();           // (both have read what each told the other)
+      collect(row, V, walk, keep, room, &keep_n, pivot, 0xffffffffu);    // at least k values: k threads have one
+      kept_n = keep_n;
+      if constexpr (BLOCKS == 2) kept_n = pair_count(kept_n, pub, turn);
+      kept = kept_n <= room;
+      if (BLOCKS == 2 && kept) {                         // the other's behind this block's: both have them all
+        const int mine = keep_n;
+        for (int i = threadIdx.x; i < kept_n - mine; i += THREADS) keep[mine + i] = sc_load(keep + i, rank ^ 1);
+        __syncthreads();
+      }
     }
-    floor_key = kept ? radix_threshold<false, false>(keep, keep_n, m, invT, 0u, (float)k, hist, red_f, bins)
-                     : radix_threshold<false, false>(row, V, m, invT, 0u, (float)k, hist, red_f, bins, nullptr, keep, &keep_n, room);
+    floor_key = kept ? radix_threshold<false, 0, AHEAD>(keep, kept_n, m, invT, 0u, (float)k, hist, red_f, bins, nullptr, nullptr, nullptr, 0,
+                                                    false, 0.f, false, local)
+                     : radix_threshold<false, MODE, AHEAD>(row, V, m, invT, 0u, (float)k, hist, red_f, bins, nullptr, keep, &keep_n, room,
+                                                       false, 0.f, false, walk, pub, &turn);
   }
   if (p > 0.f && p < 1.f) {
     if (kept) {
@@ -435,16 +572,17 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
       if (threadIdx.x == 0) sum64 = 0ULL;
       __syncthreads();
       unsigned long long z = 0;
-      for (int i = threadIdx.x; i < keep_n; i += SAMPLE_THREADS)
+      for (int i = threadIdx.x; i < kept_n; i += THREADS)
         if (ordered_key(keep[i]) >= floor_key) z += fixed_weight(expf((keep[i] - m) * invT));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
       if (lane == 0 && z) atomicAdd(&sum64, z);
       __syncthreads();
-      floor_key = radix_threshold<true, false>(keep, keep_n, m, invT, floor_key, p * ((float)sum64 * (1.f / FX_ONE)), hist, red_f, bins,
-                                               nullptr, nullptr, nullptr, 0, false, 0.f, true);
+      floor_key = radix_threshold<true, 0, AHEAD>(keep, kept_n, m, invT, floor_key, p * ((float)sum64 * (1.f / FX_ONE)), hist, red_f, bins,
+                                              nullptr, nullptr, nullptr, 0, false, 0.f, true, local);
     } else {
-      floor_key = radix_threshold<true, false>(row, V, m, invT, floor_key, 0.f, hist, red_f, bins, nullptr, keep, &keep_n, room, true, p);
+      floor_key = radix_threshold<true, MODE, AHEAD>(row, V, m, invT, floor_key, 0.f, hist, red_f, bins, nullptr, keep, &keep_n, room, true, p,
+                                                 false, walk, pub, &turn);
     }
   }
   // Running sum in index order over the values that are left: a warp owns a stretch of the row and sums it in up to 32
@@ -453,8 +591,7 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
   const int blk = max(512, ((seg + 31) / 32 + 127) / 128 * 128);
   const int s0 = min(V, warp * seg), s1 = min(V, s0 + seg);
   const bool vec = (((size_t)row) & 15) == 0;
-  auto weights4 = [&](int i, float (&w)[4]) {            // of values i .. i + 3 (0: past the stretch or not left)
-    float x[4];
+  auto values4 = [&](int i, float (&x)[4]) {             // values i .. i + 3 (past the stretch: none)
     if (vec && i + 4 <= s1) {
       const float4 v = *reinterpret_cast<const float4*>(row + i);
       x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
@@ -462,25 +599,34 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
 #pragma unroll
       for (int j = 0; j < 4; ++j) x[j] = i + j < s1 ? row[i + j] : 0.f;
     }
+  };
+  auto left4 = [&](int i, const float (&x)[4]) {         // which of them are left, a bit each
+    unsigned b = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = i + j < s1 && ordered_key(x[j]) >= floor_key ? expf((x[j] - m) * invT) : -1.f;
+    for (int j = 0; j < 4; ++j) b |= (unsigned)(i + j < s1 && ordered_key(x[j]) >= floor_key) << j;
+    return b;
   };
   float sub = 0.f;
   for (int i0 = s0, it = 0; i0 < s1; i0 += blk, ++it) {
     float acc = 0.f;
     const int end = min(s1, i0 + blk);
     for (int i = i0; i < end; i += 512) {
-      float w[4][4];
+      float x[4][4];
+      unsigned left = 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (i + 128 * u < end) weights4(i + 128 * u + 4 * lane, w[u]);
-        else w[u][0] = w[u][1] = w[u][2] = w[u][3] = -1.f;
-      }
+      for (int u = 0; u < 4; ++u)
+        if (i + 128 * u < end) values4(i + 128 * u + 4 * lane, x[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + 128 * u < end) left |= left4(i + 128 * u + 4 * lane, x[u]) << (4 * u);
+      if (!__any_sync(0xffffffffu, left)) continue;      // (below a threshold most of a row is not left)
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (!(w[u][j] < 0.f)) acc += w[u][j];
+        for (int j = 0; j < 4; ++j) {
+          const float e = expf((x[u][j] - m) * invT);
+          acc += left >> (4 * u + j) & 1u ? e : 0.f;
+        }
     }
     acc = warp_sum(acc);
     if (lane == it) sub = acc;
@@ -492,8 +638,12 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
     if (lane >= o) incl += v;
   }
   if (threadIdx.x == 0) found = -1;
-  if (lane == 31) scan[warp] = incl;
-  __syncthreads();
+  if (lane == 31) {
+    if constexpr (BLOCKS == 2) pair_tell(scan + warp, incl);
+    else scan[warp] = incl;
+  }
+  if constexpr (BLOCKS == 2) sc_barrier();
+  else __syncthreads();
   if (threadIdx.x == 0) {
     float run = 0.f;
     const int nw = SAMPLE_THREADS >> 5;
@@ -501,11 +651,11 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
     scan[nw] = run;
   }
   __syncthreads();
-  const float total = scan[SAMPLE_THREADS >> 5], local = __shfl_sync(0xffffffffu, incl, 31);
+  const float total = scan[SAMPLE_THREADS >> 5], all = __shfl_sync(0xffffffffu, incl, 31);
   const float before = scan[warp];
   const float u = uniform_draw(seeds ? seeds[r] : 0ULL, draw_index ? draw_index[r] : 0ULL);
   const float target = u * total;
-  if (local > 0.f && target >= before && target < before + local) {
+  if (all > 0.f && target >= before && target < before + all) {
     const unsigned over = __ballot_sync(0xffffffffu, sub > 0.f && target < before + incl);
     // (rounding can leave none: then the last block with anything in it.  A lane's running sum starts from a sum in another
     // order than the one its neighbour ended with, so a draw can fall between the two: a value without weight, as a masked
@@ -516,9 +666,12 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
     int pick = -1;
     const int i0 = s0 + b * blk, end = min(s1, i0 + blk);
     for (int i = i0; i < end; i += 128) {
-      float w[4], sum = 0.f;
+      float x[4], w[4], sum = 0.f;
       const int at = i + 4 * lane;
-      weights4(at, w);
+      values4(at, x);
+      const unsigned left = left4(at, x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = left >> j & 1u ? expf((x[j] - m) * invT) : -1.f;
       int last = -1;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -545,7 +698,12 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
     if (lane == 0 && pick >= 0) atomicMax(&found, pick);
   }
   __syncthreads();
-  if (threadIdx.x == 0) out[r] = found >= 0 ? found : amax;
+  if constexpr (BLOCKS == 2) {
+    if (rank == 1 && threadIdx.x == 0) asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(pair_addr(&other_found)), "r"(found) : "memory");
+    sc_barrier();
+    if (tid == 0) found = max(found, other_found);
+  }
+  if (tid == 0) out[r] = found >= 0 ? found : amax;
 }
 
 // ---------------------------------------------------------------- a row on a cluster of CTAs
@@ -603,19 +761,27 @@ sample_cluster_kernel(const float* __restrict__ logits, int V, int part, const f
   const int base = (int)me * part, n = max(0, min(part, V - base));   // elements [base, base + n)
   const float* row = logits + (size_t)r * V;
   if (threadIdx.x == 0) pub.parity = 0;
-  // the part into shared memory (float4 where the row's start allows it; part is a multiple of 4)
+  // the part into shared memory (float4 where the row's start allows it; part is a multiple of 4), its maximum on the way
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  auto seen = [&](float v, int i) { if (v > best) { best = v; bi = i; } };
   if (((((size_t)row) & 15) == 0) && (n & 3) == 0) {
     const float4* src = reinterpret_cast<const float4*>(row + base);
     float4* dst = reinterpret_cast<float4*>(sc_part);
-    for (int i = threadIdx.x; i < (n >> 2); i += SC_THREADS) dst[i] = src[i];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < (n >> 2); i += SC_THREADS) {
+      const float4 v = src[i];
+      dst[i] = v;
+      seen(v.x, 4 * i); seen(v.y, 4 * i + 1); seen(v.z, 4 * i + 2); seen(v.w, 4 * i + 3);
+    }
   } else {
-    for (int i = threadIdx.x; i < n; i += SC_THREADS) sc_part[i] = row[base + i];
+    for (int i = threadIdx.x; i < n; i += SC_THREADS) { const float v = row[base + i]; sc_part[i] = v; seen(v, i); }
   }
   __syncthreads();
   const float T = temperature[r];
   // the maximum and its first index: of the part, then of the row (the lowest rank wins a tie)
   float m_local;
-  const int a_local = block_argmax(sc_part, n, red_f, red_i, &m_local);
+  const int a_local = first_if_none(first_of_block(best, bi, red_f, red_i, &m_local));
   if (threadIdx.x == 0) { pub.f[0] = n > 0 ? m_local : -INFINITY; pub.i[0] = base + a_local; }
   sc_barrier();
   float m = -INFINITY;
@@ -635,7 +801,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int V, int part, const f
   const float invT = 1.f / T;
   unsigned int floor_key = 0;
   const int k = top_k ? top_k[r] : 0;
-  if (k > 0 && k < V) floor_key = radix_threshold<false, true>(sc_part, n, m, invT, 0u, (float)k, hist, red_f, bins, &pub);
+  if (k > 0 && k < V) floor_key = radix_threshold<false, 1>(sc_part, n, m, invT, 0u, (float)k, hist, red_f, bins, &pub);
   const float p = top_p ? top_p[r] : 0.f;
   if (p > 0.f && p < 1.f) {
     float z = 0.f;
@@ -645,7 +811,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int V, int part, const f
     }
     z = block_sum(z, red_f);
     z = sc_sum(z, &pub, bcast, nullptr);
-    floor_key = radix_threshold<true, true>(sc_part, n, m, invT, floor_key, p * z, hist, red_f, bins, &pub);
+    floor_key = radix_threshold<true, 1>(sc_part, n, m, invT, floor_key, p * z, hist, red_f, bins, &pub);
   }
   // running sum in index order over the kept elements: a thread owns a contiguous piece of
   // the part, a CTA the part, the ranks follow each other
@@ -729,9 +895,8 @@ extern "C" int gg_sample(const float* logits, int R, int V, const float* tempera
         cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || num_sms <= 0)
       num_sms = 148;
   }
-  // (with more rows than clusters fit at once, two CTAs per SM, a CTA per row is about as fast:
-  // 64 rows are 512 CTAs where 444 fit, a second round of as long again; 8 rows on clusters
-  // take 25 us with top-k, 45 with both, where a CTA per row takes 48 and 55)
+  // (with more rows than clusters fit at once, two CTAs per SM, two CTAs a row are faster: 37 rows on clusters take 28 us without
+  // thresholds, 52 with top-k, 74 with top-p alone, 38 rows in pairs 27, 39 and 66)
   if (use_cluster && V >= SC_MIN_V && smem <= 160 * 1024 && R * SC_CLUSTER <= 2 * num_sms) {
     static bool set = false;
     if (!set) {
@@ -760,10 +925,31 @@ extern "C" int gg_sample(const float* logits, int R, int V, const float* tempera
   // room for values in shared memory, most of a multiprocessor's: the registers of 1024 threads leave no second CTA anyway, and
   // how a row's sums are formed does not depend on how many rows there are (half of it for more rows than multiprocessors: 149
   // rows of 128 k with top_p alone 277 us against 189, flat ones 386 against 311; 200 with top_k as well 114 against 118)
-  const int room = 48 * 1024;
-  cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room * (int)sizeof(float));
+  const int room = 48 * 1024, bytes = room * (int)sizeof(float);
+  // two multiprocessors a row while there are two for each
+  const bool pair = use_cluster && V >= SC_MIN_V && 2 * R <= num_sms;
+  cudaError_t e = pair ? cudaFuncSetAttribute(sample_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)
+                       : cudaFuncSetAttribute(sample_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "sample: %s", cudaGetErrorString(e));
-  gg_launch(sample_kernel, dim3(R), dim3(SAMPLE_THREADS), room * sizeof(float), stream, logits, V, temperature, top_k, top_p, seeds,
-            draw_index, out, room);
+  if (pair) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2, R);
+    cfg.blockDim = dim3(SAMPLE_THREADS / 2);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = gg_pdl_enabled() ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, sample_kernel<2>, logits, V, temperature, top_k, top_p, seeds, draw_index, out, room);
+    if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "sample: launch: %s", cudaGetErrorString(e));
+    return gg_check_launch("sample");
+  }
+  gg_launch(sample_kernel<1>, dim3(R), dim3(SAMPLE_THREADS), bytes, stream, logits, V, temperature, top_k, top_p, seeds, draw_index, out, room);
   return gg_check_launch("sample");
 }

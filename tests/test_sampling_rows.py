@@ -66,3 +66,29 @@ def test_tokens_lie_where_the_draw_does(ops, V, R, std, ways):
         wide = kept_probabilities(logits[r], float(torch.tensor(temps[r], dtype=torch.float32)), ks[r], p32 + 1e-4 if 0 < p32 < 1 else p32)
         assert wide[got] > 0, (r, got)
         assert float(cum[got] - q[got]) - 1e-4 <= u <= float(cum[got]) + 1e-4, (r, got)
+
+
+@pytest.mark.parametrize("V", [16384, 40003, 128256, 262400])
+@pytest.mark.parametrize("std", [2.5, 0.3])
+def test_rows_on_two_multiprocessors_draw_what_they_draw_on_one(ops, V, std):
+    """38 to 74 rows take two multiprocessors each, more of them one: the same sums in the same order, so the same tokens."""
+    R, many = 64, 150
+    gen = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(R, V, device="cuda", generator=gen) * std
+    logits[1] = torch.round(logits[1] * 4) / 4 + 0.0
+    logits[2, ::3] = -float("inf")
+    logits[3, : V // 2] = logits[3, V // 2:V // 2 * 2]          # the maximum twice, in both halves of the threads
+    logits[4, 7], logits[5, 9] = float("nan"), float("inf")
+    logits[6] = -float("inf")
+    ways = [(0, 0.9), (50, 0.9), (400, 0.0), (0, 0.0), (1024, 0.8), (3000, 0.95), (0, 0.3), (1, 0.0), (20000, 0.99)]
+    for s in range(6):
+        dev = lambda x, dt: torch.tensor(x, dtype=dt, device="cuda")  # noqa: E731
+        args = (dev([0.0 if r % 11 == 3 else 0.6 + 0.1 * (r % 5) for r in range(many)], torch.float32),
+                dev([ways[(r % R + s) % len(ways)][0] for r in range(many)], torch.int32),
+                dev([ways[(r % R + s) % len(ways)][1] for r in range(many)], torch.float32),
+                dev([r % R + 100 * s for r in range(many)], torch.int64), dev([3] * many, torch.int64))
+        args = (args[0][torch.arange(many, device="cuda") % R].contiguous(), *args[1:])
+        two, one = torch.empty(R, dtype=torch.int32, device="cuda"), torch.empty(many, dtype=torch.int32, device="cuda")
+        ops.sample(logits, *(a[:R].contiguous() for a in args), two)
+        ops.sample(logits[torch.arange(many, device="cuda") % R].contiguous(), *args, one)
+        assert torch.equal(two, one[:R]) and torch.equal(one[R:2 * R], one[:R])
