@@ -12,7 +12,7 @@
 // The products are float32 products made of three tf32 ones: x = hi + lo, hi to 11 bits, lo what is left (its first 11
 // bits count); hi hi + hi lo + lo hi, the term left out and what lo drops are 2^-21 of a product.  hi hi and the small terms
 // have accumulators of their own where tensor memory has the room (the tensor core's sums are cut off, not rounded).  Sums
-// of logarithms are float64 and are subtracted there, so strong decays cost no accuracy.
+// of logarithms are formed in float64, so strong decays cost no accuracy.
 // Infinities and NaN reach what they reach token by token: a bad value column, factor or decay the rows from its token on, a
 // bad k those rows in all columns, a bad q its own row, and the state.  There they are NaN, also where the walk would have
 // kept an infinity.  What rounds to infinity at 11 bits (from 2^128 (1 - 2^-12) on; no bfloat16 value does) counts as one.
@@ -83,8 +83,11 @@ __device__ __forceinline__ LcTokens lc_tokens(const LinearArgs& p, int t0, int n
   }
   return x;
 }
-// By one warp: L [128] (inclusive sums of log2 of the decays) and the factors b [128] of the chunk's n tokens.
-__device__ __forceinline__ void lc_sums(const LinearArgs& p, const LcTokens& x, int n, int h, double* L, float* b) {
+// Sums of logarithms as two float32 parts (48 bits): a difference of two is then three float32 subtractions and as exact as a float64
+// one that is rounded to float32 (which takes the multiprocessor's few float64 units and a conversion).
+struct LcSums { float hi[LC_C], lo[LC_C]; };
+// By one warp: L (inclusive sums of log2 of the decays) and the factors b [128] of the chunk's n tokens.  Returns their whole sum.
+__device__ __forceinline__ double lc_sums(const LinearArgs& p, const LcTokens& x, int n, int h, LcSums& L, float* b) {
   const int lane = threadIdx.x & 31;
   const float fixed = p.decay ? 0.f : p.log2_decay[h];
   double a[4], s = 0.0;
@@ -104,8 +107,14 @@ __device__ __forceinline__ void lc_sums(const LinearArgs& p, const LcTokens& x, 
   double before = __shfl_up_sync(0xffffffffu, incl, 1);
   if (lane == 0) before = 0.0;                         // (not incl - s: a NaN would reach the lane's tokens before it)
 #pragma unroll
-  for (int i = 0; i < 4; ++i) L[4 * lane + i] = before + a[i];
+  for (int i = 0; i < 4; ++i) {
+    const double l = before + a[i];
+    L.hi[4 * lane + i] = (float)l;
+    L.lo[4 * lane + i] = (float)(l - (double)(float)l);
+  }
+  return __shfl_sync(0xffffffffu, before + a[3], 31);
 }
+__device__ __forceinline__ float lc_power(float hi, float lo, float hi2, float lo2) { return exp2f((hi - hi2) + (lo - lo2)); }
 
 __device__ __forceinline__ void lc_split(float x, float& hi, float& lo) {
   hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
@@ -241,7 +250,7 @@ template <int STAGES> struct LcRing {
   __device__ __forceinline__ unsigned phase() const { return (s / STAGES) & 1; }
   // worker: the slot may be written
   __device__ __forceinline__ bool wait_empty(const LinearArgs& p, int* abort_s) {
-    ok = ok && mbar_wait(empty0 + 8 * slot(), phase() ^ 1) && !*(volatile int*)abort_s;
+    ok = ok && mbar_wait(empty0 + 8 * slot(), phase() ^ 1);
     ok = __all_sync(0xffffffffu, ok);
     if (!ok && (threadIdx.x & 31) == 0) { atomicExch(p.status, LC_ERR_EMPTY); atomicExch(abort_s, 1); }
     return ok;
@@ -256,7 +265,7 @@ template <int STAGES> struct LcRing {
   }
   // issuer
   __device__ __forceinline__ bool wait_full(const LinearArgs& p, int* abort_s) {
-    ok = ok && mbar_wait(full0 + 8 * slot(), phase()) && !*(volatile int*)abort_s;
+    ok = ok && mbar_wait(full0 + 8 * slot(), phase());
     if (!ok) { atomicExch(p.status, LC_ERR_FULL); atomicExch(abort_s, 1); }
     tc_fence_after();
     return ok;
@@ -281,7 +290,7 @@ linear_products_kernel(const LinearArgs p) {
   constexpr int STAGES = 2;
   extern __shared__ unsigned char lc_smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 1];
-  __shared__ double Ls[8][LC_C];
+  __shared__ LcSums Ls[8];
   __shared__ float ws[8][LC_C];
   __shared__ unsigned tmem_base_s;
   __shared__ int abort_s;
@@ -314,12 +323,12 @@ linear_products_kernel(const LinearArgs p) {
     v.load(vb, p.values_stride, n, cols);
   }
   if (warp < p.heads) {                                // (at most eight heads)
-    lc_sums(p, lc_tokens(p, t0, n, h0 + warp), n, h0 + warp, Ls[warp], ws[warp]);
+    const double all = lc_sums(p, lc_tokens(p, t0, n, h0 + warp), n, h0 + warp, Ls[warp], ws[warp]);
     __syncwarp();
-    const double all = Ls[warp][LC_C - 1];
+    const float hi = (float)all, lo = (float)(all - (double)hi);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) ws[warp][4 * lane + i] *= exp2f((float)(all - Ls[warp][4 * lane + i]));
-    if (lane == 0 && m0 == 0) p.factor[place * p.H + h0 + warp] = exp2f((float)all);
+    for (int i = 0; i < 4; ++i) ws[warp][4 * lane + i] *= lc_power(hi, lo, Ls[warp].hi[4 * lane + i], Ls[warp].lo[4 * lane + i]);
+    if (lane == 0 && m0 == 0) p.factor[place * p.H + h0 + warp] = exp2f(hi);
   }
   tc_fence_before();
   __syncthreads();
@@ -433,8 +442,9 @@ linear_rows_kernel(const LinearArgs p) {
   constexpr int BUFS = NB <= 64 ? 2 : 1;
   extern __shared__ unsigned char lc_smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 3];
-  __shared__ double Ls[8][LC_C];
-  __shared__ float bs[8][LC_C], fs[8][LC_C];
+  __shared__ __align__(16) LcSums Ls[8];
+  __shared__ __align__(16) float bs[8][LC_C];
+  __shared__ float fs[8][LC_C];
   __shared__ int first_s[8][NB], marked_s[8];          // of the heads' columns: the first token with infinity or NaN in v
   __shared__ unsigned tmem_base_s;
   __shared__ int abort_s;
@@ -499,7 +509,7 @@ linear_rows_kernel(const LinearArgs p) {
       lc_sums(p, tokens, n, h0 + warp, Ls[warp], bs[warp]);
       __syncwarp();
 #pragma unroll
-      for (int e = 0; e < 4; ++e) fs[warp][4 * lane + e] = exp2f((float)Ls[warp][4 * lane + e]);
+      for (int e = 0; e < 4; ++e) fs[warp][4 * lane + e] = exp2f(Ls[warp].hi[4 * lane + e]);
     }
     asm volatile("bar.sync 1, 512;" ::: "memory");
     const int quarter = warp & 3, i = quarter * 32 + lane;      // the row this thread has in tensor memory
@@ -598,7 +608,7 @@ linear_rows_kernel(const LinearArgs p) {
       if (hh == 0) ring.ok = ring.ok && lc_wait_done(scored, 0, p, &abort_s);
       LcAcross<NB> v;                                  // and the chunk's own tokens
       v.load(rv + (size_t)h * dv, p.values_stride, n, dv);
-      const double Li = Ls[hh][i];
+      const float Lhi = Ls[hh].hi[i], Llo = Ls[hh].lo[i];
       for (int s = 0; s < kj && ring.ok; ++s) {
         // this thread's eight scores of the step: row i, keys 32 s + 8 (warp / 4) ..
         unsigned m[8], x[8];
@@ -608,12 +618,18 @@ linear_rows_kernel(const LinearArgs p) {
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                      : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]) : "r"(tmem + lane_off + 128 + j0));
         tc_wait_load();
-        float w[8];
+        // (no branches: a masked key's power may overflow and is not taken; with them the eight powers came one after the other)
+        float w[8], hi[8], lo[8], bj[8];
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+          *reinterpret_cast<float4*>(hi + e) = *reinterpret_cast<const float4*>(Ls[hh].hi + j0 + e);
+          *reinterpret_cast<float4*>(lo + e) = *reinterpret_cast<const float4*>(Ls[hh].lo + j0 + e);
+          *reinterpret_cast<float4*>(bj + e) = *reinterpret_cast<const float4*>(bs[hh] + j0 + e);
+        }
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const int j = j0 + e;
-          const float sc = __uint_as_float(m[e]) + __uint_as_float(x[e]);
-          w[e] = j <= i ? sc * (exp2f((float)(Li - Ls[hh][j])) * bs[hh][j]) : 0.f;
+          const float f = (__uint_as_float(m[e]) + __uint_as_float(x[e])) * (lc_power(Lhi, Llo, hi[e], lo[e]) * bj[e]);
+          w[e] = j0 + e <= i ? f : 0.f;
         }
         if (!ring.wait_empty(p, &abort_s)) break;
         const unsigned at = base + ring.slot() * STAGE;
@@ -697,10 +713,14 @@ template <int NB, bool RETENTION, typename TA> static int lc_rows(const LinearAr
   return gg_check_launch("linear_rows");
 }
 
-// The rows: a CTA takes as many heads of a group as leave a CTA for every multiprocessor and two for most.
+// The rows: a CTA takes one to eight heads of a group, so many that the machine is done soonest.  A chunk's products q_i . k_j take a
+// CTA about as long as 0.8 of a head (10 k clocks of 12 k), and one CTA fits on a multiprocessor: 64 heads of a group and 16 chunks as
+// 128 CTAs of eight heads 92 us, as 256 of four 101; 16 heads on 4 groups as 128 CTAs of two 37, as 256 of one 45.
 template <bool RETENTION, typename TA> static int lc_all_rows(LinearArgs p, int num_tiles, cudaStream_t stream) {
   p.heads = 1;
-  while (p.heads < 8 && p.H / p.G % (2 * p.heads) == 0 && (long long)num_tiles * (p.H / (2 * p.heads)) >= 3 * 148 / 2) p.heads *= 2;
+  auto turns = [&](int heads) { return ((long long)num_tiles * (p.H / heads) + 147) / 148 * (4 + 5 * heads); };
+  for (int heads = 2; heads <= 8 && p.H / p.G % heads == 0; heads *= 2)
+    if (turns(heads) < turns(p.heads)) p.heads = heads;
   if (p.dv <= 64) return lc_rows<64, RETENTION, TA>(p, num_tiles, stream);
   if (p.dv <= 128) return lc_rows<128, RETENTION, TA>(p, num_tiles, stream);
   return lc_rows<256, RETENTION, TA>(p, num_tiles, stream);
