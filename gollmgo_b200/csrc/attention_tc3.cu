@@ -295,6 +295,8 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const float cap2 = X ? a.softcap * AT3_LOG2E : 0.f, to_cap = cap2 > 0.f ? sc / cap2 : 0.f;
     const int row_chunk = X && a.chunk > 0 ? (pos / a.chunk) * a.chunk : 0;
     const int tile_chunk = X && a.chunk > 0 ? ((first + nrows - 1) / a.chunk) * a.chunk : 0;
+    // the keys that this row sees: [row_from, row_end)
+    const int row_from = max(max(lo, row_chunk), a.window > 0 ? pos - a.window + 1 : 0), row_end = row_ok ? pos + 1 : 0;
     float m_ref = -INFINITY, l = 0.f;
     const int stale_hi = (hi + ps - 1) / ps * ps;        // end of the last page that is fetched
     bool ok = true;
@@ -344,12 +346,16 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
       }
       if (!interior) {
+        // the row's keys of the tile, [from, end), a bit each: two instructions a score (with the conditions written out a score, a
+        // chain of branches each, a masked tile took 9 to 20 thousand clocks, an unmasked one takes 5)
+        const int from = row_from - kb, end = row_end - kb;
 #pragma unroll
-        for (int i = 0; i < AT3_BK; ++i) {
-          const int tk = kb + i;
-          const bool keep = row_ok && tk >= lo && tk <= pos && (a.window <= 0 || tk > pos - a.window) &&
-                            (!X || tk >= row_chunk);
-          if (!keep) sv[i] = -INFINITY;
+        for (int c = 0; c < AT3_BK; c += 32) {
+          const int f = min(max(from - c, 0), 32), e = min(max(end - c, 0), 32);
+          const unsigned keep = (e >= 32 ? ~0u : (1u << e) - 1u) & (f >= 32 ? 0u : ~0u << f);
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (!(keep & (1u << i))) sv[c + i] = -INFINITY;
         }
       }
       // the maximum, three at a time in four chains (a chain of 128 dependent operations would be
