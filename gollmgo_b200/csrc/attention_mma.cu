@@ -773,6 +773,9 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_prefill_mma_kernel(AttnArgs 
   load_q_frags<D>(qf, [&](int r) { return wrow0 + r < nrows ? qbase + (size_t)r * a.q_stride : nullptr; });
   const bool row0_ok = wrow0 + g < nrows, row1_ok = wrow0 + g + 8 < nrows;
   const int wlast = first + min(wrow0 + 15, nrows - 1);  // last position this warp needs
+  // the keys that the thread's two rows see: so many from there on (one comparison a score; conditions of their own are branches)
+  const int from0 = max(lo, a.window > 0 ? pos0 - a.window + 1 : 0), from1 = max(lo, a.window > 0 ? pos1 - a.window + 1 : 0);
+  const unsigned keys0 = row0_ok ? max(pos0 + 1 - from0, 0) : 0, keys1 = row1_ok ? max(pos1 + 1 - from1, 0) : 0;
 
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   float o[D / 8][4];
@@ -804,11 +807,9 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_prefill_mma_kernel(AttnArgs 
         for (int j = 0; j < 8; ++j) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int tk = kb + j * 8 + c2 + (e & 1);
-            const int pos = (e & 2) ? pos1 : pos0;
-            const bool ok = ((e & 2) ? row1_ok : row0_ok) && tk >= lo && tk <= pos &&
-                            (a.window <= 0 || tk > pos - a.window);
-            s[j][e] = ok ? s[j][e] * sc : -INFINITY;
+            const int tk = kb + j * 8 + c2 + (e & 1), from = (e & 2) ? from1 : from0;
+            const unsigned n = (e & 2) ? keys1 : keys0;
+            s[j][e] = (unsigned)(tk - from) < n ? s[j][e] * sc : -INFINITY;
           }
         }
       }
@@ -1133,6 +1134,9 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_prefill_mma_x_kernel(AttnArg
   // chunked: the first key each of this thread's two rows sees, and the first any row of the warp sees
   const int cs0 = a.chunk > 0 ? (max(pos0, 0) / a.chunk) * a.chunk : 0, cs1 = a.chunk > 0 ? (max(pos1, 0) / a.chunk) * a.chunk : 0;
   const int wfirst = a.chunk > 0 ? ((first + wrow0) / a.chunk) * a.chunk : 0;
+  // the keys that the thread's two rows see (softmax): so many from there on
+  const int from0 = max(max(lo, cs0), a.window > 0 ? pos0 - a.window + 1 : 0), from1 = max(max(lo, cs1), a.window > 0 ? pos1 - a.window + 1 : 0);
+  const unsigned keys0 = row0_ok ? max(pos0 + 1 - from0, 0) : 0, keys1 = row1_ok ? max(pos1 + 1 - from1, 0) : 0;
   // this head's slope over the distance (base-2 exponents) and the two rows' scales (a query temperature is part of them)
   const float slope = !SIG && a.slopes ? a.slopes[h] * LOG2E : 0.f;
   const float scale0 = SIG ? a.scale : a.scale * query_temperature(a, pos0), scale1 = SIG ? a.scale : a.scale * query_temperature(a, pos1);
@@ -1167,8 +1171,8 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_prefill_mma_x_kernel(AttnArg
           for (int e = 0; e < 4; ++e) {
             const int tk = kb + j * 8 + c2 + (e & 1);
             const int pos = (e & 2) ? pos1 : pos0;
-            const bool ok = ((e & 2) ? row1_ok : row0_ok) && tk >= tlo && tk < thi && tk <= pos &&
-                            (a.window <= 0 || tk > pos - a.window || tk < a.keep_first);
+            const bool ok = ((e & 2) ? row1_ok : row0_ok) & (tk >= tlo) & (tk < thi) & (tk <= pos) &
+                            ((a.window <= 0) | (tk > pos - a.window) | (tk < a.keep_first));
             float x = s[j][e] * scale;
             if (cap > 0.f) {
               float th;
@@ -1176,7 +1180,8 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_prefill_mma_x_kernel(AttnArg
               x = cap * th;
             }
             x += tab[min(max(pos - tk, 0), a.dist_max)];
-            s[j][e] = ok ? sigmoid_weight(x) : 0.f;
+            const float w = sigmoid_weight(x);
+            s[j][e] = ok ? w : 0.f;
           }
         }
 #pragma unroll
@@ -1191,11 +1196,9 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_prefill_mma_x_kernel(AttnArg
         for (int j = 0; j < 8; ++j) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int tk = kb + j * 8 + c2 + (e & 1);
-            const int pos = (e & 2) ? pos1 : pos0;
-            const bool ok = ((e & 2) ? row1_ok : row0_ok) && tk >= lo && tk <= pos &&
-                            (a.window <= 0 || tk > pos - a.window) && tk >= ((e & 2) ? cs1 : cs0);
-            s[j][e] = ok ? score_exp2(s[j][e], (e & 2) ? scale1 : scale0, cap, inv_cap) : -INFINITY;
+            const int tk = kb + j * 8 + c2 + (e & 1), from = (e & 2) ? from1 : from0;
+            const float x = score_exp2(s[j][e], (e & 2) ? scale1 : scale0, cap, inv_cap);
+            s[j][e] = (unsigned)(tk - from) < ((e & 2) ? keys1 : keys0) ? x : -INFINITY;
           }
         }
         if (slope != 0.f) {                        // (a masked score stays -inf)
@@ -1360,10 +1363,12 @@ __global__ void __launch_bounds__(MMA_THREADS) attn_decode_mma_x_kernel(AttnArgs
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             const int tk = tok0 + j * 8 + c2;
-            s[j][0] = tk < hi ? score_exp2(s[j][0], scale, cap, inv_cap) : -INFINITY;
-            s[j][2] = tk < hi ? score_exp2(s[j][2], scale, cap, inv_cap) : -INFINITY;
-            s[j][1] = tk + 1 < hi ? score_exp2(s[j][1], scale, cap, inv_cap) : -INFINITY;
-            s[j][3] = tk + 1 < hi ? score_exp2(s[j][3], scale, cap, inv_cap) : -INFINITY;
+            const float x0 = score_exp2(s[j][0], scale, cap, inv_cap), x1 = score_exp2(s[j][1], scale, cap, inv_cap);
+            const float x2 = score_exp2(s[j][2], scale, cap, inv_cap), x3 = score_exp2(s[j][3], scale, cap, inv_cap);
+            s[j][0] = tk < hi ? x0 : -INFINITY;
+            s[j][1] = tk + 1 < hi ? x1 : -INFINITY;
+            s[j][2] = tk < hi ? x2 : -INFINITY;
+            s[j][3] = tk + 1 < hi ? x3 : -INFINITY;
             if (a.slopes) {
               const float away = (float)(ctx - 1 - tk);
               s[j][0] -= slope0 * away; s[j][2] -= slope1 * away;
