@@ -464,6 +464,163 @@ delta_out_vec_kernel(const float* __restrict__ o_raw, const TA* __restrict__ gat
   }
 }
 
+// ---------------------------------------------------------------- one token a sequence: all of it in one kernel
+// grid (H, B), 512 threads, a cluster of the rep heads that share q and k: convolution, norms, gates, recurrence, gated norm and the
+// window of a (sequence, head).  Eight lanes a column as in delta_recur, 64 columns at a time, NC times; the
+// state is asked into L2 before the products ahead are done.  Every block of a cluster makes q and k for itself; their window moves on once all have
+// read it.  What bounds it is the chain of launches it replaces: 4 sequences of 16 heads 128 x 128, layer 21.5 us with delta_prep,
+// delta_recur and delta_out (5.7 + 7.4 + 2.7 where they overlap), 18.5 in one.
+struct DeltaStepArgs {
+  const __nv_bfloat16* x;            // [T, x_stride]: columns [q: G d | k: G d | v: H dv]
+  long long x_stride;
+  const float* conv_w;
+  float* conv_state;
+  const float *zb, *za;
+  long long zb_stride, za_stride;
+  const float *a_log, *dt_bias;
+  float* state;
+  const int *cu_q_lens, *context_lens, *state_slots;
+  int G, H, d, dv, taps;
+  const __nv_bfloat16* gate;
+  long long gate_stride;
+  const float* norm_w;
+  float eps;
+  int gate_act;
+  __nv_bfloat16* out;                // [T, H dv]
+};
+#define DS_THREADS 512
+template <int DPT, int NC>
+__global__ void __launch_bounds__(DS_THREADS) delta_step_kernel(const DeltaStepArgs p) {
+  constexpr int D = DPT * DR_LANES, DV = 64 * NC;
+  __shared__ __align__(16) float qs[D], ks[D], vs[DV], os[DV];
+  __shared__ float gates[2];
+  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, r = tid & (DR_LANES - 1), cl = tid / DR_LANES;
+  const int rep = p.H / p.G, kvh = h / rep, C = 2 * p.G * D + p.H * DV, keep = p.taps - 1;
+  const int t = p.cu_q_lens[b], slot = p.state_slots[b];
+  const bool carried = slot >= 0 && p.context_lens[b] > 1;
+  pdl_trigger();
+  float* shead = p.state + ((size_t)max(slot, 0) * p.H + h) * DV * D;
+  if (carried && r < DPT / 4) {                        // the state's lines into L2 while the products ahead run (read after the wait)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(shead + (size_t)(cl + 64 * j) * D + 32 * r));
+  }
+  // four channels a thread: q, k, then v
+  constexpr int QT = D / 4, UNITS = 2 * QT + DV / 4;
+  const bool mine = tid < UNITS;
+  const int u = mine ? tid : 0, c = u < QT ? kvh * D + 4 * u : u < 2 * QT ? (p.G + kvh) * D + 4 * (u - QT) : 2 * p.G * D + h * DV + 4 * (u - 2 * QT);
+  float w[16];
+  float4 win[3];
+  if (mine) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < p.taps) *reinterpret_cast<float4*>(w + 4 * i) = *reinterpret_cast<const float4*>(p.conv_w + (size_t)c * p.taps + 4 * i);
+  }
+  pdl_wait();
+  float4 x4 = make_float4(0.f, 0.f, 0.f, 0.f), S[NC][DPT / 4];
+  if (mine) x4 = load4(p.x + (size_t)t * p.x_stride + c);
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+    win[s] = mine && carried && s < keep ? *reinterpret_cast<const float4*>(p.conv_state + ((size_t)slot * keep + s) * C + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int j = 0; j < NC; ++j)
+#pragma unroll
+    for (int i = 0; i < DPT / 4; ++i)
+      S[j][i] = carried ? *reinterpret_cast<const float4*>(shead + (size_t)(cl + 64 * j) * D + 32 * i + 4 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid == DS_THREADS - 1) {
+    gates[0] = 1.f / (1.f + expf(-p.zb[(size_t)t * p.zb_stride + h]));
+    gates[1] = expf(-expf(p.a_log[h]) * softplus_f(p.za[(size_t)t * p.za_stride + h] + p.dt_bias[h]));
+  }
+  if (tid < (UNITS + 31) / 32 * 32) {                  // (by whole warps)
+    const float xs[4] = {x4.x, x4.y, x4.z, x4.w};
+    float y[4], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float acc = 0.f;
+      const float ws[3] = {e == 0 ? win[0].x : e == 1 ? win[0].y : e == 2 ? win[0].z : win[0].w,
+                           e == 0 ? win[1].x : e == 1 ? win[1].y : e == 2 ? win[1].z : win[1].w,
+                           e == 0 ? win[2].x : e == 1 ? win[2].y : e == 2 ? win[2].z : win[2].w};
+      if (p.taps == 4) {
+#pragma unroll
+        for (int s = 0; s < 3; ++s) acc = fmaf(w[4 * e + s], ws[s], acc);
+        acc = fmaf(w[4 * e + 3], xs[e], acc);
+      } else if (p.taps == 3) {
+        acc = fmaf(w[3 * e], ws[0], acc);
+        acc = fmaf(w[3 * e + 1], ws[1], acc);
+        acc = fmaf(w[3 * e + 2], xs[e], acc);
+      } else {
+        acc = fmaf(w[2 * e], ws[0], acc);
+        acc = fmaf(w[2 * e + 1], xs[e], acc);
+      }
+      y[e] = mine ? silu_f(acc) : 0.f;
+    }
+    ss = y[0] * y[0] + y[1] * y[1] + (y[2] * y[2] + y[3] * y[3]);
+#pragma unroll
+    for (int o = QT / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float f = u < 2 * QT ? rsqrtf(ss + 1e-6f) * (u < QT ? rsqrtf((float)D) : 1.f) : 1.f;
+    if (mine) {
+      float* to = u < QT ? qs + 4 * u : u < 2 * QT ? ks + 4 * (u - QT) : vs + 4 * (u - 2 * QT);
+      *reinterpret_cast<float4*>(to) = make_float4(y[0] * f, y[1] * f, y[2] * f, y[3] * f);
+    }
+  }
+  // all blocks of the cluster have read the window
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (mine && slot >= 0 && (u >= 2 * QT || h % rep == 0)) {
+    float* to = p.conv_state + (size_t)slot * keep * C + c;
+    if (keep == 3) { store4(to, win[1]); store4(to + C, win[2]); store4(to + 2 * (size_t)C, x4); }
+    else if (keep == 2) { store4(to, win[1]); store4(to + C, x4); }
+    else store4(to, x4);
+  }
+  float4 q4[DPT / 4], k4[DPT / 4];
+#pragma unroll
+  for (int i = 0; i < DPT / 4; ++i) {
+    q4[i] = *reinterpret_cast<const float4*>(qs + 32 * i + 4 * r);
+    k4[i] = *reinterpret_cast<const float4*>(ks + 32 * i + 4 * r);
+  }
+  const float beta = gates[0], g = gates[1];
+  const float2 g2 = make_float2(g, g);
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    float2 dot2 = make_float2(0.f, 0.f), o2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < DPT / 4; ++i) {
+      dot2 = ffma2(make_float2(k4[i].x, k4[i].y), make_float2(S[j][i].x, S[j][i].y), dot2);
+      dot2 = ffma2(make_float2(k4[i].z, k4[i].w), make_float2(S[j][i].z, S[j][i].w), dot2);
+    }
+    float dot = dot2.x + dot2.y;
+#pragma unroll
+    for (int o = 1; o < DR_LANES; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    const float uu = beta * (vs[cl + 64 * j] - g * dot);
+    const float2 u2 = make_float2(uu, uu);
+#pragma unroll
+    for (int i = 0; i < DPT / 4; ++i) {
+      const float2 lo = ffma2(make_float2(k4[i].x, k4[i].y), u2, fmul2(g2, make_float2(S[j][i].x, S[j][i].y)));
+      const float2 hi = ffma2(make_float2(k4[i].z, k4[i].w), u2, fmul2(g2, make_float2(S[j][i].z, S[j][i].w)));
+      o2 = ffma2(make_float2(q4[i].x, q4[i].y), lo, o2);
+      o2 = ffma2(make_float2(q4[i].z, q4[i].w), hi, o2);
+      if (slot >= 0) *reinterpret_cast<float4*>(shead + (size_t)(cl + 64 * j) * D + 32 * i + 4 * r) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    float o = o2.x + o2.y;
+#pragma unroll
+    for (int m = 1; m < DR_LANES; m <<= 1) o += __shfl_xor_sync(0xffffffffu, o, m);
+    if (r == 0) os[cl + 64 * j] = o;
+  }
+  __syncthreads();
+  if (tid < 32) {                                      // the gated norm: two, four or eight values a lane
+    constexpr int N = DV / 32;
+    float v[N], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) { v[i] = os[32 * i + tid]; ss += v[i] * v[i]; }
+    const float f = rsqrtf(warp_sum(ss) / (float)DV + p.eps);
+    const __nv_bfloat16* z = p.gate + (size_t)t * p.gate_stride + (size_t)h * DV;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const float zz = to_f32(z[32 * i + tid]);
+      p.out[((size_t)t * p.H + h) * DV + 32 * i + tid] =
+          __float2bfloat16_rn(v[i] * f * p.norm_w[32 * i + tid] * (p.gate_act == 1 ? 1.f / (1.f + expf(-zz)) : silu_f(zz)));
+    }
+  }
+}
+
 // ---------------------------------------------------------------- launchers
 // The window of a short convolution over the C channels x[:, 0 .. C) moved on by this step's tokens
 // (also for the state-space layer, ssm.cu).
@@ -598,4 +755,45 @@ extern "C" int gg_delta_out(const float* o_raw, const void* gate, long long gate
   else
     return gg_fail(GG_ERR_INVALID, "delta_out: unknown dtype %d", dtype);
   return gg_check_launch("delta_out");
+}
+
+// delta_prep, delta_recur and delta_out for a step of one token a sequence (bfloat16, a decay per head, a weight in the norm).
+// Returns GG_ERR_UNSUPPORTED, and launches nothing, where sizes or addresses are not for it.
+extern "C" int gg_delta_step(const void* x, long long x_stride, const float* conv_w, float* conv_state, const float* zb, long long zb_stride,
+                             const float* za, long long za_stride, const float* a_log, const float* dt_bias, float* state,
+                             const int* cu_q_lens, const int* context_lens, const int* state_slots, int B, int G, int H, int d, int dv,
+                             int taps, const void* gate, long long gate_stride, const float* norm_w, float eps, int gate_act, void* out,
+                             cudaStream_t stream) {
+  GG_REQUIRE(B >= 0 && G > 0 && H > 0 && H % G == 0 && d > 0 && dv > 0, "delta_step: bad sizes B=%d G=%d H=%d d=%d dv=%d", B, G, H, d, dv);
+  GG_REQUIRE(x && conv_w && conv_state && zb && za && a_log && dt_bias && state && gate && norm_w && out, "delta_step: a pointer is null");
+  const int rep = H / G;
+  const size_t addresses = (size_t)x | (size_t)conv_w | (size_t)conv_state | (size_t)state;
+  if ((d != 64 && d != 128) || (dv != 64 && dv != 128 && dv != 256) || taps < 2 || taps > 4 || (rep != 1 && rep != 2 && rep != 4 && rep != 8) ||
+      x_stride % 4 || addresses % 16 || B > 65535)
+    return GG_ERR_UNSUPPORTED;
+  // Up to 32 MB of states: beyond, the recurrence's blocks of sixteen columns, several on a multiprocessor, keep more of them on their
+  // way.  Layer, us, three kernels / one, 16 heads 128 x 128: 8 sequences 30.7 / 26.6, 16: 38.9 / 34.8, 33: 55.3 / 55.3, 64: 67.6 / 75.8;
+  // 32 heads: 8: 57.3 / 53.2, 16: 67.6 / 67.6, 33: 92.2 / 100.4; 16 heads 64 x 128: 16: 32.8 / 26.7, 64: 53.2 / 49.2.
+  if ((long long)B * H * d * dv > 1ll << 23) return GG_ERR_UNSUPPORTED;
+  if (B == 0) return GG_OK;
+  DeltaStepArgs p = {(const __nv_bfloat16*)x, x_stride, conv_w, conv_state, zb, za, zb_stride, za_stride, a_log, dt_bias, state, cu_q_lens,
+                     context_lens, state_slots, G, H, d, dv, taps, (const __nv_bfloat16*)gate, gate_stride, norm_w, eps, gate_act, (__nv_bfloat16*)out};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(H, B);
+  cfg.blockDim = dim3(DS_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = rep;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gg_pdl_enabled() ? 2 : 1;
+  cudaError_t e;
+  if (d == 64) e = dv == 64 ? cudaLaunchKernelEx(&cfg, delta_step_kernel<8, 1>, p) : dv == 128 ? cudaLaunchKernelEx(&cfg, delta_step_kernel<8, 2>, p) : cudaLaunchKernelEx(&cfg, delta_step_kernel<8, 4>, p);
+  else e = dv == 64 ? cudaLaunchKernelEx(&cfg, delta_step_kernel<16, 1>, p) : dv == 128 ? cudaLaunchKernelEx(&cfg, delta_step_kernel<16, 2>, p) : cudaLaunchKernelEx(&cfg, delta_step_kernel<16, 4>, p);
+  if (e != cudaSuccess) return gg_fail(GG_ERR_CUDA, "delta_step: %s", cudaGetErrorString(e));
+  return gg_check_launch("delta_step");
 }

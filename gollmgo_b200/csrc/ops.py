@@ -1098,6 +1098,30 @@ def delta_out(o_raw: torch.Tensor, gate: torch.Tensor, weight: Optional[torch.Te
                               _p(out), _stream()))
 
 
+def delta_step(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, zb: torch.Tensor, za: torch.Tensor,
+               a_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, cu_q_lens: torch.Tensor, context_lens: torch.Tensor,
+               state_slots: torch.Tensor, num_seqs: int, kv_heads: int, heads: int, d: int, dv: int, gate: torch.Tensor,
+               norm_w: torch.Tensor, eps: float, out: torch.Tensor, gate_act: str = "silu") -> bool:
+    """delta_prep, delta_recur and delta_out in one kernel for a step of one token a sequence, bfloat16 with a decay per head.
+    False, and nothing done, where sizes or addresses are not for it."""
+    _cuda(conv_w, conv_state, a_log, dt_bias, state, norm_w, out)
+    C, taps = conv_w.shape
+    if x.stride(1) != 1 or x.dtype != torch.bfloat16 or C != 2 * kv_heads * d + heads * dv or conv_w.dtype != torch.float32 \
+            or conv_state.dtype != torch.float32 or zb.dtype != torch.float32 or za.dtype != torch.float32 or zb.stride(1) != 1 \
+            or za.stride(1) != 1 or zb.shape[1] != heads or za.shape[1] != heads or dt_bias.numel() != heads or state.dtype != torch.float32 \
+            or tuple(state.shape[1:]) != (heads, dv, d) or gate.stride(1) != 1 or gate.dtype != out.dtype or norm_w.dtype != torch.float32 \
+            or out.dtype != torch.bfloat16 or x.shape[0] != num_seqs:
+        raise KernelError("delta_step: bad shapes or dtypes")
+    rc = lib().gg_delta_step(_p(x), ctypes.c_longlong(x.stride(0)), _p(conv_w), _p(conv_state), _p(zb), ctypes.c_longlong(zb.stride(0)),
+                             _p(za), ctypes.c_longlong(za.stride(0)), _p(a_log), _p(dt_bias), _p(state), _p(cu_q_lens), _p(context_lens),
+                             _p(state_slots), num_seqs, kv_heads, heads, d, dv, taps, _p(gate), ctypes.c_longlong(gate.stride(0)),
+                             _p(norm_w), ctypes.c_float(eps), {"silu": 0, "sigmoid": 1}[gate_act], _p(out), _stream())
+    if rc == 3:                                            # GG_ERR_UNSUPPORTED
+        return False
+    _check(rc)
+    return True
+
+
 # ---------------------------------------------------------------- state-space layer
 def ssm_prep(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: Optional[torch.Tensor], conv_state: Optional[torch.Tensor],
              a_log: torch.Tensor, dt_bias: torch.Tensor, cu_q_lens: torch.Tensor, context_lens: torch.Tensor,

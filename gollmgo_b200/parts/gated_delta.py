@@ -207,19 +207,23 @@ class GatedDeltaRule:
         else:
             ba = linear(x, self.w_ba, ws.get("delta_ba", T, H + hw))
             zb, za = ba[:, :H], ba[:, H:]
-        qkv = ws.get("delta_qkv", T, self.channels)
-        beta, decay = ws.get("delta_beta", T, H), ws.get("delta_decay", T, hw)
-        B = batch.num_seqs
-        ops.delta_prep(proj, self.conv_w, conv_state, zb, za, self.a_log, self.dt_bias, batch.cu_q_lens, batch.context_lens,
-                       batch.state_slots, B, self.nkv, self.nh, self.d, self.dv, qkv, beta, decay)
-        o = ws.get("delta_o", T, self.nh * self.dv)
-        self._recur(qkv, beta, decay, state, batch, o)
         y = ws.get("delta_y", T, self.nh * self.dv)
         if self.gate_rank:
             gate = linear(proj[:, self.gate_col:self.a_col if self.a_rank else self.proj_width], self.w_g2,
                           ws.get("delta_gate", T, self.nh * self.dv))
         else:
             gate = proj[:, self.gate_col:self.gate_col + self.gate_cols]
+        B = batch.num_seqs
+        if T == B and batch.num_portions == 0 and self.dw == 1 and self.taps > 1 and proj.dtype == torch.bfloat16 and ops.delta_step(
+                proj, self.conv_w, conv_state, zb, za, self.a_log, self.dt_bias, state, batch.cu_q_lens, batch.context_lens,
+                batch.state_slots, B, self.nkv, H, self.d, self.dv, gate, self.norm_w, self.eps, y, self.gate_act):
+            return linear(y, self.w_o, ws.get(self.out_buffer, T, self.hidden), then)
+        qkv = ws.get("delta_qkv", T, self.channels)
+        beta, decay = ws.get("delta_beta", T, H), ws.get("delta_decay", T, hw)
+        ops.delta_prep(proj, self.conv_w, conv_state, zb, za, self.a_log, self.dt_bias, batch.cu_q_lens, batch.context_lens,
+                       batch.state_slots, B, self.nkv, self.nh, self.d, self.dv, qkv, beta, decay)
+        o = ws.get("delta_o", T, self.nh * self.dv)
+        self._recur(qkv, beta, decay, state, batch, o)
         ops.delta_out(o, gate, self.norm_w, self.eps, self.nh, self.dv, y, self.gate_act)
         return linear(y, self.w_o, ws.get(self.out_buffer, T, self.hidden), then)
 
