@@ -45,6 +45,9 @@ struct GsmFuse {
   // and u = clamp(up, -limit, limit), g * sigmoid(alpha * g) * (u + shift)
   float act_limit, act_alpha, act_shift;
   int relu2;                  // GSM_OUT_BF16: the square of relu of the result
+  // GSM_OUT_BF16, split > 0: rows of W from split on go to tail [M, N - split] in float32, the others to out [M, split]
+  int split;
+  float* tail;
 };
 
 #define GSM_STAGES 6
@@ -267,7 +270,10 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
               if (fuse.in_partials) v *= row_scale[tok];
               if (MODE == GSM_OUT_BF16 && fuse.relu2) { v = fmaxf(v, 0.f); v *= v; }
               if (MODE == GSM_OUT_F32) reinterpret_cast<float*>(out)[(size_t)tok * N + n] = v;
-              else reinterpret_cast<__nv_bfloat16*>(out)[(size_t)tok * N + n] = __float2bfloat16_rn(v);
+              else if (MODE == GSM_OUT_BF16 && fuse.split > 0) {
+                if (n < fuse.split) reinterpret_cast<__nv_bfloat16*>(out)[(size_t)tok * fuse.split + n] = __float2bfloat16_rn(v);
+                else fuse.tail[(size_t)tok * (N - fuse.split) + n - fuse.split] = v;
+              } else reinterpret_cast<__nv_bfloat16*>(out)[(size_t)tok * N + n] = __float2bfloat16_rn(v);
             }
           }
         }
@@ -285,7 +291,8 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
 static int gemm_small_m_run(const void* x, long long ldx, const void* W, void* out, int M, int N,
                             int K, int mode, const float* in_partials, int in_tiles, int hidden,
                             float eps, float* resid, const float* norm_w, float* out_partials,
-                            float act_limit, float act_alpha, float act_shift, cudaStream_t stream, int relu2 = 0) {
+                            float act_limit, float act_alpha, float act_shift, cudaStream_t stream, int relu2 = 0,
+                            int split = 0, float* tail = nullptr) {
   GG_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_small_m: bad sizes M=%d N=%d K=%d", M, N, K);
   GG_REQUIRE(M <= 16, "gemm_small_m: %d tokens; this kernel takes at most 16", M);
   GG_REQUIRE(K % 8 == 0 && ldx % 8 == 0, "gemm_small_m: K=%d and the row stride %lld of x must be multiples of 8", K, ldx);
@@ -299,6 +306,7 @@ static int gemm_small_m_run(const void* x, long long ldx, const void* W, void* o
   fuse.inv_h = hidden > 0 ? 1.0f / (float)hidden : 0.f; fuse.eps = eps;
   fuse.resid = resid; fuse.norm_w = norm_w; fuse.out_partials = out_partials;
   fuse.act_limit = act_limit; fuse.act_alpha = act_alpha; fuse.act_shift = act_shift; fuse.relu2 = relu2;
+  fuse.split = split; fuse.tail = tail;
   const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
   const __nv_bfloat16* wp = (const __nv_bfloat16*)W;
   const int num_tiles = mode == GSM_OUT_SILU ? (N + 7) / 8 : (N + 15) / 16;
@@ -354,6 +362,15 @@ extern "C" int gg_gemm_small_m_clamped(const void* x, long long ldx, const void*
                                        float limit, float alpha, float shift, cudaStream_t stream) {
   GG_REQUIRE(limit > 0.f, "gemm_small_m: the clamped activation needs a positive limit");
   return gemm_small_m_run(x, ldx, W, out, M, N, K, 2, nullptr, 0, 0, 0.f, nullptr, nullptr, nullptr, limit, alpha, shift, stream);
+}
+
+// Two products of the same x in one launch: rows [0, split) of W to out [M, split] in bfloat16, the rest to tail [M, N - split] in float32.
+// in_partials (or null) as above.
+extern "C" int gg_gemm_small_m_tail(const void* x, long long ldx, const void* W, void* out, float* tail, int M, int N, int split, int K,
+                                    const float* in_partials, int in_tiles, int hidden, float eps, cudaStream_t stream) {
+  GG_REQUIRE(split > 0 && split < N && tail, "gemm_small_m: a tail of %d of %d rows", N - split, N);
+  return gemm_small_m_run(x, ldx, W, out, M, N, K, 0, in_partials, in_tiles, hidden, eps, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f, stream, 0,
+                          split, tail);
 }
 
 // out = the square of relu(x W^T), bfloat16.

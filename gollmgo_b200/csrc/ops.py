@@ -352,6 +352,26 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: boo
                                        _p(resid), _p(norm_w), _p(out_partials), _stream()))
 
 
+def gemm_small_m_tail(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tail: torch.Tensor, in_partials: Optional[torch.Tensor] = None,
+                      hidden: int = 0, eps: float = 0.0) -> None:
+    """gemm_small_m for two products of one x: the first rows of w to out (bfloat16), the others to tail (float32)."""
+    M, K = x.shape
+    split, N = out.shape[1], w.shape[0]
+    if w.shape != (split + tail.shape[1], K) or out.shape[0] != M or tail.shape[0] != M or not out.is_contiguous() or not tail.is_contiguous() \
+            or out.dtype != torch.bfloat16 or tail.dtype != torch.float32 or x.dtype != torch.bfloat16 or x.stride(1) != 1 \
+            or w.dtype != torch.bfloat16 or not w.is_contiguous():
+        raise KernelError("gemm_small_m_tail: shapes or dtypes do not fit")
+    in_tiles = 0
+    if in_partials is not None:
+        if in_partials.dtype != torch.float32 or in_partials.dim() != 2 or in_partials.shape[1] != 16 \
+                or not in_partials.is_contiguous() or hidden <= 0:
+            raise KernelError("gemm_small_m_tail: in_partials must be contiguous float32 [tiles, 16] with the hidden size given")
+        in_tiles = in_partials.shape[0]
+    _cuda(w, out, tail, in_partials)
+    _check(lib().gg_gemm_small_m_tail(_p(x), ctypes.c_longlong(x.stride(0)), _p(w), _p(out), _p(tail), M, N, split, K, _p(in_partials),
+                                      in_tiles, int(hidden), ctypes.c_float(eps), _stream()))
+
+
 def gemm_small_m_clamped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, limit: float, alpha: float,
                          shift: float) -> None:
     """The gated product of gemm_small_m (w [2N, K]: gate rows, then up rows) with the clamped

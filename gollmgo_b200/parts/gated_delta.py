@@ -31,7 +31,7 @@ import torch
 from ..cache import FixedStateNeed
 from ..csrc import ops
 from ..weights import WeightSpec
-from .linear import linear
+from .linear import linear, linear_with_tail
 from .linear_recurrence import ChunkTiles
 from .registry import register_mixer
 
@@ -96,7 +96,7 @@ class GatedDeltaRule:
                             ops.delta_solved_floats(T, T // limit, self.nkv, self.nh, self.d))
             ws.reserve("linear_states", self.scratch[0], torch.float32)
             ws.reserve("delta_solved", self.scratch[1], torch.float32)
-        self.w_proj = self.w_ba = self.w_o = self.w_a2 = self.w_g2 = None
+        self.w_all = self.w_proj = self.w_ba = self.w_o = self.w_a2 = self.w_g2 = None
         self.conv_w = self.a_log = self.dt_bias = self.norm_w = None
 
     def _layout(self):
@@ -169,7 +169,10 @@ class GatedDeltaRule:
             self.w_g2 = torch.zeros(g2.shape[0], self.a_col - self.gate_col if self.a_rank else self.proj_width - self.gate_col,
                                     dtype=g2.dtype, device=g2.device)
             self.w_g2[:, :self.gate_rank] = g2
-        self.w_proj = w_proj.contiguous()
+        self.w_all, self.w_proj = None, w_proj.contiguous()
+        if self.w_ba.dtype == dt == torch.bfloat16:        # one behind the other: steps of a few tokens multiply both in one launch
+            self.w_all = torch.cat([self.w_proj, self.w_ba], dim=0)
+            self.w_proj, self.w_ba = self.w_all[:self.proj_width], self.w_all[self.proj_width:]
         self.w_o = get(n["o"]).contiguous()
         self.conv_w = torch.cat([get(n[x] + ".conv").float() for x in ("q", "k", "v")], dim=0).contiguous()
         self.a_log = get(n["A_log"]).float().contiguous()
@@ -198,14 +201,13 @@ class GatedDeltaRule:
         state = cache[0]
         conv_state = cache[1] if self.taps > 1 else state        # unused without taps to carry
         H, hw = self.nh, self.nh * self.dw
-        proj = linear(x, self.w_proj, ws.get("delta_proj", T, self.proj_width))
+        proj, ba = ws.get("delta_proj", T, self.proj_width), ws.get("delta_ba", T, H + hw)
         if self.a_rank:
             # beta straight from x; the decay's input through its two products (the inner values are columns of proj)
-            ba = ws.get("delta_ba", T, H + hw)
-            zb = linear(x, self.w_ba, ba.view(-1)[:T * H].view(T, H))
+            proj, zb = linear_with_tail(x, self.w_all, self.w_proj, self.w_ba, proj, ba.view(-1)[:T * H].view(T, H))
             za = linear(proj[:, self.a_col:], self.w_a2, ba.view(-1)[T * H:].view(T, hw))
         else:
-            ba = linear(x, self.w_ba, ws.get("delta_ba", T, H + hw))
+            proj, ba = linear_with_tail(x, self.w_all, self.w_proj, self.w_ba, proj, ba)
             zb, za = ba[:, :H], ba[:, H:]
         y = ws.get("delta_y", T, self.nh * self.dv)
         if self.gate_rank:

@@ -57,3 +57,24 @@ def test_refuses_what_it_does_not_take(ops):
     assert not ops.delta_step(x, z(C, taps), z(B, taps - 1, C), z(B, H), z(B, H), z(H), z(H), z(B, H, dv, d), i32([0, 1, 2]), i32([1, 1]), i32([0, 1]),
                               B, G, H, d, dv, x[:, C:], z(dv), 1e-6, y)
     assert bool((y == 7.0).all())
+
+
+@pytest.mark.parametrize("M,split,more,K", [(1, 16, 1, 64), (4, 5120, 32, 2048), (16, 40, 16, 200), (9, 200, 33, 520)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_two_products_in_one_launch(ops, M, split, more, K, normed):
+    """gemm_small_m with a float32 tail beside the two products, also behind a norm folded into x."""
+    gen = torch.Generator(device="cuda").manual_seed(split)
+    x = torch.randn(M, K, device="cuda", generator=gen).bfloat16()
+    w = torch.randn(split + more, K, device="cuda", generator=gen).bfloat16() * K ** -0.5
+    kw = {}
+    if normed:
+        parts = torch.rand(-(-K // 16), 16, device="cuda", generator=gen) + 1.0
+        kw = dict(in_partials=parts, hidden=K, eps=1e-6)
+    out, tail = torch.empty(M, split, device="cuda", dtype=torch.bfloat16), torch.empty(M, more, device="cuda")
+    ops.gemm_small_m_tail(x, w, out, tail, **kw)
+    a, b = torch.empty_like(out), torch.empty_like(tail)
+    ops.gemm_small_m(x, w[:split].contiguous(), a, **kw)
+    ops.gemm_small_m(x, w[split:].contiguous(), b, **kw)
+    # the same float32 sums; a row's block may start elsewhere along K
+    assert float((tail - b).norm() / b.norm()) < 1e-6
+    assert float((out.float() - a.float()).norm() / a.float().norm()) < 1e-3
