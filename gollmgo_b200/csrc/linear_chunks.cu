@@ -25,7 +25,6 @@
 // float32 232.  Slower: reads two steps ahead (registers spill: rows 130 and 117); groups of four warps with a step each
 // (rows 112); two issuers (no change).
 // All waits on barriers are bounded; one that runs out sets *status and the CTA winds down.
-#include "delta_chunks.cuh"
 #include "tc_common.cuh"
 
 #define LC_C 128               // tokens of a chunk
@@ -741,18 +740,6 @@ template <bool RETENTION, typename TA> static int lc_run(LinearArgs p, int num_t
   if (rc) return rc;
   return lc_all_rows<RETENTION, TA>(p, num_tiles, stream);
 }
-
-// The delta rule's rows (delta_chunks.cu): what its tokens write stands in the result's place.
-static LinearArgs lc_of_delta(const DeltaChunkArgs& c) {
-  LinearArgs p = {};
-  p.rows = c.rows; p.row_stride = c.row_stride; p.q_col = 0; p.k_col = c.k_col; p.values = c.o_raw; p.values_stride = (long long)c.H * c.dv;
-  p.decay = c.decay; p.state = c.state; p.scratch = c.scratch; p.tile_seq = c.tile_seq; p.tile_q0 = c.tile_q0; p.tiles = c.tiles;
-  p.cu_q_lens = c.cu_q_lens; p.context_lens = c.context_lens; p.state_slots = c.state_slots;
-  p.B = c.B; p.G = c.G; p.H = c.H; p.d = c.d; p.dv = c.dv; p.o_raw = c.o_raw; p.status = c.status;
-  return p;
-}
-bool delta_rows_supported(const DeltaChunkArgs& p) { return lc_supported(lc_of_delta(p)); }
-int delta_rows(const DeltaChunkArgs& p, cudaStream_t stream) { return lc_all_rows<false, float>(lc_of_delta(p), p.tiles, stream); }
 
 // gg_delta_recur's plain recurrence over the sequences whose chunks of 128 tokens are the tiles (all chunks of a sequence, in
 // their order); the others are left alone.  Returns GG_ERR_UNSUPPORTED, and launches nothing, where sizes or addresses are not

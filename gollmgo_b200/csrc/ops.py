@@ -1054,10 +1054,11 @@ def delta_chunks_ok(d: int, dv: int) -> bool:
     return d % 32 == 0 and d <= 128 and dv % 16 == 0 and dv <= 256
 
 
-def delta_solved_floats(num_tokens: int, num_seqs: int, kv_heads: int, heads: int, d: int) -> int:
-    """Size of delta_chunks' second scratch for a step of num_tokens in num_seqs portions: solved keys per head, keys, a factor per
-    token and head."""
-    return (num_tokens // LINEAR_CHUNK + num_seqs + 1) * LINEAR_CHUNK * (heads + kv_heads) * (64 if d <= 64 else 128) + num_tokens * heads
+def delta_solved_floats(num_tokens: int, num_seqs: int, kv_heads: int, heads: int, d: int, dv: int = 256) -> int:
+    """Size of delta_chunks' second scratch for a step of num_tokens in num_seqs portions: solved keys per head, keys, states in the
+    middle of a chunk of LINEAR_CHUNK, a factor per token and head."""
+    tiles = num_tokens // LINEAR_CHUNK + num_seqs + 1
+    return tiles * (LINEAR_CHUNK * (heads + kv_heads) * (64 if d <= 64 else 128) + heads * (d * dv + LINEAR_CHUNK + 2))
 
 
 def delta_chunks(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
@@ -1065,8 +1066,8 @@ def delta_chunks(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, sta
                  context_lens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, kv_heads: int, heads: int, d: int,
                  dv: int, o_raw: torch.Tensor) -> bool:
     """delta_recur (a decay per head) over the sequences whose chunks of LINEAR_CHUNK tokens tile_seq and tile_q0 list, as
-    linear_chunks does for the plain recurrence.  scratch: float32 of linear_scratch_floats(); solved: of delta_solved_floats().
-    False, and nothing done, where sizes or addresses are not for these kernels."""
+    linear_chunks does for the plain recurrence, in float32.  scratch: float32 of linear_scratch_floats(); solved: of
+    delta_solved_floats().  False, and nothing done, where sizes or addresses are not for these kernels."""
     _cuda(qkv, beta, decay, state, scratch, solved, o_raw)
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, d) or decay.shape[-1] != heads \
             or qkv.dtype != torch.float32 or scratch.dtype != torch.float32 or solved.dtype != torch.float32:

@@ -26,6 +26,9 @@ convolutions' tensors are the q, k, v names + ".conv").
 """
 from __future__ import annotations
 
+import math
+from dataclasses import dataclass
+
 import torch
 
 from ..cache import FixedStateNeed
@@ -35,13 +38,43 @@ from .linear import linear, linear_with_tail
 from .linear_recurrence import ChunkTiles
 from .registry import register_mixer
 
-# Portions of so many tokens take the chunk form (csrc/delta_chunks.cu): its three kernels take some 45 us however short they are,
-# the walk as long as its longest portion.  A B200, us, chunks / walk, values of 128 (16 heads on 4, 32 on 8; 16 on 4 with 64 keys):
-#   128 keys: 192: 58 / 43, 62 / 55   256: 62 / 55, 66 / 70   512: 77 / 102, 87 / 133   8 x 256: 158 / 190, 269 / 356   16 x 64: 126 / 98
-#   64 keys:  256: 52 / 43            512: 64 / 78            8 x 256: 124 / 113
-# A few short portions beside a long one: 256 + 3 x 30: 72 / 108; many: 256 + 30 x 8: 214 / 119 (ChunkTiles divides those).
-def chunks_from(d):
-    return 320 if d > 64 else 384
+# Portions of so many tokens may take the chunk form (csrc/delta_chunks.cu).  A B200, us, chunks / walk, values of 128, 16 heads on 4
+# (128 keys also 32 on 8):
+#   128 keys: 256: 56 / 50, 67 / 64   320: 64 / 62, 82 / 80   384: 68 / 74, 88 / 95   512: 76 / 97, 98 / 126   2048: 212 / 382, 336 / 497
+#   64 keys:  256: 41 / 37            384: 49 / 55            512: 52 / 73            2048: 133 / 284
+CHUNKS_FROM = 384
+
+
+@dataclass(frozen=True)
+class DeltaTiles(ChunkTiles):
+    """ChunkTiles for steps whose chunks are also estimated to take less time than the walk.  The walk takes its longest portion's
+    tokens one after the other until its blocks, sixteen value columns of a sequence and head each, fill the machine, and then what all
+    of them take; the chunks their fixed cost, one chunk after the other, and the arithmetic of all.  Estimates in us, each of two
+    parts as the root of their squares' sum; of 165 steps measured on a B200 (11 kinds of layer, 1 to 20 portions of 64 to 2048 tokens)
+    117 and 142 took what is estimated to within a tenth, and none in chunks took over 1 % longer than walked.  What decides between them, chunks / walk: 16 heads, 64 keys, 8 x 384 tokens: 179 / 157, one of 384:
+    49 / 55; 48 heads of 64 x 64, 700 + 513 + 835: 259 / 196, one of 2048: 261 / 337; 4 heads of 32 x 16, 20 x 512: 100 / 69."""
+    heads: int = 1
+    d: int = 128
+    dv: int = 128
+
+    __hash__ = ChunkTiles.__hash__
+
+    def chunk_us(self, lens):
+        D, cols = (64 if self.d <= 64 else 128), (64 if self.dv <= 64 else -(-self.dv // 128) * 128)       # (as the kernels pad them)
+        chunks = [-(-n // 64) for n in lens]
+        return (30 if cols <= 128 else 40) + math.hypot((0.06 + 1.5e-5 * D * cols) * self.heads * sum(chunks), 0.027 * D * max(chunks))
+
+    def walk_us(self, lens):
+        return math.hypot((0.095 + 7.2e-4 * self.d) * max(lens), (1.3e-4 + 4.2e-6 * self.d) * sum(lens) * self.heads * self.dv / 16)
+
+    def chosen(self, portions, q_lens, q_starts):
+        listed = super().chosen(portions, q_lens, q_starts)
+        if not listed:
+            return listed
+        here = set(listed)
+        rest = [q_lens[b] for b in portions if b not in here]          # walked behind the chunks
+        cost = self.chunk_us([q_lens[b] for b in listed]) + (5 + self.walk_us(rest) if rest else 0)
+        return listed if 1.04 * cost < self.walk_us([q_lens[b] for b in portions]) else []
 
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "beta": "b", "a": "a", "gate": "g", "o": "o", "A_log": "A_log",
@@ -87,13 +120,14 @@ class GatedDeltaRule:
         ws.reserve("delta_o", T * self.nh * self.dv, torch.float32)
         ws.reserve("delta_y", T * self.nh * self.dv, ctx.act_dtype)
         ws.reserve(self.out_buffer, T * self.hidden, ctx.act_dtype)
-        # (the chunks' rows are products of three tf32 parts: a model served in float32 keeps the walk)
+        # (float32 arithmetic too, its sums in another order: a model served in float32 keeps the walk's)
         self.chunks = None
         if self.dw == 1 and ctx.act_dtype != torch.float32 and ops.delta_chunks_ok(self.d, self.dv):
-            limit = chunks_from(self.d)
-            self.chunks = ChunkTiles(ops.LINEAR_CHUNK, at_least=limit, longest=limit, most=T // ops.LINEAR_CHUNK + T // limit)
+            limit = CHUNKS_FROM
+            self.chunks = DeltaTiles(ops.LINEAR_CHUNK, at_least=limit, longest=limit, most=T // ops.LINEAR_CHUNK + T // limit,
+                                     heads=self.nh, d=self.d, dv=self.dv)
             self.scratch = (ops.linear_scratch_floats(T, T // limit, self.nh, self.d, self.dv),
-                            ops.delta_solved_floats(T, T // limit, self.nkv, self.nh, self.d))
+                            ops.delta_solved_floats(T, T // limit, self.nkv, self.nh, self.d, self.dv))
             ws.reserve("linear_states", self.scratch[0], torch.float32)
             ws.reserve("delta_solved", self.scratch[1], torch.float32)
         self.w_all = self.w_proj = self.w_ba = self.w_o = self.w_a2 = self.w_g2 = None

@@ -125,3 +125,42 @@ def test_refuses_what_it_does_not_take(ops):
     solved = torch.empty(ops.delta_solved_floats(T, 1, H, H, d), device="cuda")
     assert not ops.delta_chunks(rows, w, w, st, scratch, solved, i32([0]), i32([0]), 1, i32([0, T]), i32([T]), i32([0]), 1, H, H, d, dv, out)
     assert bool((out == 7.0).all())
+
+
+def error(x, y):
+    return float((x.double() - y).norm() / y.norm())
+
+
+@pytest.mark.parametrize("G,H,d,dv,lens", [(4, 16, 128, 128, [1280, 768]), (2, 16, 64, 64, [2000, 1500, 700]), (1, 8, 128, 144, [3600]),
+                                           (1, 4, 96, 32, [700, 513, 835])])
+@pytest.mark.parametrize("fast", [True, False])
+def test_no_further_from_float64_than_the_walk(ops, G, H, d, dv, lens, fast):
+    """Values and decays as a layer makes them (a step's softplus times 1 to 16, or 1 - 2^-5 to 1 - 2^-13 over the heads), blocks of one, two
+    and four heads: float32 sums in another order, not fewer bits."""
+    gen = torch.Generator(device="cuda").manual_seed(H + dv)
+    rnd, uni = (lambda *s: torch.randn(*s, device="cuda", generator=gen)), (lambda *s: torch.rand(*s, device="cuda", generator=gen))  # noqa: E731
+    T, B = sum(lens), len(lens)
+    rows = torch.nn.functional.silu(rnd(T, 2 * G * d + H * dv))
+    qk = rows[:, :2 * G * d].view(T, 2 * G, d)
+    qk /= qk.norm(dim=-1, keepdim=True)
+    rows[:, :G * d] *= d ** -0.5
+    if fast:
+        start = 1e-3 * 100.0 ** uni(H)
+        decay = torch.exp(-(1 + 15 * uni(H)) * torch.nn.functional.softplus(rnd(T, H) + start + torch.log(-torch.expm1(-start))))
+    else:
+        decay = (1.0 - 2.0 ** (-5.0 - 8.0 * torch.arange(H, device="cuda") / (H - 1))).expand(T, H).contiguous()
+    beta, state = torch.sigmoid(rnd(T, H)), rnd(B, H, dv, d) * 0.3
+    slots, cu, ctx = i32(list(range(B))), i32([sum(lens[:b]) for b in range(B + 1)]), i32([n + 40 for n in lens])
+    want, after, at = torch.zeros(T, H * dv, dtype=torch.float64, device="cuda"), state.double(), 0
+    for b, n in enumerate(lens):
+        r = rows[at:at + n].double()
+        q, k = (r[:, i * G * d:(i + 1) * G * d].view(n, G, d).repeat_interleave(H // G, 1) for i in (0, 1))
+        o, after[b] = walk(q, k, r[:, 2 * G * d:].view(n, H, dv), decay[at:at + n].double(), beta[at:at + n].double(), after[b])
+        want[at:at + n] = o.reshape(n, -1)
+        at += n
+    st, st2, walked = state.clone(), state.clone(), torch.full((T, H * dv), float("nan"), device="cuda")
+    out = chunks(ops, rows, beta, decay, st, slots, cu, ctx, [(b, x) for b, n in enumerate(lens) for x in range(0, n, 128)], G, H, d, dv)
+    ops.delta_recur(rows, beta, decay, st2, cu, ctx, slots, B, G, H, d, dv, walked)
+    print(f"rows {error(out, want):.2e}, walk {error(walked, want):.2e}; state {error(st, after):.2e}, walk {error(st2, after):.2e}")
+    # measured over 40 such steps: rows 0.56 to 1.09 of the walk's error, states 0.42 to 0.76
+    assert error(out, want) < 1.25 * error(walked, want) and error(st, after) < error(st2, after)

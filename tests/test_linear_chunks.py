@@ -146,3 +146,27 @@ def test_mixers_recurrence_takes_chunks_for_long_portions(ops, monkeypatch, lens
         assert float((a - b).norm() / b.norm()) < (8e-6 if chunked else 1e-12)
     walked = [b for b, n in enumerate(lens) if n < need.at_least]
     assert torch.equal(got[0][walked], want[0][walked]) and torch.equal(got[1][lens[0]:], want[1][lens[0]:])
+
+
+@pytest.mark.parametrize("G,H,d,dv,lens,heads", [(4, 16, 64, 64, [1280, 700, 68], 2), (4, 16, 64, 200, [1280, 700, 68], 2),
+                                                 (1, 32, 64, 64, [1280, 700, 68], 4), (1, 32, 64, 128, [2048], 4), (1, 64, 64, 32, [2048, 100], 8)])
+def test_several_heads_of_a_block(ops, G, H, d, dv, lens, heads):
+    """Steps so long that a block of the rows takes two, four or eight heads of a group: beside the token-by-token kernel."""
+    gen = torch.Generator(device="cuda").manual_seed(H + dv)
+    T, B = sum(lens), len(lens)
+    tiles = [(b, x) for b, n in enumerate(lens) for x in range(0, n, 128)]
+    turns = lambda h: -(-len(tiles) * (H // h) // 148) * (4 + 5 * h)  # noqa: E731
+    assert min((h for h in (1, 2, 4, 8) if H // G % h == 0), key=turns) == heads
+    rows = torch.randn(T, 2 * G * d + H * dv, device="cuda", generator=gen)
+    rows[:, :2 * G * d] *= d ** -0.5
+    beta, decay = torch.rand(T, H, device="cuda", generator=gen), torch.exp(-0.1 * torch.rand(T, H, device="cuda", generator=gen))
+    state = torch.randn(B, H, dv, d, device="cuda", generator=gen)
+    cu, ctx, slots = i32([sum(lens[:b]) for b in range(B + 1)]), i32([n + 9 for n in lens]), i32(list(range(B)))
+    scratch = torch.full((ops.linear_scratch_floats(T, B, H, d, dv),), float("nan"), device="cuda")
+    got, want = [(state.clone(), torch.full((T, H * dv), float("nan"), device="cuda")) for _ in range(2)]
+    assert ops.linear_chunks(rows, beta, decay, got[0], scratch, i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), len(tiles), cu, ctx,
+                             slots, B, G, H, d, dv, got[1])
+    ops.delta_recur(rows, beta, decay, want[0], cu, ctx, slots, B, G, H, d, dv, want[1], plain=True)
+    assert int(ops.tc_status("cuda")[0]) == 0
+    for a, b in zip(got, want):                            # (each within 4e-6 of float64, above)
+        assert float((a - b).norm() / b.norm()) < 8e-6
