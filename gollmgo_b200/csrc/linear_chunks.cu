@@ -82,8 +82,7 @@ __device__ __forceinline__ LcTokens lc_tokens(const LinearArgs& p, int t0, int n
   }
   return x;
 }
-// Sums of logarithms as two float32 parts (48 bits): a difference of two is then three float32 subtractions and as exact as a float64
-// one that is rounded to float32 (which takes the multiprocessor's few float64 units and a conversion).
+// Sums of logarithms as two float32 parts (48 bits).
 struct LcSums { float hi[LC_C], lo[LC_C]; };
 // By one warp: L (inclusive sums of log2 of the decays) and the factors b [128] of the chunk's n tokens.  Returns their whole sum.
 __device__ __forceinline__ double lc_sums(const LinearArgs& p, const LcTokens& x, int n, int h, LcSums& L, float* b) {
@@ -113,7 +112,13 @@ __device__ __forceinline__ double lc_sums(const LinearArgs& p, const LcTokens& x
   }
   return __shfl_sync(0xffffffffu, before + a[3], 31);
 }
-__device__ __forceinline__ float lc_power(float hi, float lo, float hi2, float lo2) { return exp2f((hi - hi2) + (lo - lo2)); }
+// Two to the difference of two such sums, rounded once, as a float64 difference would be: what rounding takes from hi - hi2 goes with the
+// small parts.  (Without that, two roundings: a power of 2^-8 to 2^-14 is off by 3.0e-7 instead of 2.0e-7.  With float64 subtractions the
+// conversions take longer than these seven instructions: rows of 2048 tokens and 64 heads 97 us against 87.)
+__device__ __forceinline__ float lc_power(float hi, float lo, float hi2, float lo2) {
+  const float s = hi - hi2, t = s - hi;
+  return exp2f(s + (((hi - (s - t)) - (hi2 + t)) + (lo - lo2)));
+}
 
 __device__ __forceinline__ void lc_split(float x, float& hi, float& lo) {
   hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
