@@ -77,6 +77,22 @@ class DeltaTiles(ChunkTiles):
         return listed if 1.04 * cost < self.walk_us([q_lens[b] for b in portions]) else []
 
 
+def one_kernel(B, groups, heads, d, dv):
+    """Whether B single tokens go through delta_step (csrc/delta_rule.cu) and not through three kernels.  It saves two launches, but has a
+    block of 512 threads a sequence and head, and clusters of the heads that share q and k.  A B200, us with a small product behind, one
+    kernel / three, 64 x 64: 4 heads, 1: 4.8 / 7.4; 48 heads on 6 (clusters of eight), 8: 10.9 / 12.6, 16: 17.6 / 16.5; 32 on 8, 32: 15.9 /
+    15.7, 64: 30.5 / 24.5.  128 x 128: 16 on 4, 8: 8.1 / 12.9, 32: 20.3 / 22.4; 8 on 1, 16: 11.5 / 12.6, 32: 14.4 / 13.9.  64 x 128:
+    48 on 6, 16: 25.0 / 25.6.  64 x 256: 16 on
+    4, 16: 17.3 / 20.1, 32: 25.3 / 24.3; 8 on 1, 8: 9.0 / 10.6, 16: 14.6 / 13.9.  128 x 256, half the state in registers: 8 heads, 4: 11.1
+    / 10.3, 8: 11.1 / 13.4.  (And no more than 32 MB of states: the kernel's own limit.)"""
+    blocks = B * heads
+    if dv == 256:
+        return (48 if d == 128 else 1) <= blocks <= (64 if heads == 8 * groups else 256)
+    if heads == 8 * groups:
+        return blocks <= (768 if d != dv else 512 if d == 64 else 192)
+    return blocks <= 1024
+
+
 _NAMES = {"q": "q", "k": "k", "v": "v", "beta": "b", "a": "a", "gate": "g", "o": "o", "A_log": "A_log",
           "dt_bias": "dt_bias", "norm": "norm", "a1": "a1", "a2": "a2", "g1": "g1", "g2": "g2"}
 
@@ -250,9 +266,10 @@ class GatedDeltaRule:
         else:
             gate = proj[:, self.gate_col:self.gate_col + self.gate_cols]
         B = batch.num_seqs
-        if T == B and batch.num_portions == 0 and self.dw == 1 and self.taps > 1 and proj.dtype == torch.bfloat16 and ops.delta_step(
-                proj, self.conv_w, conv_state, zb, za, self.a_log, self.dt_bias, state, batch.cu_q_lens, batch.context_lens,
-                batch.state_slots, B, self.nkv, H, self.d, self.dv, gate, self.norm_w, self.eps, y, self.gate_act):
+        if T == B and batch.num_portions == 0 and self.dw == 1 and self.taps > 1 and proj.dtype == torch.bfloat16 \
+                and one_kernel(B, self.nkv, H, self.d, self.dv) and ops.delta_step(
+                    proj, self.conv_w, conv_state, zb, za, self.a_log, self.dt_bias, state, batch.cu_q_lens, batch.context_lens,
+                    batch.state_slots, B, self.nkv, H, self.d, self.dv, gate, self.norm_w, self.eps, y, self.gate_act):
             return linear(y, self.w_o, ws.get(self.out_buffer, T, self.hidden), then)
         qkv = ws.get("delta_qkv", T, self.channels)
         beta, decay = ws.get("delta_beta", T, H), ws.get("delta_decay", T, hw)

@@ -78,3 +78,32 @@ def test_two_products_in_one_launch(ops, M, split, more, K, normed):
     # the same float32 sums; a row's block may start elsewhere along K
     assert float((tail - b).norm() / b.norm()) < 1e-6
     assert float((out.float() - a.float()).norm() / a.float().norm()) < 1e-3
+
+
+@pytest.mark.parametrize("M", [1, 16, 17])
+@pytest.mark.parametrize("N", [64, 4736])
+def test_layer_product_with_a_tail(ops, M, N):
+    """linear_with_tail: one launch up to sixteen tokens, two products beyond and where the weights are not stored together."""
+    from gollmgo_b200.parts.linear import linear_with_tail
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, 256, device="cuda", generator=gen).bfloat16()
+    w = torch.randn(N + 32, 256, device="cuda", generator=gen).bfloat16() / 16
+    got = []
+    for together in (w, None):
+        out, tail = torch.empty(M, N, device="cuda", dtype=torch.bfloat16), torch.empty(M, 32, device="cuda")
+        a, b = linear_with_tail(x, together, w[:N], w[N:], out, tail)
+        assert a is out and b is tail
+        got.append((out.float(), tail))
+    # the same float32 sums in another order, and roundings to bfloat16 that fall on the other side
+    assert float((got[0][1] - got[1][1]).norm() / got[1][1].norm()) < 1e-6
+    assert float((got[0][0] - got[1][0]).norm() / got[1][0].norm()) < 1e-3
+
+
+def test_steps_that_keep_three_kernels():
+    """The sizes at which one kernel was measured to be the slower form (the rule's edges)."""
+    from gollmgo_b200.parts.gated_delta import one_kernel
+    assert one_kernel(1, 4, 4, 64, 64) and one_kernel(32, 4, 16, 128, 128) and one_kernel(64, 16, 16, 64, 64)
+    assert one_kernel(8, 6, 48, 64, 64) and not one_kernel(16, 6, 48, 64, 64) and not one_kernel(64, 8, 32, 64, 64)
+    assert one_kernel(16, 1, 8, 128, 128) and not one_kernel(32, 1, 8, 128, 128)
+    assert one_kernel(16, 4, 16, 64, 256) and not one_kernel(32, 4, 16, 64, 256) and not one_kernel(16, 1, 8, 64, 256)
+    assert one_kernel(8, 1, 8, 128, 256) and not one_kernel(4, 1, 8, 128, 256) and not one_kernel(1, 2, 2, 128, 256)
