@@ -24,7 +24,7 @@
 #define GSM_THREADS (GSM_WARPS * 32)
 #define GSM_SPAN 64               // k per warp per iteration
 
-enum { GSM_OUT_BF16 = 0, GSM_OUT_F32 = 1, GSM_OUT_SILU = 2, GSM_OUT_RESNORM = 3 };
+enum { GSM_OUT_BF16 = 0, GSM_OUT_F32 = 1, GSM_OUT_SILU = 2, GSM_OUT_RESNORM = 3, GSM_OUT_TAIL = 4 };
 
 // Two ways to keep an RMSNorm out of the chain of kernels (rms = sqrt(mean(h^2) + eps)):
 //   * the product that ends a mixer or feed-forward (mode GSM_OUT_RESNORM) adds its result to
@@ -45,7 +45,7 @@ struct GsmFuse {
   // and u = clamp(up, -limit, limit), g * sigmoid(alpha * g) * (u + shift)
   float act_limit, act_alpha, act_shift;
   int relu2;                  // GSM_OUT_BF16: the square of relu of the result
-  // GSM_OUT_BF16, split > 0: rows of W from split on go to tail [M, N - split] in float32, the others to out [M, split]
+  // GSM_OUT_TAIL: rows of W from split on go to tail [M, N - split] in float32, the others to out [M, split]
   int split;
   float* tail;
 };
@@ -270,7 +270,7 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
               if (fuse.in_partials) v *= row_scale[tok];
               if (MODE == GSM_OUT_BF16 && fuse.relu2) { v = fmaxf(v, 0.f); v *= v; }
               if (MODE == GSM_OUT_F32) reinterpret_cast<float*>(out)[(size_t)tok * N + n] = v;
-              else if (MODE == GSM_OUT_BF16 && fuse.split > 0) {
+              else if (MODE == GSM_OUT_TAIL) {
                 if (n < fuse.split) reinterpret_cast<__nv_bfloat16*>(out)[(size_t)tok * fuse.split + n] = __float2bfloat16_rn(v);
                 else fuse.tail[(size_t)tok * (N - fuse.split) + n - fuse.split] = v;
               } else reinterpret_cast<__nv_bfloat16*>(out)[(size_t)tok * N + n] = __float2bfloat16_rn(v);
@@ -297,7 +297,7 @@ static int gemm_small_m_run(const void* x, long long ldx, const void* W, void* o
   GG_REQUIRE(M <= 16, "gemm_small_m: %d tokens; this kernel takes at most 16", M);
   GG_REQUIRE(K % 8 == 0 && ldx % 8 == 0, "gemm_small_m: K=%d and the row stride %lld of x must be multiples of 8", K, ldx);
   GG_REQUIRE(((size_t)x % 16) == 0 && ((size_t)W % 16) == 0, "gemm_small_m: x and W must be 16-byte aligned");
-  GG_REQUIRE(mode >= 0 && mode <= 3, "gemm_small_m: unknown mode %d", mode);
+  GG_REQUIRE(mode >= 0 && mode <= 4, "gemm_small_m: unknown mode %d", mode);
   GG_REQUIRE(!in_partials || (in_tiles > 0 && hidden > 0), "gemm_small_m: partial sums without their sizes");
   GG_REQUIRE(mode != GSM_OUT_RESNORM || (resid && norm_w && out_partials), "gemm_small_m: mode 3 needs resid, norm_w and out_partials");
   if (M == 0) return GG_OK;
@@ -335,7 +335,8 @@ static int gemm_small_m_run(const void* x, long long ldx, const void* W, void* o
     if (mode == 0) GSM_LAUNCH(NT, GSM_OUT_BF16, GROUP, XB);            \
     else if (mode == 1) GSM_LAUNCH(NT, GSM_OUT_F32, GROUP, XB);        \
     else if (mode == 2) GSM_LAUNCH(NT, GSM_OUT_SILU, GROUP, XB);       \
-    else GSM_LAUNCH(NT, GSM_OUT_RESNORM, GROUP, XB);                   \
+    else if (mode == 3) GSM_LAUNCH(NT, GSM_OUT_RESNORM, GROUP, XB);    \
+    else GSM_LAUNCH(NT, GSM_OUT_TAIL, GROUP, XB);                      \
   } while (0)
   const int per_cta = (num_tiles + grid - 1) / grid;      // most row tiles one CTA gets
   if (M <= 8) {
@@ -352,6 +353,7 @@ extern "C" int gg_gemm_small_m_fused(const void* x, long long ldx, const void* W
                                      int K, int mode, const float* in_partials, int in_tiles, int hidden,
                                      float eps, float* resid, const float* norm_w, float* out_partials,
                                      cudaStream_t stream) {
+  GG_REQUIRE(mode >= 0 && mode <= 3, "gemm_small_m: unknown mode %d", mode);
   return gemm_small_m_run(x, ldx, W, out, M, N, K, mode, in_partials, in_tiles, hidden, eps, resid, norm_w, out_partials,
                           0.f, 0.f, 0.f, stream);
 }
@@ -369,8 +371,8 @@ extern "C" int gg_gemm_small_m_clamped(const void* x, long long ldx, const void*
 extern "C" int gg_gemm_small_m_tail(const void* x, long long ldx, const void* W, void* out, float* tail, int M, int N, int split, int K,
                                     const float* in_partials, int in_tiles, int hidden, float eps, cudaStream_t stream) {
   GG_REQUIRE(split > 0 && split < N && tail, "gemm_small_m: a tail of %d of %d rows", N - split, N);
-  return gemm_small_m_run(x, ldx, W, out, M, N, K, 0, in_partials, in_tiles, hidden, eps, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f, stream, 0,
-                          split, tail);
+  return gemm_small_m_run(x, ldx, W, out, M, N, K, GSM_OUT_TAIL, in_partials, in_tiles, hidden, eps, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f,
+                          stream, 0, split, tail);
 }
 
 // out = the square of relu(x W^T), bfloat16.
