@@ -21,8 +21,8 @@
 // beside that.  With the products on mma.sync (tf32 there runs at 486 multiply-adds a clock and multiprocessor) every warp
 // had to split its fragments again: 215 us for the state-space layer below and 225 for retention.
 // Measured (B200), us for the three kernels, before: 2048 tokens of one sequence, a state-space layer of 64 heads of 64 with a
-// state of 128: 40 + 11 + 97, token by token 359; 2011 tokens of three, retention of 16 heads 128 x 256: 40 + 9 + 81, packed
-// float32 232.  Slower: reads two steps ahead (registers spill: rows 130 and 117); groups of four warps with a step each
+// state of 128: 41 + 9 + 83, token by token 359; 2011 tokens of three, retention of 16 heads 128 x 256: 42 + 9 + 77, packed
+// float32 232 (each kernel alone).  Slower: reads two steps ahead (registers spill: rows 130 and 117, where they took 97); groups of four warps with a step each
 // (rows 112); two issuers (no change).
 // All waits on barriers are bounded; one that runs out sets *status and the CTA winds down.
 #include "tc_common.cuh"
@@ -719,7 +719,9 @@ template <int NB, bool RETENTION, typename TA> static int lc_rows(const LinearAr
 
 // The rows: a CTA takes one to eight heads of a group, so many that the machine is done soonest.  A chunk's products q_i . k_j take a
 // CTA about as long as 0.8 of a head (10 k clocks of 12 k), and one CTA fits on a multiprocessor: 64 heads of a group and 16 chunks as
-// 128 CTAs of eight heads 92 us, as 256 of four 101; 16 heads on 4 groups as 128 CTAs of two 37, as 256 of one 45.
+// 128 CTAs of eight heads 92 us, as 256 of four 101; 16 heads on 4 groups as 128 CTAs of two 37, as 256 of one 45.  With values of 16 to
+// 256, keys of 32 to 256, 8 to 128 heads on 1 to 32 groups and 256 to 4096 tokens no step of 84 became slower by this choice than with as
+// many heads as left 222 CTAs (0.74 to 1.00 of its time, the shorter arithmetic of the decays included).
 template <bool RETENTION, typename TA> static int lc_all_rows(LinearArgs p, int num_tiles, cudaStream_t stream) {
   p.heads = 1;
   auto turns = [&](int heads) { return ((long long)num_tiles * (p.H / heads) + 147) / 148 * (4 + 5 * heads); };

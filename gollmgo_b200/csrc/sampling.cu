@@ -29,7 +29,7 @@ __device__ __forceinline__ float uniform_draw(unsigned long long seed, unsigned 
 
 // Which values of a row a thread has: four neighbouring ones from 4 start on, every 4 stride further.  Two blocks that share a row
 // have the threads of one twice as large between them.  AHEAD: how many pairs of loads are on their way beside the pair at hand;
-// 0: eight loads at a time, for a pass of a few instructions a value alone (argmax of 128 k: 5.9 us, with pairs of loads 7.6).
+// 0: eight loads at a time, for a pass of a few instructions a value alone (argmax of 128 k: 5.0 us, with pairs of loads 7.5).
 template <int AHEAD = 1> struct Walk { int start, stride; };
 
 // f(i, v, there) for every four values v at row[4 i] that are this thread's, by whole warps (there: inside the row).  A pass runs its
@@ -491,9 +491,11 @@ __device__ unsigned int radix_threshold(const float* row, int V, float m, float 
 // (those above the k-th largest of the threads' own maxima, some hundreds), or one pass for the sum and the leading byte
 // of top_p and one that copies the values of that byte to shared memory (`room` of them; what does not fit is walked where
 // it is); the sums in index order.  What bounds it: the chain of passes, each a few turns of a loop by 16 or 32 warps, whose code
-// arrives from L2 too (each_four).  128 k values, 148 rows: 49 us with top_k, 96 with top_p alone (before loops of two loads: 55, 117).
-// BLOCKS = 2: the row on two multiprocessors, each with half of the threads (PairPub); the same numbers in the same order.  64 rows:
-// 40 us with top_k, 66 with top_p alone, 28 without either, where one multiprocessor a row took 50, 114 and 36.
+// arrives from L2 too (each_four).  128 k values, 148 rows: 41 us with top_k, 90 with top_p alone (before loops of two loads: 55, 117).
+// BLOCKS = 2: the row on two multiprocessors, each with half of the threads (PairPub); the same numbers in the same order.  64 rows, us
+// without thresholds, with top_k, with top_p alone, with both; two multiprocessors a row / one: 128 k values 21 / 26, 33 / 37, 58 / 85,
+// 44 / 52; 32 k 10.4 / 11.3, 21 / 22, 26 / 33, 31 / 33; 16384 (the fewest) 8.6 / 8.6, 18.7 / 19.2, 19.8 / 23.4, 26.9 / 28.4; 38 and 74
+// rows alike.
 template <int BLOCKS>
 __global__ void __launch_bounds__(SAMPLE_THREADS / BLOCKS)
 sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__ temperature,
@@ -912,8 +914,8 @@ extern "C" int gg_sample(const float* logits, int R, int V, const float* tempera
         cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || num_sms <= 0)
       num_sms = 148;
   }
-  // (with more rows than clusters fit at once, two CTAs per SM, two CTAs a row are faster: 37 rows on clusters take 28 us without
-  // thresholds, 52 with top-k, 74 with top-p alone, 38 rows in pairs 27, 39 and 66)
+  // (with more rows than clusters fit at once, two CTAs per SM, two CTAs a row are faster: 37 rows of 128 k on clusters take 22 us
+  // without thresholds, 46 with top-k, 70 with top-p alone, 38 rows in pairs 21, 32 and 58)
   if (use_cluster && V >= SC_MIN_V && smem <= 160 * 1024 && R * SC_CLUSTER <= 2 * num_sms) {
     static bool set = false;
     if (!set) {
