@@ -164,3 +164,25 @@ def test_no_further_from_float64_than_the_walk(ops, G, H, d, dv, lens, fast):
     print(f"rows {error(out, want):.2e}, walk {error(walked, want):.2e}; state {error(st, after):.2e}, walk {error(st2, after):.2e}")
     # measured over 40 such steps: rows 0.56 to 1.09 of the walk's error, states 0.42 to 0.76
     assert error(out, want) < 1.25 * error(walked, want) and error(st, after) < error(st2, after)
+
+
+@pytest.mark.parametrize("where", ["v", "k", "beta"])
+def test_bad_values_in_wide_rows(ops, where):
+    """The same where a block's rows have 128 and sixteen columns and four heads: what is no number reaches what it reaches in the walk, in
+    its chunk and behind it, and the other heads and sequences not at all."""
+    G, H, d, dv, lens, at = 2, 8, 128, 144, [700, 2048, 2000], 700 + 1000
+    rows, beta, decay, state, slots, cu, ctx, tiles = make(lens, [0, 5, 0], G, H, d, dv, 0.05)
+    assert len(tiles) * H >= 222 and H // G % 2 == 0       # (two heads a block)
+    clean = chunks(ops, rows, beta, decay, state.clone(), slots, cu, ctx, tiles, G, H, d, dv)
+    if where == "beta":
+        beta[at, 3] = float("nan")
+    else:
+        rows[at, {"k": G * d + d + 3, "v": 2 * G * d + 3 * dv + 130}[where]] = float("nan")
+    st, st2, walked = state.clone(), state.clone(), torch.full((sum(lens), H * dv), 7.0, device="cuda")
+    out = chunks(ops, rows, beta, decay, st, slots, cu, ctx, tiles, G, H, d, dv)
+    ops.delta_recur(rows, beta, decay, st2, cu, ctx, slots, len(lens), G, H, d, dv, walked)
+    assert torch.equal(torch.isfinite(out), torch.isfinite(walked)) and torch.equal(torch.isfinite(st), torch.isfinite(st2))
+    assert bool((~torch.isfinite(out[at:700 + 2048])).any())
+    fine = torch.isfinite(out)
+    assert torch.equal(out[:at], clean[:at]) and torch.equal(out[700 + 2048:], clean[700 + 2048:])
+    assert float((out[fine] - clean[fine]).norm() / clean[fine].norm()) < 1e-12
